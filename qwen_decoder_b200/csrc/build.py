@@ -32,10 +32,12 @@ NVCC_FLAGS = [
 LIBRARIES: Dict[str, str] = {
     "elementwise": "elementwise.cu",
     "gemm_generic": "gemm_generic.cu",
+    "gemm_f32": "gemm_f32.cu",
     "gemm_skinny": "gemm_skinny.cu",
     "gemm_stream": "gemm_stream.cu",
     "gemm_tc5": "gemm_tc5.cu",
     "attention_generic": "attention_generic.cu",
+    "attention_f32": "attention_f32.cu",
     "attention_flash": "attention_flash.cu",
     "attention_decode_rope": "attention_decode_rope.cu",
     "attention_tc5": "attention_tc5.cu",

@@ -261,6 +261,62 @@ def gemm_generic(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
         _I(T), _I(N), _I(K), _LL(x.stride(0)), _LL(out.stride(0)), _stream()), "gemm_generic")
 
 
+F32_FEW_TOKENS = 8         # up to here a float32 product is bound by reading its weights, beyond by the FMA units
+
+
+def gemm_f32_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether the float32 kernels for rows of whole 16-byte pieces take this product (``gemm_generic`` takes any)."""
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and x.shape[1] % 4 == 0 and x.stride(0) % 4 == 0
+            and x.stride(1) == 1 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+def gemm_f32_splits(T: int, N: int, K: int) -> int:
+    """Shares of K of a float32 product of more than 16 tokens: those with which the multiprocessor with the most tiles
+    (128 features x up to 128 tokens x a share of K) is done first, counting what the partial sums cost to write and read
+    again; no share below 128 of K."""
+    if T <= F32_FEW_TOKENS or N % 4:
+        return 1
+    tiles = _f32_tiles(T, N)
+    steps, sms, best = -(-K // 32), sm_count(), None
+    rows = -(-T // tiles[1])
+    for s in range(1, max(1, min(24, steps // 4)) + 1):
+        rounds = -(-tiles[0] * tiles[1] * s // sms)
+        cost = rounds * (-(-steps // s) + 4) * tiles[2] + (s * T * N * 8 / 2048 + 2000 if s > 1 else 0)
+        if best is None or cost < best[0]:
+            best = (cost, s)
+    return best[1]
+
+
+def _f32_tiles(T: int, N: int):
+    """(tiles over N, tiles over T, cycles of a tile's step of 32 k) of the float32 product of ``T`` tokens."""
+    if T <= 64:
+        places = 4 if T <= 32 else 8
+        rows, cols = -(-T // 8) * 8, 1024 // places
+        return -(-N // cols), 1, max(rows * cols * 32 // 128, cols * 9)
+    m_tiles = -(-T // 128)
+    rows = -(-(-(-T // m_tiles)) // 16) * 16
+    return -(-N // 128), -(-T // rows), rows * 32
+
+
+def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
+             splits: Optional[int] = None) -> None:
+    """out[T, N] = x[T, K] @ w[N, K]^T (+ bias), all float32, float32 FMA; x and out may be row-strided.  ``splits``: shares
+    of K (by default ``gemm_f32_splits``)."""
+    T, K = x.shape
+    N = w.shape[0]
+    assert gemm_f32_supported(x, w) and w.shape[1] == K and out.shape == (T, N)
+    assert out.dtype == torch.float32 and out.stride(1) == 1
+    _contig(w, "w")
+    if bias is not None:
+        assert bias.dtype == torch.float32 and bias.numel() == N
+    if splits is None:
+        splits = gemm_f32_splits(T, N, K)
+    part = torch.empty((splits, T, N), dtype=torch.float32, device=x.device) if splits > 1 else None
+    _check(library("gemm_f32").qd_gemm_f32(
+        _ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(part), _I(T), _I(N), _I(K), _LL(x.stride(0)), _LL(out.stride(0)),
+        _I(splits), _stream()), "gemm_f32")
+
+
 SKINNY_MAX_TOKENS = 64      # what the mma.sync few-token kernels take
 # Who takes a product of T tokens was settled by measurement in whole decode steps (profiles/); the numbers are
 # module attributes so that a measurement can move them, not switches of the environment.
@@ -533,6 +589,36 @@ def paged_attention_generic(q: torch.Tensor, q_stride: int, out: torch.Tensor, k
         _ptr(q), _LL(q_stride), _ptr(out), _LL(out.stride(0)), _ptr(kv), _I(dtype_code(q.dtype)),
         _ptr(block_table), _I(block_table.shape[1]), _ptr(token_req), _ptr(positions), _I(n_tokens),
         _I(H), _I(G), _I(d), _I(page_size), _F(scale), _I(window), _stream()), "paged_attention_generic")
+
+
+def attention_f32_supported(dtype: torch.dtype, H: int, G: int, d: int) -> bool:
+    return dtype == torch.float32 and d % 4 == 0 and d <= 128 and H % G == 0
+
+
+def attention_f32_splits(n_tokens: int, H: int, G: int, max_keys: int) -> int:
+    """Shares of the keys: two CTAs to a multiprocessor where the (token, kv head) pairs are fewer, no share below 64 keys
+    (two rounds of a CTA's eight warps)."""
+    pairs = n_tokens * G * -(-(H // G) // 8)
+    if pairs > _TICKETS:
+        return 1
+    return max(1, min(2 * sm_count() // max(1, pairs), -(-max_keys // 64), 64))
+
+
+def attention_f32(q: torch.Tensor, q_stride: int, out: torch.Tensor, kv: torch.Tensor, block_table: torch.Tensor,
+                  token_req: torch.Tensor, positions: torch.Tensor, n_tokens: int, H: int, G: int, d: int, page_size: int,
+                  scale: float, window: int, splits: int) -> None:
+    """As ``paged_attention_generic``, float32 with a head size of at most 128 in multiples of 4; the keys of a (token, kv
+    head) are shared by ``splits`` CTAs."""
+    assert attention_f32_supported(q.dtype, H, G, d) and kv.dtype == out.dtype == torch.float32
+    assert block_table.dtype == torch.int32 and block_table.dim() == 2
+    assert token_req.dtype == torch.int32 and positions.dtype == torch.int32
+    assert out.shape == (n_tokens, H * d) and tuple(kv.shape[1:]) == (2, G, page_size, d)
+    _contig(out, "out"); _contig(kv, "kv"); _contig(block_table, "block_table")
+    part_o, part_ml, tickets = decode_scratch(n_tokens, H, d, G * -(-(H // G) // 8), splits, q.device)
+    _check(library("attention_f32").qd_attention_f32(
+        _ptr(q), _LL(q_stride), _ptr(out), _ptr(kv), _ptr(block_table), _I(block_table.shape[1]), _ptr(token_req),
+        _ptr(positions), _I(n_tokens), _I(H), _I(G), _I(d), _I(page_size), _F(scale), _I(window), _I(splits), _ptr(part_o),
+        _ptr(part_ml), _ptr(tickets), _stream()), "attention_f32")
 
 
 FLASH_HEAD_DIMS = (16, 32, 48, 64, 96, 128)

@@ -116,6 +116,11 @@ class GQAttention(Mixer):
                 if _PREFILL_TC5 and kernels.prefill_tc5_supported(x.dtype, H, G, d, ps) else kernels.prefill_attention
             fn(qkv, qkv.stride(0), attn, cache.kv, cache.group.block_table[nd:], ctx.cu_tokens[nd:],
                ctx.start_pos[nd:], ctx.num_requests - nd, ctx.num_tokens - nd, H, G, d, ps, self.scale, window)
+        elif kernels.attention_f32_supported(x.dtype, H, G, d):
+            kernels.attention_f32(
+                qkv, qkv.stride(0), attn, cache.kv, cache.group.block_table, ctx.token_request, ctx.positions,
+                ctx.num_tokens, H, G, d, ps, self.scale, window,
+                kernels.attention_f32_splits(ctx.num_tokens, H, G, min(ctx.max_context, window or ctx.max_context)))
         else:
             kernels.paged_attention_generic(
                 qkv, qkv.stride(0), attn, cache.kv, cache.group.block_table, ctx.token_request,

@@ -1,0 +1,65 @@
+"""The float32 kernels for rows of whole 16-byte pieces, at the edges of their tiles, against float64."""
+import math
+
+import pytest
+import torch
+
+from test_kernels_gpu import DEV, _paged_setup, close
+import plain_model
+
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("guard_regions")]
+
+
+@pytest.mark.parametrize("T", [1, 2, 3, 5, 8, 9, 17, 25, 33, 41, 64, 65, 97, 128, 129, 203, 260])
+@pytest.mark.parametrize("N,K,splits", [(8, 4, 1), (129, 36, 1), (260, 516, 3), (1000, 2048, None), (8200, 132, None)])
+def test_gemm_f32(T, N, K, splits):
+    from qwen_decoder_b200 import kernels
+    if splits and T <= kernels.F32_FEW_TOKENS:
+        splits = 1
+    g = torch.Generator(device=DEV).manual_seed(T * N + K)
+    x = torch.empty(T, K + 8, device=DEV).normal_(generator=g)[:, 4:4 + K]          # rows of a wider buffer
+    w = torch.empty(N, K, device=DEV).normal_(0.0, 0.05, generator=g)
+    for bias in (None, torch.empty(N, device=DEV).normal_(generator=g)):
+        out = torch.empty(T, N + 3, dtype=torch.float32, device=DEV)
+        out.fill_(7.0)
+        kernels.gemm_f32(x, w, bias, out[:, :N], splits=splits)
+        close(out[:, :N], x.double() @ w.double().t() + (bias.double() if bias is not None else 0.0), torch.float32)
+        assert bool((out[:, N:] == 7.0).all())
+
+
+def test_gemm_f32_dispatch():
+    """What the kernel for whole pieces refuses (a row that is none, a start off the boundary) takes the general one."""
+    from qwen_decoder_b200 import kernels
+    from qwen_decoder_b200.parts import matmul_backend
+    g = torch.Generator(device=DEV).manual_seed(5)
+    for T, N, K, shift in ((3, 40, 30, 0), (20, 40, 32, 1), (20, 40, 32, 0)):
+        wide = torch.empty(T, K + 4, device=DEV).normal_(generator=g)
+        x = wide[:, shift:shift + K]
+        w = torch.empty(N, K, device=DEV).normal_(generator=g)
+        assert kernels.gemm_f32_supported(x, w) == (K % 4 == 0 and shift == 0)
+        out = torch.empty(T, N, dtype=torch.float32, device=DEV)
+        matmul_backend.linear(x, w, None, out)
+        close(out, x.double() @ w.double().t(), torch.float32)
+
+
+@pytest.mark.parametrize("cfg", [(16, 2, 128, 16, None), (7, 1, 64, 32, None), (3, 3, 4, 8, 37), (24, 2, 100, 16, 50), (4, 2, 16, 1, None)])
+@pytest.mark.parametrize("splits", [1, 3, 64])
+def test_attention_f32(cfg, splits):
+    from qwen_decoder_b200 import kernels
+    H, G, d, page_size, window = cfg
+    lens = [133, 1, 33]
+    kv, bt, ks, vs = _paged_setup(torch.float32, lens, G, d, page_size, seed=8)
+    items = [(0, p) for p in (0, 3, 31, 32, 95, 132)] + [(1, 0)] + [(2, p) for p in (4, 32)]
+    q = torch.randn(len(items), (H + 2 * G) * d, generator=torch.Generator().manual_seed(9))     # q, k and v side by side
+    q[2] *= 4.0
+    out = torch.empty(len(items), H * d, dtype=torch.float32, device=DEV)
+    tr, pos = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in zip(*items))
+    for _ in range(2):                                       # the second launch finds the tickets as the first left them
+        kernels.attention_f32(q.to(DEV), q.shape[1], out, kv.to(DEV), bt.to(DEV), tr, pos, len(items), H, G, d, page_size,
+                              1.0 / math.sqrt(d), window or 0, splits)
+    for i, (r, p) in enumerate(items):
+        n = p + 1
+        qq = torch.zeros(n, H * d, dtype=torch.float64)
+        qq[p] = q[i, :H * d].double()
+        want = plain_model.attention(qq, ks[r][:n].double().reshape(n, G * d), vs[r][:n].double().reshape(n, G * d), H, G, d, window)[p]
+        close(out[i], want, torch.float32, scale=float(vs[r][:n].abs().max()))
