@@ -264,6 +264,15 @@ def gemm_generic(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
 F32_FEW_TOKENS = 8         # up to here a float32 product is bound by reading its weights, beyond by the FMA units
 
 
+# Smaller matrices stay with ``gemm_generic``: a few microseconds either way, and there a row's sums do not depend on how many
+# rows there are.
+F32_MIN_WEIGHTS = 1 << 17
+
+
+def gemm_f32_wanted(x: torch.Tensor, w: torch.Tensor) -> bool:
+    return w.numel() > F32_MIN_WEIGHTS and gemm_f32_supported(x, w)
+
+
 def gemm_f32_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether the float32 kernels for rows of whole 16-byte pieces take this product (``gemm_generic`` takes any)."""
     return (x.dtype == torch.float32 and w.dtype == torch.float32 and x.shape[1] % 4 == 0 and x.stride(0) % 4 == 0
@@ -315,6 +324,51 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out
     _check(library("gemm_f32").qd_gemm_f32(
         _ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(part), _I(T), _I(N), _I(K), _LL(x.stride(0)), _LL(out.stride(0)),
         _I(splits), _stream()), "gemm_f32")
+
+
+# A product of more tokens than this on the tensor cores: at 32 tokens the FMA tiles and they are equal (3B sizes, gate/up 91
+# against 88 us, the output projection 14.1 against 15.5), at 40 105 against 91, at 203 478 against 160.  Smaller matrices than
+# F32_SPLIT_MIN_WEIGHTS stay with the FMA tiles: two launches more.
+F32_SPLIT_TOKENS = 32
+F32_SPLIT_MIN_WEIGHTS = 1 << 20
+
+
+def gemm_f32_split_wanted(T: int, N: int, K: int) -> bool:
+    return T > F32_SPLIT_TOKENS and N * K >= F32_SPLIT_MIN_WEIGHTS
+
+
+def gemm_f32_split_shares(T: int, N: int, K: int) -> int:
+    """Shares of K of a float32 product on the tensor cores: those with which the busiest multiprocessor is done first."""
+    t_tiles = -(-T // 224)
+    cols = -(-(-(-T // t_tiles)) // 32) * 32
+    tiles, blocks, sms, best = -(-N // 128) * t_tiles, -(-K // 64), sm_count(), None
+    for s in range(1, (max(1, min(16, blocks // 2)) if N % 4 == 0 else 1) + 1):
+        # cycles, as measured: a block of 64 k takes 24 a token column (fetching the three pieces of the tokens), at least
+        # 3,500 (reading and cutting W); 4,000 for a tile's beginning and end; partial sums at about 2 KB a cycle for the whole
+        # chip, and a launch
+        cost = -(-tiles * s // sms) * (-(-blocks // s) * max(24 * cols, 3500) + 4000) + (s * T * N * 8 // 2048 + 4000 if s > 1 else 0)
+        if best is None or cost < best[0]:
+            best = (cost, s)
+    return best[1]
+
+
+def gemm_f32_split(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
+                   splits: Optional[int] = None) -> None:
+    """As ``gemm_f32``, on the tensor cores with both operands cut into three bfloat16 pieces that sum to them exactly."""
+    T, K = x.shape
+    N = w.shape[0]
+    assert gemm_f32_supported(x, w) and w.shape[1] == K and out.shape == (T, N)
+    assert out.dtype == torch.float32 and out.stride(1) == 1
+    _contig(w, "w")
+    if bias is not None:
+        assert bias.dtype == torch.float32 and bias.numel() == N
+    if splits is None:
+        splits = gemm_f32_split_shares(T, N, K)
+    pieces = torch.empty((3, T, -(-K // 64) * 64), dtype=torch.bfloat16, device=x.device)
+    part = torch.empty((splits, T, N), dtype=torch.float32, device=x.device) if splits > 1 else None
+    _check(library("gemm_f32_split").qd_gemm_f32_split(
+        _ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(pieces), _ptr(part), _I(T), _I(N), _I(K), _LL(x.stride(0)),
+        _LL(out.stride(0)), _I(splits), _stream()), "gemm_f32_split")
 
 
 SKINNY_MAX_TOKENS = 64      # what the mma.sync few-token kernels take
@@ -770,6 +824,7 @@ def prefill_attention_tc5_status() -> int:
 # library -> (its status function, its wait probe): the kernels with bounded waits on mbarriers or a grid barrier
 _STATUS = {"gemm_stream": ("qd_gemm_stream_status", "qd_gemm_stream_wait_probe"),
            "gemm_tc5": ("qd_gemm_tc5_status", "qd_gemm_tc5_wait_probe"),
+           "gemm_f32_split": ("qd_gemm_f32_split_status", "qd_gemm_f32_split_wait_probe"),
            "attention_tc5": ("qd_prefill_attention_tc5_status", "qd_prefill_attention_tc5_wait_probe"),
            "attention_flash": ("qd_decode_attention_tma_status", "qd_decode_attention_tma_wait_probe")}
 

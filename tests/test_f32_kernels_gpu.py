@@ -27,12 +27,33 @@ def test_gemm_f32(T, N, K, splits):
         assert bool((out[:, N:] == 7.0).all())
 
 
+@pytest.mark.parametrize("T", [1, 32, 33, 100, 128, 203, 224, 225, 449])
+@pytest.mark.parametrize("N,K,splits", [(8, 4, 1), (130, 68, 1), (260, 516, 2), (1000, 2048, None), (256, 1152, 1)])
+def test_gemm_f32_split(T, N, K, splits):
+    """The tensor cores on operands cut into three pieces: edges of tiles of 128 features and of 224 tokens, a last block of k
+    that is not whole, shares of K, an accumulator moved several times (K = 2048 and 1152 in one share)."""
+    from qwen_decoder_b200 import kernels
+    g = torch.Generator(device=DEV).manual_seed(T * N + K)
+    x = torch.empty(T, K + 8, device=DEV).normal_(generator=g)[:, 4:4 + K]
+    x[T // 2, K // 2] *= 1e4                                 # one element far above the others
+    w = torch.empty(N, K, device=DEV).normal_(0.0, 0.05, generator=g)
+    for bias in (None, torch.empty(N, device=DEV).normal_(generator=g)):
+        out = torch.empty(T, N + 4, dtype=torch.float32, device=DEV)
+        out.fill_(7.0)
+        kernels.gemm_f32_split(x, w, bias, out[:, :N], splits=splits)
+        want = x.double() @ w.double().t() + (bias.double() if bias is not None else 0.0)
+        # row by row: at most 16 MMAs a chunk of the large products at 2^-24 of the largest partial sum each, and roundings
+        rows = want.abs().amax(dim=1, keepdim=True).clamp(min=1e-3)
+        assert float(((out[:, :N].double() - want).abs() / rows).max()) < 3e-6
+        assert bool((out[:, N:] == 7.0).all())
+
+
 def test_gemm_f32_dispatch():
     """What the kernel for whole pieces refuses (a row that is none, a start off the boundary) takes the general one."""
     from qwen_decoder_b200 import kernels
     from qwen_decoder_b200.parts import matmul_backend
     g = torch.Generator(device=DEV).manual_seed(5)
-    for T, N, K, shift in ((3, 40, 30, 0), (20, 40, 32, 1), (20, 40, 32, 0)):
+    for T, N, K, shift in ((3, 400, 510, 0), (20, 400, 512, 1), (20, 400, 512, 0), (20, 40, 32, 0), (40, 1100, 1000, 0)):
         wide = torch.empty(T, K + 4, device=DEV).normal_(generator=g)
         x = wide[:, shift:shift + K]
         w = torch.empty(N, K, device=DEV).normal_(generator=g)
