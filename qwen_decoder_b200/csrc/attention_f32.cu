@@ -174,16 +174,30 @@ attention_f32_kernel(const float* __restrict__ q, long long q_stride, float* __r
   if (!last || warp >= nh) return;
   __threadfence();
   const size_t at = ((size_t)t * H + h0 + warp) * splits;
-  float top = -INFINITY;
-  for (int s = 0; s < splits; s++) top = fmaxf(top, __ldcg(part_ml + (at + s) * 2));
+  float top = -INFINITY, sum = 0.f;
   float4 a = zero;
-  float sum = 0.f;
-  for (int s = 0; s < splits; s++) {
-    const float f = expf(__ldcg(part_ml + (at + s) * 2) - top);
-    sum = fmaf(__ldcg(part_ml + (at + s) * 2 + 1), f, sum);
-    if (on) {
-      const float4 b = __ldcg(reinterpret_cast<const float4*>(part_o + (at + s) * d + lane * 4));
-      a.x = fmaf(b.x, f, a.x); a.y = fmaf(b.y, f, a.y); a.z = fmaf(b.z, f, a.z); a.w = fmaf(b.w, f, a.w);
+  constexpr int PB = 8;                              // shares in flight: each would be a trip to L2 of its own
+  for (int s0 = 0; s0 < splits; s0 += PB) {
+    float2 mlv[PB];
+    float4 pv[PB];
+#pragma unroll
+    for (int u = 0; u < PB; u++) {
+      const bool in = s0 + u < splits;
+      mlv[u] = in ? __ldcg(reinterpret_cast<const float2*>(part_ml) + at + s0 + u) : make_float2(-INFINITY, 0.f);
+      pv[u] = in && on ? __ldcg(reinterpret_cast<const float4*>(part_o + (at + s0 + u) * d + lane * 4)) : zero;
+    }
+    float best = top;
+#pragma unroll
+    for (int u = 0; u < PB; u++) best = fmaxf(best, mlv[u].x);
+    if (best == -INFINITY) continue;                 // none of these shares had a key
+    const float old = expf(top - best);
+    top = best;
+    sum *= old; a.x *= old; a.y *= old; a.z *= old; a.w *= old;
+#pragma unroll
+    for (int u = 0; u < PB; u++) {
+      const float f = expf(mlv[u].x - best);
+      sum = fmaf(mlv[u].y, f, sum);
+      a.x = fmaf(pv[u].x, f, a.x); a.y = fmaf(pv[u].y, f, a.y); a.z = fmaf(pv[u].z, f, a.z); a.w = fmaf(pv[u].w, f, a.w);
     }
   }
   const float inv = 1.0f / sum;

@@ -11,6 +11,15 @@
 #include <math.h>
 
 #define SB 1024
+#define S_AHEAD 8          // loads of a thread in flight: a row is one multiprocessor's 600 KB from L2, several times
+#define S_LIST 2048        // entries that may be among the k largest, at most
+#define S_WALK 256         // a list up to here is searched by every thread, once for each of its entries; else the row's segments
+
+// One CTA per row.  The k-th largest logit: the k-th largest of the 1,024 threads' own maxima is a lower bound of it (each is an
+// entry of its own), so one more pass collects the entries that reach the bound, usually little more than k, and what follows
+// works on that list; four passes with counts in shared memory (most logits share a few leading bytes, and their counters) remain
+// for k above 1,024 and for lists that overflow.  At 151,936 logits and k = 40 those passes took 129 us; a float32 step of four
+// sampled requests took 3.38 ms with them and 3.20 so (with attention_f32.cu's combine, which went with it).
 
 __device__ __forceinline__ unsigned order_key(float f) {
   unsigned u = __float_as_uint(f);
@@ -31,17 +40,26 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
   __shared__ unsigned s_hist[256];
   __shared__ float s_scratch[40];
   __shared__ unsigned s_prefix, s_remaining;
-  __shared__ int s_result;
+  __shared__ int s_result, s_count;
+  __shared__ unsigned list_key[S_LIST], s_some[SB / 32];
+  __shared__ int list_idx[S_LIST];
   int r = blockIdx.x, tid = threadIdx.x;
   const float* row = logits + (size_t)r * V;
 
   // 1. maximum and its lowest index
   float best = -INFINITY;
   int bi = 0x7fffffff;
-  for (int i = tid; i < V; i += SB) {
-    float v = row[i];
-    if (v > best || bi == 0x7fffffff) { best = v; bi = i; }
+  for (int i0 = tid; i0 < V; i0 += S_AHEAD * SB) {
+    float v[S_AHEAD];
+#pragma unroll
+    for (int u = 0; u < S_AHEAD; u++) v[u] = i0 + u * SB < V ? row[i0 + u * SB] : 0.0f;
+#pragma unroll
+    for (int u = 0; u < S_AHEAD; u++) {
+      const int i = i0 + u * SB;
+      if (i < V && (v[u] > best || bi == 0x7fffffff)) { best = v[u]; bi = i; }
+    }
   }
+  const unsigned own_key = order_key(best);
   s_val[tid] = best; s_idx[tid] = bi;
   __syncthreads();
   for (int s = SB / 2; s > 0; s >>= 1) {
@@ -65,7 +83,68 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
   // 2. threshold = k-th largest logit (radix select on order-preserving keys)
   int k = top_k[r];
   float threshold = -INFINITY;
-  if (k > 0 && k < V) {
+  bool listed = false;
+  if (k > 0 && k < V && k <= SB) {
+    // the k-th largest of the threads' maxima, then of the list, by the same selection on keys
+    auto select = [&](int n, auto&& key_at) {
+      if (tid == 0) { s_prefix = 0; s_remaining = (unsigned)k; }
+      __syncthreads();
+      for (int shift = 24; shift >= 0; shift -= 8) {
+        if (tid < 256) s_hist[tid] = 0;
+        __syncthreads();
+        const unsigned prefix = s_prefix, mask = shift == 24 ? 0u : (0xffffffffu << (shift + 8));
+        for (int i = tid; i < n; i += SB) {
+          const unsigned key = key_at(i);
+          if ((key & mask) == prefix) atomicAdd(&s_hist[(key >> shift) & 255u], 1u);
+        }
+        __syncthreads();
+        if (tid < 32) {
+          // lane l holds the eight digits below 256 - 8 l: the digit where the count from above reaches the rest
+          unsigned c[8], sum = 0;
+#pragma unroll
+          for (int u = 0; u < 8; u++) { c[u] = s_hist[255 - (tid * 8 + u)]; sum += c[u]; }
+          unsigned incl = sum;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (tid >= o) incl += v;
+          }
+          const unsigned rem = s_remaining, before = incl - sum;
+          __syncwarp();
+          if (before < rem && rem <= incl) {
+            unsigned left = rem - before;
+            int u = 0;
+            while (left > c[u]) left -= c[u++];
+            s_prefix = prefix | ((unsigned)(255 - (tid * 8 + u)) << shift);
+            s_remaining = left;
+          }
+        }
+        __syncthreads();
+      }
+      return s_prefix;
+    };
+    const unsigned bound = select(SB, [&](int) { return own_key; });
+    if (tid == 0) s_count = 0;
+    __syncthreads();
+    for (int i0 = tid; i0 < V; i0 += S_AHEAD * SB) {
+      float v[S_AHEAD];
+#pragma unroll
+      for (int u = 0; u < S_AHEAD; u++) v[u] = i0 + u * SB < V ? row[i0 + u * SB] : 0.0f;
+#pragma unroll
+      for (int u = 0; u < S_AHEAD; u++) {
+        const int i = i0 + u * SB;
+        const unsigned key = order_key(v[u]);
+        if (i < V && key >= bound) {
+          const int at = atomicAdd(&s_count, 1);
+          if (at < S_LIST) { list_key[at] = key; list_idx[at] = i; }
+        }
+      }
+    }
+    __syncthreads();
+    listed = s_count <= S_LIST;
+    if (listed) threshold = key_to_float(select(s_count, [&](int i) { return list_key[i]; }));
+  }
+  if (k > 0 && k < V && !listed) {
     if (tid == 0) { s_prefix = 0; s_remaining = (unsigned)k; }
     __syncthreads();
     for (int shift = 24; shift >= 0; shift -= 8) {
@@ -98,11 +177,34 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
   int seg = (V + SB - 1) / SB;
   int lo = tid * seg, hi = lo + seg < V ? lo + seg : V;
   float part = 0.0f;
-  for (int i = lo; i < hi; i++) {
-    float v = row[i];
-    if (v >= threshold) part += expf((v - mx) / temp);
+  const int n = s_count;
+  if (listed && n <= S_WALK) {
+    // every entry that is kept is in the list: those of the segment in their order
+    for (int last = lo - 1; last < hi;) {
+      int next = hi;
+      float v = 0.0f;
+      for (int j = 0; j < n; j++) {
+        const int i = list_idx[j];
+        if (i > last && i < next) {
+          const float w = key_to_float(list_key[j]);
+          if (w >= threshold) { next = i; v = w; }
+        }
+      }
+      if (next < hi) part += expf((v - mx) / temp);
+      last = next;
+    }
+  } else {
+    for (int i = lo; i < hi; i++) {
+      float v = row[i];
+      if (v >= threshold) part += expf((v - mx) / temp);
+    }
   }
   s_val[tid] = part;
+  // which segments hold anything: the search below passes over the others
+  {
+    const unsigned some = __ballot_sync(0xffffffffu, part > 0.0f);
+    if ((tid & 31) == 0) s_some[tid >> 5] = some;
+  }
   __syncthreads();
   float total = block_sum(part, s_scratch);
   // 4. first index whose running sum reaches r * total
@@ -110,9 +212,11 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
     float target = draws[r] * total;
     float cum = 0.0f;
     int found = -1;
-    for (int sgi = 0; sgi < SB && found < 0; sgi++) {
+    for (int word = 0; word < SB / 32 && found < 0; word++)
+    for (unsigned bits = s_some[word]; bits && found < 0; bits &= bits - 1) {
+      const int sgi = word * 32 + __ffs(bits) - 1;
       float next = cum + s_val[sgi];
-      if (target <= next && s_val[sgi] > 0.0f) {
+      if (target <= next) {
         int a = sgi * seg, b = a + seg < V ? a + seg : V;
         for (int i = a; i < b; i++) {
           float v = row[i];
