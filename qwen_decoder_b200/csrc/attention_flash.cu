@@ -72,14 +72,13 @@ __device__ __forceinline__ float fast_exp2(float x) {
 // The end of a decode attention CTA, shared by the kernels below: the warps' partial results (o, running
 // maxima m and denominators l of 16 rows each) are merged in shared memory; with one split the result is
 // written, otherwise it goes to scratch and the CTA that finishes last for its (token, kv head) adds up all
-// splits.  Every warp must be done with the stage buffers that start at smem_raw.  Head h's split s lies at place
-// h * row_stride + row0 + s of the scratch.
+// splits.  Every warp must be done with the stage buffers that start at smem_raw.
 template <int HD>
 __device__ __forceinline__ void dec_finish(float (&o)[HD / 8][4], float m0, float m1, float l0, float l1,
                                            unsigned char* smem_raw, int warp, int lane, int gs, int g, int t, int s,
                                            int H, int G, int splits, bf16* __restrict__ out,
                                            float* __restrict__ part_o, float* __restrict__ part_ml,
-                                           unsigned* __restrict__ tickets, size_t row_stride, size_t row0) {
+                                           unsigned* __restrict__ tickets) {
   l0 = quad_sum(l0);
   l1 = quad_sum(l1);
   __syncthreads();  // every warp is done with its stage buffers: reuse them for the merge
@@ -127,7 +126,7 @@ __device__ __forceinline__ void dec_finish(float (&o)[HD / 8][4], float m0, floa
       raw.y = pack_bf16(O.z * inv, O.w * inv);
       *reinterpret_cast<uint2*>(out + (size_t)t * H * HD + (size_t)h * HD + dim) = raw;
     } else {
-      const size_t pi = (size_t)h * row_stride + row0 + s;
+      const size_t pi = ((size_t)t * H + h) * splits + s;
       *reinterpret_cast<float4*>(part_o + pi * HD + dim) = O;
       if (dim == 0) { part_ml[pi * 2] = M; part_ml[pi * 2 + 1] = L; }
     }
@@ -153,7 +152,7 @@ __device__ __forceinline__ void dec_finish(float (&o)[HD / 8][4], float m0, floa
   constexpr int PB = 16;
   for (int idx = threadIdx.x; idx < gs * (HD / 4); idx += DEC_WARPS * 32) {
     const int row = idx / (HD / 4), d4 = idx - row * (HD / 4);
-    const size_t base = ((size_t)g * gs + row) * row_stride + row0;
+    const size_t base = ((size_t)t * H + (size_t)g * gs + row) * splits;
     const float2* ml_g = reinterpret_cast<const float2*>(part_ml) + base;
     float2 mlv[PB];
     float4 pv[PB];
@@ -344,8 +343,7 @@ decode_attention_kernel(const bf16* __restrict__ q, long long q_stride, bf16* __
   }
   cp_async_wait<0>();
   pdl_launch_dependents();
-  dec_finish<HD>(o, m0, m1, l0, l1, smem_raw, warp, lane, gs, g, t, s, H, G, splits, out, part_o, part_ml, tickets,
-                 splits, (size_t)t * H * splits);
+  dec_finish<HD>(o, m0, m1, l0, l1, smem_raw, warp, lane, gs, g, t, s, H, G, splits, out, part_o, part_ml, tickets);
 }
 
 // ------------------------------------------------------------------ the same with K/V through TMA
@@ -367,7 +365,7 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const bf
                             const int* __restrict__ token_req, const int* __restrict__ positions, int H, int G,
                             int page_size, float scale_log2e, int window, int splits,
                             float* __restrict__ part_o, float* __restrict__ part_ml,
-                            unsigned* __restrict__ tickets, int* __restrict__ status, int shared) {
+                            unsigned* __restrict__ tickets, int* __restrict__ status) {
   static_assert(HD % 64 == 0, "boxes of 64 columns");
   constexpr int NB = HD / 64;                      // boxes per K or V chunk
   constexpr int BOX = 16 * 64;                     // elements of a box (2 KB)
@@ -378,13 +376,9 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const bf
   __shared__ int page_ring[DEC_WARPS][64];
   // the swizzle pattern follows address bits 7-9: stages start on 1024-byte boundaries
   bf16* smem = reinterpret_cast<bf16*>(smem_raw + ((1024 - (fa_smem(smem_raw) & 1023)) & 1023));
-  int s = blockIdx.x, t = blockIdx.z;
-  const int g = blockIdx.y;
+  const int s = blockIdx.x, g = blockIdx.y, t = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gs = H / G;
-  int pos = positions[t], req = token_req[t], pos4[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) pos4[i] = lane + 32 * i < shared ? positions[lane + 32 * i] : pos;
   if (threadIdx.x == 0) {
     dead = 0;
     for (int w = 0; w < DEC_WARPS; w++)
@@ -392,76 +386,15 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const bf
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(fa_smem(&bars[w][st])), "r"(1));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  size_t row_stride = splits, row0 = (size_t)t * H * splits;
-  if (shared) {
-    // ``shared`` = T tokens, up to 128, a lane looks at four.  All in one chunk: ``splits`` CTAs to each request.  Else the
-    // T * splits CTAs go by the least number of chunks, four at least, that none has to exceed: the longest request no longer
-    // decides.  A step of 23 requests of up to 2,048 tokens beside a portion of 489, 7B sizes: 8.30 -> 8.19 ms (with the TMA copies).
-    // Steps that only decode don't ask for it: ragged they gain (7B, 23 requests of up to 4,001: 3.98 -> 3.76 ms; 3B, 64 of up to
-    // 4,096: 3.42 -> 3.24) but equal lengths lose 0.3 us a launch to looking (64 of 2,049: 3.072 -> 3.084 ms).
-    int apart = 0;
-#pragma unroll
-    for (int i = 0; i < 4; i++) apart |= pos4[i] ^ pos;
-    if (__any_sync(0xffffffffu, apart & ~(DEC_CHUNK - 1))) {
-      const int T = shared, idx = t * splits + s;
-      int c[4], sum = 0;
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const int lo_t = window > 0 && pos4[i] - window + 1 > 0 ? pos4[i] - window + 1 : 0;
-        c[i] = lane + 32 * i < T ? pos4[i] / DEC_CHUNK + 1 - lo_t / DEC_CHUNK : 0;
-        sum += c[i];
-      }
-      sum = __reduce_add_sync(0xffffffffu, sum);
-      int lo = max(4, sum / (T * splits)), hi = max(4, sum / (T * (splits - 1)) + 1), n[4], total;    // hi is enough: T CTAs are rounding
-      auto count = [&](int most) {
-        const float inv = 1.f / (float)most;
-        total = 0;
-#pragma unroll
-        for (int i = 0; i < 4; i++) total += n[i] = __float2int_ru((float)c[i] * inv);
-        return __reduce_add_sync(0xffffffffu, total);
-      };
-      for (int i = 0; i < 5 && lo < hi; i++) {
-        const int mid = (lo + hi) / 2;
-        if (count(mid) <= T * splits) hi = mid; else lo = mid + 1;
-      }
-      const int all = count(hi);
-      int end = total;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, end, o);
-        if (lane >= o) end += v;
-      }
-      if (all <= T * splits) {       // always, but for the quotients' rounding
-        int at = end - total, found = -1, first_of = 0, parts = 0;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          if (idx >= at && idx < at + n[i]) { found = lane + 32 * i; first_of = at; parts = n[i]; }
-          at += n[i];
-        }
-        const unsigned who = __ballot_sync(0xffffffffu, found >= 0);
-        if (!who) {
-          pdl_wait();
-          return;
-        }
-        const int from = __ffs(who) - 1;
-        t = __shfl_sync(0xffffffffu, found, from);
-        row0 = __shfl_sync(0xffffffffu, first_of, from);
-        row_stride = T * splits;
-        splits = __shfl_sync(0xffffffffu, parts, from);
-        s = idx - (int)row0;
-        pos = positions[t];
-        req = token_req[t];
-      }
-    }
-  }
   __syncthreads();
+  const int pos = positions[t];
   const int n_keys = pos + 1;
   const int key_lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
   const int chunk_lo = key_lo / DEC_CHUNK, chunk_hi = (n_keys + DEC_CHUNK - 1) / DEC_CHUNK;
   const int per = (chunk_hi - chunk_lo + splits - 1) / splits;
   const int c0 = chunk_lo + s * per;
   const int c1 = min(chunk_hi, c0 + per);
-  const int* bt = block_table + (size_t)req * max_blocks;
+  const int* bt = block_table + (size_t)token_req[t] * max_blocks;
   bf16* wbuf = smem + (size_t)warp * DEC_STAGES * STAGE;
   const int first = c0 + warp;
   const int n_my = first < c1 ? (c1 - first + DEC_WARPS - 1) / DEC_WARPS : 0;
@@ -591,8 +524,7 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const bf
     __syncwarp();
   }
   pdl_launch_dependents();
-  dec_finish<HD>(o, m0, m1, l0, l1, smem_raw, warp, lane, gs, g, t, s, H, G, splits, out, part_o, part_ml, tickets,
-                 row_stride, row0);
+  dec_finish<HD>(o, m0, m1, l0, l1, smem_raw, warp, lane, gs, g, t, s, H, G, splits, out, part_o, part_ml, tickets);
 }
 
 // out[t, h, :] = sum_s O_s * 2^(m_s - M) / sum_s l_s * 2^(m_s - M)
@@ -697,7 +629,7 @@ template <int HD>
 static int launch_decode_tma(const CUtensorMap& map, const bf16* q, long long q_stride, bf16* out, const int* block_table,
                              int max_blocks, const int* token_req, const int* positions, int T, int H, int G,
                              int page_size, float scale, int window, int splits, float* part_o, float* part_ml,
-                             unsigned* tickets, int* status, int by_length, cudaStream_t stream) {
+                             unsigned* tickets, int* status, cudaStream_t stream) {
   size_t smem = (size_t)DEC_WARPS * DEC_STAGES * 2 * DEC_CHUNK * HD * sizeof(bf16) + 1024;
   if (cudaFuncSetAttribute(decode_attention_tma_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess) {
@@ -707,20 +639,18 @@ static int launch_decode_tma(const CUtensorMap& map, const bf16* q, long long q_
   dim3 grid(splits, G, T);
   qd_launch(decode_attention_tma_kernel<HD>, dim3(grid), dim3(DEC_WARPS * 32), smem, stream, map, q, q_stride, out,
             block_table, max_blocks, token_req, positions, H, G, page_size, scale * 1.4426950408889634f, window, splits,
-            part_o, part_ml, tickets, status, by_length && splits > 1 ? T : 0);
+            part_o, part_ml, tickets, status);
   return qd_last_error();
 }
 
 // As qd_decode_attention with K/V fetched by TMA tensor copies: head size 64 or 128, tickets required when
-// splits > 1, the cache 16-byte aligned; ``n_pages`` = pages of ``kv``.  Anything else is refused.  ``by_length`` (up to 128 tokens):
-// ``splits`` is the mean, a request's number goes by its length.
+// splits > 1, the cache 16-byte aligned; ``n_pages`` = pages of ``kv``.  Anything else is refused.
 extern "C" int qd_decode_attention_tma(const void* q, long long q_stride, void* out, const void* kv, long long n_pages,
                                        const int* block_table, int max_blocks, const int* token_req,
                                        const int* positions, int T, int H, int G, int d, int page_size, float scale,
                                        int window, int splits, float* part_o, float* part_ml, unsigned* tickets,
-                                       int by_length, cudaStream_t stream) {
+                                       cudaStream_t stream) {
   if (T <= 0) return 0;
-  if (by_length && T > 128) return QD_ERR_UNSUPPORTED;
   if (G <= 0 || H % G != 0 || H / G > 16 || page_size % DEC_CHUNK != 0 || splits < 1 || splits > 64 || T > 65535 ||
       G > 65535 || (d != 64 && d != 128) || n_pages < 1)
     return QD_ERR_UNSUPPORTED;
@@ -741,9 +671,9 @@ extern "C" int qd_decode_attention_tma(const void* q, long long q_stride, void* 
     return QD_ERR_UNSUPPORTED;
   if (d == 64)
     return launch_decode_tma<64>(map, (const bf16*)q, q_stride, (bf16*)out, block_table, max_blocks, token_req, positions,
-                                 T, H, G, page_size, scale, window, splits, part_o, part_ml, tickets, status, by_length, stream);
+                                 T, H, G, page_size, scale, window, splits, part_o, part_ml, tickets, status, stream);
   return launch_decode_tma<128>(map, (const bf16*)q, q_stride, (bf16*)out, block_table, max_blocks, token_req, positions,
-                                T, H, G, page_size, scale, window, splits, part_o, part_ml, tickets, status, by_length, stream);
+                                T, H, G, page_size, scale, window, splits, part_o, part_ml, tickets, status, stream);
 }
 
 // 0 if no bounded wait of the TMA decode kernel has run out on the current device (reported once).  Synchronises.

@@ -47,7 +47,7 @@ struct PeFns {
   decltype(&qd_prefill_attention) attention_regs;       // mma.sync, any supported head size
   decltype(&qd_prefill_attention_tc5) attention_tc5;    // tcgen05, head size 64 or 128
   decltype(&qd_decode_attention) attention_decode;      // split-KV, for the single tokens of a mixed step
-  decltype(&qd_decode_attention_tma) attention_decode_tma;      // the same by TMA copies (null: not at this head size)
+  decltype(&qd_decode_attention_tma) attention_decode_tma;      // the same by TMA copies, the same bits (null: not at this head size)
   PeGemmEx gemm_ex;
   cublasHandle_t blas;             // the caller's handle, bound to ``stream``
   PeGemmBatched gemm_batched;
@@ -73,8 +73,7 @@ struct PeParams {
   // the down projection over ``down_shares`` equal shares of F as one batched product that leaves float32 partial
   // sums [down_shares, T, D] in ``down_part`` for the next norm's kernel (0: the plain product into ``delta``).
   // With few tokens, a long K and few output features the plain product fills the GPU with too few CTAs.
-  float* down_part; int down_shares;
-  int decode_by_length;            // the single tokens' CTAs go by their lengths (attention_decode_tma)
+  float* down_part; int down_shares, pad2;
 };
 
 extern "C" int qd_prompt_exec_struct_sizes(int* layer_bytes, int* params_bytes) {
@@ -131,7 +130,7 @@ extern "C" int qd_prompt_exec(const PeParams* pp, cudaStream_t stream) {
     if (nd > 0 && p.fn.attention_decode_tma && (p.decode_splits == 1 || p.tickets))
       PE_TRY(p.fn.attention_decode_tma(p.qkv, n_qkv, p.attn, L.kv, p.n_pages, p.block_table, p.max_blocks, p.token_req,
                                        p.positions, nd, H, G, d, p.page_size, p.scale, p.window, p.decode_splits, p.part_o,
-                                       p.part_ml, p.tickets, p.decode_by_length, stream));
+                                       p.part_ml, p.tickets, stream));
     else if (nd > 0)
       PE_TRY(p.fn.attention_decode(p.qkv, n_qkv, p.attn, L.kv, p.block_table, p.max_blocks, p.token_req, p.positions,
                                    nd, H, G, d, p.page_size, p.scale, p.window, p.decode_splits, p.part_o, p.part_ml,

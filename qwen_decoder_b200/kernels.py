@@ -693,19 +693,15 @@ _tickets = {}
 _DECODE_TMA = _os.environ.get("QD_DECODE_TMA", "1") != "0"
 
 
-DECODE_BY_LENGTH_TOKENS = 128      # a lane looks at four tokens
-
-
-def decode_by_tma(n_tokens: int, d: int):
-    """Whether split-KV decode attention fetches by TMA copies, and whether its CTAs go by the requests' lengths."""
-    tma = _DECODE_TMA and d in (64, 128)
-    return tma, tma and 2 <= n_tokens <= DECODE_BY_LENGTH_TOKENS
+def decode_by_tma(d: int) -> bool:
+    """Whether split-KV decode attention fetches by TMA copies (the same bits either way)."""
+    return _DECODE_TMA and d in (64, 128)
 
 
 def decode_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, kv: torch.Tensor,
                      block_table: torch.Tensor, token_req: torch.Tensor, positions: torch.Tensor,
                      n_tokens: int, H: int, G: int, d: int, page_size: int, scale: float, window: int,
-                     splits: int, fused_combine: bool = True, by_length: bool = False) -> None:
+                     splits: int, fused_combine: bool = True) -> None:
     """One query token per request over its cached keys (tensor cores, keys split over ``splits``
     CTAs per (request, kv head); partial results go through scratch memory when splits > 1)."""
     assert q.dtype == torch.bfloat16 and kv.dtype == torch.bfloat16 and out.dtype == torch.bfloat16
@@ -713,7 +709,6 @@ def decode_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, kv: torc
     assert block_table.dtype == torch.int32 and block_table.dim() == 2
     _contig(out, "out"); _contig(kv, "kv"); _contig(block_table, "block_table")
     part_o = part_ml = tickets = None
-    tma, can_share = decode_by_tma(n_tokens, d)
     if splits > 1:
         part_o = torch.empty((n_tokens * H * splits, d), dtype=torch.float32, device=q.device)
         part_ml = torch.empty((n_tokens * H * splits, 2), dtype=torch.float32, device=q.device)
@@ -721,13 +716,13 @@ def decode_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, kv: torc
             tickets = _tickets.get(q.device)
             if tickets is None:     # zero once; every launch leaves them zero again
                 tickets = _tickets[q.device] = torch.zeros(_TICKETS, dtype=torch.int32, device=q.device)
-    if tma and splits <= 64 and (splits == 1 or tickets is not None):
+    if decode_by_tma(d) and splits <= 64 and (splits == 1 or tickets is not None):
         # K/V chunks by TMA tensor copies instead of 16-byte cp.async
         _check(library("attention_flash").qd_decode_attention_tma(
             _ptr(q), _LL(q_stride), _ptr(out), _ptr(kv), _LL(kv.shape[0]), _ptr(block_table),
             _I(block_table.shape[1]), _ptr(token_req), _ptr(positions), _I(n_tokens), _I(H), _I(G), _I(d),
             _I(page_size), _F(scale), _I(window), _I(splits), _ptr(part_o), _ptr(part_ml), _ptr(tickets),
-            _I(int(by_length and can_share)), _stream()), "decode_attention_tma")
+            _stream()), "decode_attention_tma")
         return
     _check(library("attention_flash").qd_decode_attention(
         _ptr(q), _LL(q_stride), _ptr(out), _ptr(kv), _ptr(block_table), _I(block_table.shape[1]),
@@ -1812,7 +1807,7 @@ class PromptParams(ctypes.Structure):
                                         "attn", "delta", "gu", "act", "hrows")] + \
         [("n_decode", ctypes.c_int), ("decode_splits", ctypes.c_int)] + \
         [(n, ctypes.c_void_p) for n in ("token_req", "part_o", "part_ml", "tickets", "down_part")] + \
-        [("down_shares", ctypes.c_int), ("decode_by_length", ctypes.c_int)]
+        [("down_shares", ctypes.c_int), ("pad2", ctypes.c_int)]
 
 
 def prompt_exec_struct_sizes_match() -> bool:

@@ -141,8 +141,7 @@ class NativePrompt:
         use_tc5 = self.attention_impl(group.page_size)
         # a mixed step: its single tokens (first in the batch) go to the split-KV decode kernel
         nd = ctx.num_decode if kernels.flash_decode_supported(bf, H, G, d, group.page_size) else 0
-        tma, p.decode_by_length = kernels.decode_by_tma(nd, d)
-        p.fn = kernels.prompt_fns(bool(use_tc5), nd > 0, nd > 0 and tma)
+        p.fn = kernels.prompt_fns(bool(use_tc5), nd > 0, nd > 0 and kernels.decode_by_tma(d))
         keep = None
         if nd:
             from .attention import decode_splits
