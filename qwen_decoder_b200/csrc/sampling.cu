@@ -123,7 +123,9 @@ sample_kernel(const float* __restrict__ logits, int V, const float* __restrict__
       }
       return s_prefix;
     };
-    const unsigned bound = select(SB, [&](int) { return own_key; });
+    unsigned bound = select(SB, [&](int) { return own_key; });
+    // kept is what reaches the threshold by value, and -0 reaches +0 though its key lies below
+    if (bound == order_key(0.0f)) bound = order_key(-0.0f);
     if (tid == 0) s_count = 0;
     __syncthreads();
     for (int i0 = tid; i0 < V; i0 += S_AHEAD * SB) {

@@ -42,3 +42,19 @@ def test_sample_selection(V, kind):
     kernels.sample(torch.from_numpy(logits).to(DEV), t(temps, torch.float32), t(ks, torch.int32), t(draws, torch.float32), out)
     for r, got in enumerate(out.tolist()):
         assert 0 <= got < V and fits(logits[r], ks[r], float(temps[r]), float(draws[r]), got), (r, ks[r], got)
+
+
+def test_zeros_of_both_signs_tie():
+    """k = 2 with the largest value 0 at five places, two of them +0: the threshold is +0, -0 reaches it too, so each of the five is
+    drawn a fifth of the time."""
+    from qwen_decoder_b200 import kernels
+    V, n = 2000, 64
+    row = np.full(V, -30.0, np.float32)
+    row[[777, 1500]], row[[5, 40, 41]] = 0.0, -0.0
+    draws = ((np.arange(n) + 0.5) / n).astype(np.float32)
+    out = torch.empty(n, dtype=torch.int32, device=DEV)
+    kernels.sample(torch.from_numpy(np.tile(row, (n, 1))).to(DEV), torch.full((n,), 0.7, device=DEV),
+                   torch.full((n,), 2, dtype=torch.int32, device=DEV), torch.from_numpy(draws).to(DEV), out)
+    want = [[5, 40, 41, 777, 1500][int(d * 5)] for d in draws]       # five equal shares, no draw within 1e-3 of a border
+    assert all(abs(d * 5 - round(d * 5)) > 1e-3 for d in draws)
+    assert out.tolist() == want
