@@ -6,8 +6,9 @@
 // denominator, rescaled output).  Tiles start at multiples of 32 counted from key 0,
 // so the order of every sum depends only on the token's own position: the result
 // does not depend on how the prompt was cut or on what else is in the batch.
-// It serves the whole float32 path, and the bfloat16 path for sizes the tensor-core
-// kernels refuse.  Prefill portions and decode tokens take the same code: a portion's
+// It serves the float32 path at the head sizes that attention_f32.cu (where the order of
+// sums depends on the position alone too) refuses, and the bfloat16 path for sizes the
+// tensor-core kernels refuse.  Prefill portions and decode tokens take the same code: a portion's
 // K/V were written to the pages before this kernel runs (gpu_decoder.cu:377-397).
 #include "common.cuh"
 #include <math.h>

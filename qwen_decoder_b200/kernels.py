@@ -650,29 +650,27 @@ def attention_f32_supported(dtype: torch.dtype, H: int, G: int, d: int) -> bool:
 
 
 def attention_f32_splits(n_tokens: int, H: int, G: int, max_keys: int) -> int:
-    """Shares of the keys: two CTAs to a multiprocessor where the (token, kv head) pairs are fewer, no share below 64 keys
-    (two rounds of a CTA's eight warps)."""
+    """CTAs of a cluster per (token, kv head): up to two per multiprocessor, none without a wave of 128 keys.  The result does not
+    depend on it."""
     pairs = n_tokens * G * -(-(H // G) // 8)
-    if pairs > _TICKETS:
-        return 1
-    return max(1, min(2 * sm_count() // max(1, pairs), -(-max_keys // 64), 64))
+    return max(1, min(2 * sm_count() // max(1, pairs), -(-max_keys // 128), 8))
 
 
 def attention_f32(q: torch.Tensor, q_stride: int, out: torch.Tensor, kv: torch.Tensor, block_table: torch.Tensor,
                   token_req: torch.Tensor, positions: torch.Tensor, n_tokens: int, H: int, G: int, d: int, page_size: int,
                   scale: float, window: int, splits: int) -> None:
     """As ``paged_attention_generic``, float32 with a head size of at most 128 in multiples of 4; the keys of a (token, kv
-    head) are shared by ``splits`` CTAs."""
+    head) are shared by the ``splits`` CTAs of a cluster (rounded down to 1, 2, 4 or 8)."""
     assert attention_f32_supported(q.dtype, H, G, d) and kv.dtype == out.dtype == torch.float32
     assert block_table.dtype == torch.int32 and block_table.dim() == 2
     assert token_req.dtype == torch.int32 and positions.dtype == torch.int32
     assert out.shape == (n_tokens, H * d) and tuple(kv.shape[1:]) == (2, G, page_size, d)
     _contig(out, "out"); _contig(kv, "kv"); _contig(block_table, "block_table")
-    part_o, part_ml, tickets = decode_scratch(n_tokens, H, d, G * -(-(H // G) // 8), splits, q.device)
+    ctas = 1 << (min(splits, 8).bit_length() - 1)
     _check(library("attention_f32").qd_attention_f32(
         _ptr(q), _LL(q_stride), _ptr(out), _ptr(kv), _ptr(block_table), _I(block_table.shape[1]), _ptr(token_req),
-        _ptr(positions), _I(n_tokens), _I(H), _I(G), _I(d), _I(page_size), _F(scale), _I(window), _I(splits), _ptr(part_o),
-        _ptr(part_ml), _ptr(tickets), _stream()), "attention_f32")
+        _ptr(positions), _I(n_tokens), _I(H), _I(G), _I(d), _I(page_size), _F(scale), _I(window), _I(ctas), _stream()),
+        "attention_f32")
 
 
 FLASH_HEAD_DIMS = (16, 32, 48, 64, 96, 128)

@@ -84,3 +84,38 @@ def test_attention_f32(cfg, splits):
         qq[p] = q[i, :H * d].double()
         want = plain_model.attention(qq, ks[r][:n].double().reshape(n, G * d), vs[r][:n].double().reshape(n, G * d), H, G, d, window)[p]
         close(out[i], want, torch.float32, scale=float(vs[r][:n].abs().max()))
+
+
+def _attend(q, out, kv, bt, tr, pos, cfg, splits):
+    from qwen_decoder_b200 import kernels
+    H, G, d, page_size, window = cfg
+    kernels.attention_f32(q, q.shape[1], out, kv, bt, tr, pos, q.shape[0], H, G, d, page_size, 1.0 / math.sqrt(d), window or 0, splits)
+
+
+@pytest.mark.parametrize("cfg", [(16, 2, 128, 16, None), (7, 1, 64, 32, None), (6, 3, 20, 8, 1100), (24, 2, 100, 16, 50)])
+def test_attention_f32_token_alone(cfg):
+    """A token's result has the same bits alone and among others, whatever the CTAs of its cluster: contexts of one run, one wave,
+    eight waves, runs of 8, 16 and 24 keys."""
+    H, G, d, page_size, window = cfg
+    lens = [2300, 1, 700]
+    kv, bt, ks, vs = _paged_setup(torch.float32, lens, G, d, page_size, seed=3)
+    items = [(0, p) for p in (0, 7, 8, 127, 128, 1023, 1024, 1500, 2047, 2048, 2299)] + [(1, 0)] + [(2, p) for p in (4, 255, 256, 699)]
+    tr, pos = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in zip(*items))
+    q = torch.empty(len(items), H * d, device=DEV).normal_(generator=torch.Generator(device=DEV).manual_seed(4))
+    kv, bt = kv.to(DEV), bt.to(DEV)
+    want = torch.empty(len(items), H * d, device=DEV)
+    _attend(q, want, kv, bt, tr, pos, cfg, 8)
+    for splits in (1, 2, 4):
+        out = torch.empty_like(want)
+        _attend(q, out, kv, bt, tr, pos, cfg, splits)
+        assert torch.equal(out, want), splits
+    for i in range(len(items)):
+        out = torch.empty(1, H * d, device=DEV)
+        _attend(q[i:i + 1], out, kv, bt, tr[i:i + 1].contiguous(), pos[i:i + 1].contiguous(), cfg, 1 << i % 4)
+        assert torch.equal(out[0], want[i]), items[i]
+    for i, (r, p) in enumerate(items):
+        n = p + 1
+        qq = torch.zeros(n, H * d, dtype=torch.float64)
+        qq[p] = q[i].cpu().double()
+        ref = plain_model.attention(qq, ks[r][:n].double().reshape(n, G * d), vs[r][:n].double().reshape(n, G * d), H, G, d, window)[p]
+        close(want[i], ref, torch.float32, scale=float(vs[r][:n].abs().max()))
