@@ -270,17 +270,22 @@ extern "C" int qd_attention_f32(const float* q, long long q_stride, float* out, 
                                 int max_blocks, const int* token_req, const int* positions, int T, int H, int G, int d,
                                 int page_size, float scale, int window, int ctas, cudaStream_t stream) {
   if (T <= 0) return 0;
-  if (d <= 0 || d > 128 || d % 4 || G <= 0 || H <= 0 || H % G || page_size <= 0 || T > 65535 || q_stride % 4 ||
+  if (d <= 0 || d > 128 || d % 4 || G <= 0 || H <= 0 || H % G || page_size <= 0 || q_stride % 4 ||
       (ctas != 1 && ctas != 2 && ctas != 4 && ctas != 8) || (((uintptr_t)q | (uintptr_t)out | (uintptr_t)kv) & 15))
     return QD_ERR_UNSUPPORTED;
   const int group = H / G, nh = group >= 5 ? 8 : group >= 3 ? 4 : group, blocks = (group + nh - 1) / nh;
   if ((long long)G * blocks > 65535) return QD_ERR_UNSUPPORTED;
-  const dim3 grid(ctas, G * blocks, T);
-  int rc = 0;
+  for (int t0 = 0; t0 < T; t0 += 65535) {            // as many tokens as a grid takes
+    const dim3 grid(ctas, G * blocks, T - t0 < 65535 ? T - t0 : 65535);
+    const float* qt = q + (long long)t0 * q_stride;
+    float* ot = out + (size_t)t0 * H * d;
+    int rc = 0;
 #define AF(NH)                                                                                                              \
-  rc = launch_attention_f32<NH>(grid, stream, q, q_stride, out, kv, block_table, max_blocks, token_req, positions, H, G, d,     \
-                                page_size, scale, window, ctas, blocks)
-  if (nh == 8) AF(8); else if (nh == 4) AF(4); else if (nh == 2) AF(2); else AF(1);
+    rc = launch_attention_f32<NH>(grid, stream, qt, q_stride, ot, kv, block_table, max_blocks, token_req + t0, positions + t0, \
+                                  H, G, d, page_size, scale, window, ctas, blocks)
+    if (nh == 8) AF(8); else if (nh == 4) AF(4); else if (nh == 2) AF(2); else AF(1);
 #undef AF
-  return rc;
+    if (rc) return rc;
+  }
+  return 0;
 }

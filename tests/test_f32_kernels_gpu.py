@@ -119,3 +119,18 @@ def test_attention_f32_token_alone(cfg):
         qq[p] = q[i].cpu().double()
         ref = plain_model.attention(qq, ks[r][:n].double().reshape(n, G * d), vs[r][:n].double().reshape(n, G * d), H, G, d, window)[p]
         close(want[i], ref, torch.float32, scale=float(vs[r][:n].abs().max()))
+
+
+def test_attention_f32_more_tokens_than_a_grid():
+    """65,537 tokens of one head of 4 in one step, as the general kernel takes them."""
+    from qwen_decoder_b200 import kernels
+    T, page_size, cfg = 65537, 16, (1, 1, 4, 16, 24)
+    kv, bt, _, _ = _paged_setup(torch.float32, [64], 1, 4, page_size, seed=5)
+    kv, bt = kv.to(DEV), bt.to(DEV)
+    q = torch.empty(T, 4, device=DEV).normal_(generator=torch.Generator(device=DEV).manual_seed(6))
+    pos = (torch.arange(T, device=DEV) % 64).to(torch.int32)
+    tr = torch.zeros(T, dtype=torch.int32, device=DEV)
+    out, want = torch.empty(T, 4, device=DEV), torch.empty(T, 4, device=DEV)
+    _attend(q, out, kv, bt, tr, pos, cfg, 1)
+    kernels.paged_attention_generic(q, 4, want, kv, bt, tr, pos, T, 1, 1, 4, page_size, 0.5, 24)
+    assert float((out - want).abs().max()) < 2e-6 * float(want.abs().max())
