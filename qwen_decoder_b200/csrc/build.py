@@ -33,7 +33,6 @@ LIBRARIES: Dict[str, str] = {
     "elementwise": "elementwise.cu",
     "gemm_generic": "gemm_generic.cu",
     "gemm_f32": "gemm_f32.cu",
-    "gemm_f32_split": "gemm_f32_split.cu",
     "gemm_skinny": "gemm_skinny.cu",
     "gemm_stream": "gemm_stream.cu",
     "gemm_tc5": "gemm_tc5.cu",
@@ -61,7 +60,7 @@ HEADERS = ["common.cuh", "entry_points.h"]
 # further files a library's source includes (hashed into its key)
 EXTRA_DEPS: Dict[str, List[str]] = {
     "decode_attention_noalloc": ["attention_flash.cu", "decode_attention_noalloc.h"],
-    "gemm_f32_split": ["tc5_ops.cuh"],
+    "gemm_f32": ["tc5_ops.cuh"],
     "gated_block": ["short_conv.cuh"],
     "attention_diff": ["short_conv.cuh", "mma_sync.cuh"],
     "qkv_prep": ["short_conv.cuh"],

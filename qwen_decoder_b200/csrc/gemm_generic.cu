@@ -1,8 +1,10 @@
 // Generic contraction Y[T, N] = X[T, K] * W[N, K]^T (+ bias[N]) on CUDA cores with
-// float32 FMA: any T, N, K.  It is the whole float32 path's matrix product (no
-// TF32, no tensor cores) and the bfloat16 path's fallback for sizes the tensor-core
-// kernels refuse.  Each output element is one FMA chain over k = 0..K-1 in order,
-// so a row's result does not depend on the other rows of the batch.
+// float32 FMA: any T, N, K.  It takes the float32 path's small matrices and what is not
+// in whole 16-byte pieces (gemm_f32.cu has the others: no TF32 there either) and the
+// bfloat16 path's sizes that the tensor-core kernels refuse.  Each output element is one
+// FMA chain over k = 0..K-1 in order, so a row's result does not depend on the other
+// rows of the batch; which of the two takes a product goes by N and K, so neither does a
+// step's.
 //
 // The reference calls cublasHgemm for these products (gpu_kernels.cu:431-436) and
 // adds the bias in a separate kernel (gpu_kernels.cu:70-79).

@@ -261,16 +261,18 @@ def gemm_generic(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
         _I(T), _I(N), _I(K), _LL(x.stride(0)), _LL(out.stride(0)), _stream()), "gemm_generic")
 
 
-F32_FEW_TOKENS = 8         # up to here a float32 product is bound by reading its weights, beyond by the FMA units
+F32_FEW_TOKENS = 64        # up to here the warps that read a float32 product's weights also cut its tokens
+F32_SEGMENT = 448          # tokens of a float32 product that are worked on at once: bounds its scratch memory
 
-
-# Smaller matrices stay with ``gemm_generic``: a few microseconds either way, and there a row's sums do not depend on how many
-# rows there are.
-F32_MIN_WEIGHTS = 1 << 17
+# Smaller matrices stay with ``gemm_generic``: a few microseconds either way; and so do shorter rows, where one FMA chain is at
+# least as close to the exact sum (all terms of one sign with all lower bits set: 64 of k 0.8e-7 root mean square against 1.0e-7,
+# 128 0.96e-7 against 0.98e-7, 256 3.5e-7 against 1.0e-7).  (Which of the two takes a product must not depend on the number of
+# tokens: a token's result would.)
+F32_MIN_WEIGHTS, F32_MIN_K = 1 << 17, 256
 
 
 def gemm_f32_wanted(x: torch.Tensor, w: torch.Tensor) -> bool:
-    return w.numel() > F32_MIN_WEIGHTS and gemm_f32_supported(x, w)
+    return w.numel() > F32_MIN_WEIGHTS and w.shape[1] >= F32_MIN_K and gemm_f32_supported(x, w)
 
 
 def gemm_f32_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -279,38 +281,18 @@ def gemm_f32_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
             and x.stride(1) == 1 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
-def gemm_f32_splits(T: int, N: int, K: int) -> int:
-    """Shares of K of a float32 product of more than 16 tokens: those with which the multiprocessor with the most tiles
-    (128 features x up to 128 tokens x a share of K) is done first, counting what the partial sums cost to write and read
-    again; no share below 128 of K."""
-    if T <= F32_FEW_TOKENS or N % 4:
-        return 1
-    tiles = _f32_tiles(T, N)
-    steps, sms, best = -(-K // 32), sm_count(), None
-    rows = -(-T // tiles[1])
-    for s in range(1, max(1, min(24, steps // 4)) + 1):
-        rounds = -(-tiles[0] * tiles[1] * s // sms)
-        cost = rounds * (-(-steps // s) + 4) * tiles[2] + (s * T * N * 8 / 2048 + 2000 if s > 1 else 0)
-        if best is None or cost < best[0]:
-            best = (cost, s)
-    return best[1]
-
-
-def _f32_tiles(T: int, N: int):
-    """(tiles over N, tiles over T, cycles of a tile's step of 32 k) of the float32 product of ``T`` tokens."""
-    if T <= 64:
-        places = 4 if T <= 32 else 8
-        rows, cols = -(-T // 8) * 8, 1024 // places
-        return -(-N // cols), 1, max(rows * cols * 32 // 128, cols * 9)
-    m_tiles = -(-T // 128)
-    rows = -(-(-(-T // m_tiles)) // 16) * 16
-    return -(-N // 128), -(-T // rows), rows * 32
+def gemm_f32_runs(N: int, K: int) -> int:
+    """Runs of the blocks (128 features x 64 of k) of a float32 product: as many as are needed for the shortest longest run, of two
+    blocks at least, with a multiprocessor to each.  By N and K alone: where a run ends a sum is rounded."""
+    blocks = -(-N // 128) * -(-K // 64)
+    return -(-blocks // max(2, -(-blocks // sm_count())))
 
 
 def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
              splits: Optional[int] = None) -> None:
-    """out[T, N] = x[T, K] @ w[N, K]^T (+ bias), all float32, float32 FMA; x and out may be row-strided.  ``splits``: shares
-    of K (by default ``gemm_f32_splits``)."""
+    """out[T, N] = x[T, K] @ w[N, K]^T (+ bias), all float32, on the tensor cores with both operands cut into three bfloat16 pieces;
+    x and out may be row-strided.  A row's result does not depend on the other rows or on T.  ``splits``: so many equal shares of K
+    to every tile of 128 features, instead of ``gemm_f32_runs``."""
     T, K = x.shape
     N = w.shape[0]
     assert gemm_f32_supported(x, w) and w.shape[1] == K and out.shape == (T, N)
@@ -318,57 +300,19 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out
     _contig(w, "w")
     if bias is not None:
         assert bias.dtype == torch.float32 and bias.numel() == N
-    if splits is None:
-        splits = gemm_f32_splits(T, N, K)
-    part = torch.empty((splits, T, N), dtype=torch.float32, device=x.device) if splits > 1 else None
+    tiles, kb = -(-N // 128), -(-K // 64)
+    runs = gemm_f32_runs(N, K) if splits is None else tiles * splits
+    shares = 1 if tiles * kb % runs == 0 and tiles * kb // runs % kb == 0 else -(-runs // tiles) + 1
+    # (scratch of at most 256 MB, or what 64 tokens need)
+    seg = min(T, max(F32_FEW_TOKENS, min(F32_SEGMENT, (1 << 26) // (shares * N))))
+    pieces = torch.empty((3, seg, kb * 64), dtype=torch.bfloat16, device=x.device) if T > F32_FEW_TOKENS else None
+    part = torch.empty((shares, seg, N), dtype=torch.float32, device=x.device) if shares > 1 else None
     _check(library("gemm_f32").qd_gemm_f32(
-        _ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(part), _I(T), _I(N), _I(K), _LL(x.stride(0)), _LL(out.stride(0)),
-        _I(splits), _stream()), "gemm_f32")
-
-
-# A product of more tokens than this on the tensor cores: at 32 tokens the FMA tiles and they are equal (3B sizes, gate/up 91
-# against 88 us, the output projection 14.1 against 15.5), at 40 105 against 91, at 203 478 against 160.  Smaller matrices than
-# F32_SPLIT_MIN_WEIGHTS stay with the FMA tiles: two launches more.
-F32_SPLIT_TOKENS = 32
-F32_SPLIT_MIN_WEIGHTS = 1 << 20
-
-
-def gemm_f32_split_wanted(T: int, N: int, K: int) -> bool:
-    return T > F32_SPLIT_TOKENS and N * K >= F32_SPLIT_MIN_WEIGHTS
-
-
-def gemm_f32_split_shares(T: int, N: int, K: int) -> int:
-    """Shares of K of a float32 product on the tensor cores: those with which the busiest multiprocessor is done first."""
-    t_tiles = -(-T // 224)
-    cols = -(-(-(-T // t_tiles)) // 32) * 32
-    tiles, blocks, sms, best = -(-N // 128) * t_tiles, -(-K // 64), sm_count(), None
-    for s in range(1, (max(1, min(16, blocks // 2)) if N % 4 == 0 else 1) + 1):
-        # cycles, as measured: a block of 64 k takes 24 a token column (fetching the three pieces of the tokens), at least
-        # 3,500 (reading and cutting W); 4,000 for a tile's beginning and end; partial sums at about 2 KB a cycle for the whole
-        # chip, and a launch
-        cost = -(-tiles * s // sms) * (-(-blocks // s) * max(24 * cols, 3500) + 4000) + (s * T * N * 8 // 2048 + 4000 if s > 1 else 0)
-        if best is None or cost < best[0]:
-            best = (cost, s)
-    return best[1]
-
-
-def gemm_f32_split(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
-                   splits: Optional[int] = None) -> None:
-    """As ``gemm_f32``, on the tensor cores with both operands cut into three bfloat16 pieces that sum to them exactly."""
-    T, K = x.shape
-    N = w.shape[0]
-    assert gemm_f32_supported(x, w) and w.shape[1] == K and out.shape == (T, N)
-    assert out.dtype == torch.float32 and out.stride(1) == 1
-    _contig(w, "w")
-    if bias is not None:
-        assert bias.dtype == torch.float32 and bias.numel() == N
-    if splits is None:
-        splits = gemm_f32_split_shares(T, N, K)
-    pieces = torch.empty((3, T, -(-K // 64) * 64), dtype=torch.bfloat16, device=x.device)
-    part = torch.empty((splits, T, N), dtype=torch.float32, device=x.device) if splits > 1 else None
-    _check(library("gemm_f32_split").qd_gemm_f32_split(
         _ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(pieces), _ptr(part), _I(T), _I(N), _I(K), _LL(x.stride(0)),
-        _LL(out.stride(0)), _I(splits), _stream()), "gemm_f32_split")
+        _LL(out.stride(0)), _I(runs), _I(seg), _stream()), "gemm_f32")
+
+
+gemm_f32_split = gemm_f32
 
 
 SKINNY_MAX_TOKENS = 64      # what the mma.sync few-token kernels take
@@ -827,7 +771,7 @@ def prefill_attention_tc5_status() -> int:
 # library -> (its status function, its wait probe): the kernels with bounded waits on mbarriers or a grid barrier
 _STATUS = {"gemm_stream": ("qd_gemm_stream_status", "qd_gemm_stream_wait_probe"),
            "gemm_tc5": ("qd_gemm_tc5_status", "qd_gemm_tc5_wait_probe"),
-           "gemm_f32_split": ("qd_gemm_f32_split_status", "qd_gemm_f32_split_wait_probe"),
+           "gemm_f32": ("qd_gemm_f32_status", "qd_gemm_f32_wait_probe"),
            "attention_tc5": ("qd_prefill_attention_tc5_status", "qd_prefill_attention_tc5_wait_probe"),
            "attention_flash": ("qd_decode_attention_tma_status", "qd_decode_attention_tma_wait_probe")}
 

@@ -1,8 +1,8 @@
 """Which kernel a contraction runs on.
 
-float32: float32 FMA (``csrc/gemm_f32.cu`` where rows are whole 16-byte pieces, else ``csrc/gemm_generic.cu``) or, for many
-tokens, the tensor cores on operands cut into three bfloat16 pieces that sum to them exactly (``csrc/gemm_f32_split.cu``); no
-TF32 anywhere.
+float32: the tensor cores on operands cut into three bfloat16 pieces that sum to them exactly (``csrc/gemm_f32.cu``), small
+matrices, short rows and rows that are no whole 16-byte pieces float32 FMA (``csrc/gemm_generic.cu``); no TF32 anywhere.  Which of
+the two goes by the matrix, never by the number of tokens, and in neither does a row's result depend on the other rows.
 bfloat16: ``mode`` chooses.
   * ``auto``    few tokens (<= 64): the hand-written weight-streaming tensor-core kernel
                 (``csrc/gemm_skinny.cu``); more tokens: cuBLAS for products large enough to
@@ -55,8 +55,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: 
     if not x.is_cuda:
         raise kernels.KernelError("contractions run on a CUDA device only (there is no CPU path)")
     if x.dtype == torch.float32 and mode != "generic" and kernels.gemm_f32_wanted(x, w) and out.dtype == torch.float32:
-        take = kernels.gemm_f32_split if kernels.gemm_f32_split_wanted(x.shape[0], w.shape[0], x.shape[1]) else kernels.gemm_f32
-        take(x, w, bias, out)
+        kernels.gemm_f32(x, w, bias, out)
         counters["own"] += 1
         return
     if x.dtype == torch.float32 or mode == "generic":

@@ -86,6 +86,59 @@ def test_attention_f32(cfg, splits):
         close(out[i], want, torch.float32, scale=float(vs[r][:n].abs().max()))
 
 
+def _product(x, w, bias=None):
+    from qwen_decoder_b200 import kernels
+    out = torch.empty(x.shape[0], w.shape[0], dtype=torch.float32, device=DEV)
+    kernels.gemm_f32(x, w, bias, out)
+    return out
+
+
+@pytest.mark.parametrize("N,K", [(1000, 2048), (2560, 512), (256, 5504), (20000, 132), (515, 516)])
+def test_gemm_f32_rows_alone(N, K):
+    """A row's result has the same bits whatever the number of rows and wherever the row lies among them: every form for few tokens,
+    tiles of 2, 3 and 4 slots, a second tile, a second segment."""
+    g = torch.Generator(device=DEV).manual_seed(N + K)
+    x = torch.empty(500, K, device=DEV).normal_(generator=g)
+    w = torch.empty(N, K, device=DEV).normal_(0.0, 0.05, generator=g)
+    b = torch.empty(N, device=DEV).normal_(generator=g)
+    want = _product(x, w, b)
+    for first, n in [(0, 1), (499, 1), (3, 16), (5, 17), (100, 33), (7, 48), (1, 64), (2, 65), (250, 129), (11, 203), (0, 224), (40, 225), (13, 449)]:
+        assert torch.equal(_product(x[first:first + n], w, b), want[first:first + n]), (first, n)
+
+
+@pytest.mark.parametrize("kind", ["one", "few", "positive", "low_bits", "normal"])
+@pytest.mark.parametrize("K", [256, 512, 2048])
+@pytest.mark.parametrize("T", [4, 100])
+def test_gemm_f32_error(kind, K, T):
+    """No further from float64 than one float32 FMA chain over k: on rows of which one term carries the result (the chain rounds it
+    once), where no error cancels, and where the lower bits of both operands are all ones.  (Beside the chain's error: the roundings
+    of the smaller sums, 2^-8 of half a unit.)  Three terms: at most two additions that are cut off, less than a unit (2^-23) each,
+    and one rounding of half a unit, of the terms' magnitude."""
+    from qwen_decoder_b200 import kernels
+    g = torch.Generator(device=DEV).manual_seed(K)
+    N = 1024
+    x, w = torch.empty(T, K, device=DEV).normal_(generator=g), torch.empty(N, K, device=DEV).normal_(generator=g)
+    if kind in ("one", "few"):
+        n = 1 if kind == "one" else 3
+        keep = torch.rand(T, K, device=DEV, generator=g).topk(n, dim=1).indices
+        x = torch.zeros_like(x).scatter_(1, keep, x.gather(1, keep))
+    elif kind == "positive":
+        x, w = x.abs(), w.abs()
+    elif kind == "low_bits":
+        x, w = (t.abs().view(torch.int32).bitwise_or(0xFFFF).view(torch.float32) for t in (x, w))
+    want = x.double() @ w.double().t()
+    scale = x.double().abs() @ w.double().abs().t()
+    off = ((_product(x, w).double() - want).abs() / scale)
+    if kind == "few":
+        assert float(off.max()) <= 2.5 * 2.0 ** -23
+        return
+    chain = torch.empty(T, N, dtype=torch.float32, device=DEV)
+    kernels.gemm_generic(x, w, None, chain)
+    ref = (chain.double() - want).abs() / scale
+    assert float(off.max()) <= float(ref.max()) * (1 + 2.0 ** -7), (float(off.max()), float(ref.max()))
+    assert float(off.pow(2).mean()) <= float(ref.pow(2).mean()) * (1 + 2.0 ** -6)
+
+
 def _attend(q, out, kv, bt, tr, pos, cfg, splits):
     from qwen_decoder_b200 import kernels
     H, G, d, page_size, window = cfg
