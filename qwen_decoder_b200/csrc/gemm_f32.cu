@@ -11,7 +11,8 @@
 //
 // A row's sums do not depend on the other rows or on their number.  The blocks of 64 k of all tiles of 128 features are cut into
 // ``runs`` equal runs, one per multiprocessor, by N and K alone; where a run ends inside a tile, the runs' sums of that tile are
-// added up in their order by a kernel of its own.
+// added up in their order by a kernel of its own.  A result that is not finite, or so small that pieces may have left bfloat16's
+// range, is made again as one FMA chain over k, which is what gemm_generic.cu computes.
 //
 // The weights are the MMA's 128 rows, the tokens its columns.  Warps 0-7 cut W (float32) into tiles as the tensor cores read them
 // (K-major, 128-byte swizzle), warp 16 issues TMA loads, warp 17 the MMAs, warps 8-15 add up the blocks' sums (cutting and adding in
@@ -54,6 +55,8 @@ __device__ __forceinline__ void cut3(float x, float y, unsigned& p1, unsigned& p
   p3 = round2(xr - __uint_as_float(p2 << 16), yr - __uint_as_float(p2 & 0xFFFF0000u));
 }
 
+__device__ __forceinline__ bool fs_doubtful(float s) { return !(fabsf(s) >= 0x1p-80f && fabsf(s) <= 3.4e38f) && s != 0.f; }
+
 struct FsArgs {
   const float* X; const float* W; const float* bias; float* Y; float* part;      // part [shares, T, N]
   long long ldx, ldy;
@@ -61,6 +64,17 @@ struct FsArgs {
   int t_tiles, t_rows, n_cols;                       // the second form: tiles of tokens, MMA columns (t_rows in whole 16)
   int* status;
 };
+
+// A result (bias included) that pieces cannot be trusted with is the FMA chain's.  (A row of zeros stays as it is.)
+__device__ __noinline__ void fs_chain(const float* x, const float* w, int K, const float* bias, float* y) {
+  if (!fs_doubtful(*y)) return;
+  float s = 0.f;
+  for (int k = 0; k < K; k++) s = fmaf(x[k], w[k], s);
+  *y = bias ? s + *bias : s;
+}
+__device__ __forceinline__ void fs_settle(const FsArgs& a, int t, int n, float* y) {
+  fs_chain(a.X + (size_t)t * a.ldx, a.W + (size_t)n * a.K, a.K, a.bias ? a.bias + n : nullptr, y);
+}
 
 // the run that has block b
 __host__ __device__ __forceinline__ int fs_run_of(long long b, int runs, int total) { return (int)(((b + 1) * runs + total - 1) / total) - 1; }
@@ -100,7 +114,8 @@ __device__ __forceinline__ int fs_blocks(const FsArgs& a) {
   return n * a.t_tiles;
 }
 
-// Stores a thread's sums of feature n, tokens t0 .. t_end - 1, and sets them to zero.
+// Stores a thread's sums of feature n, tokens t0 .. t_end - 1, and sets them to zero.  (What is doubtful is looked for once all are
+// stored: this code is unrolled, runs once a tile and comes from memory, 10 us of it when it held the chain's call.)
 template <int M>
 __device__ __forceinline__ void fs_store(const FsArgs& a, int run, int tile, int n, int t0, int t_end, float (&sum)[M]) {
   long long ld;
@@ -112,13 +127,19 @@ __device__ __forceinline__ void fs_store(const FsArgs& a, int run, int tile, int
 #pragma unroll
     for (int c = 0; c < M; c++) sum[c] += b;
   }
+  bool doubtful = false;
   float* p = o + t0 * ld;
 #pragma unroll
   for (int c = 0; c < M; c++) {
-    if (in && t0 + c < t_end) *p = sum[c];
+    if (in && t0 + c < t_end) {
+      *p = sum[c];
+      doubtful = doubtful || fs_doubtful(sum[c]);
+    }
     p += ld;
     sum[c] = 0.f;
   }
+  if (doubtful && whole)
+    for (int t = t0; t < min(t0 + M, t_end); t++) fs_settle(a, t, n, o + t * ld);
 }
 
 // the product of two pieces over a block of k, by one thread: 4 MMAs into ``nt`` columns at d
@@ -547,8 +568,15 @@ f32_runs_kernel(const FsArgs a) {
       const int t = t0 + 8 * r;
       if (t >= a.T) continue;
       float* y = a.Y + t * a.ldy + n;
+      bool doubtful = false;
 #pragma unroll
-      for (int u = 0; u < V; u++) y[u] = a.bias ? s[r][u] + a.bias[n + u] : s[r][u];
+      for (int u = 0; u < V; u++) {
+        const float q = a.bias ? s[r][u] + a.bias[n + u] : s[r][u];
+        y[u] = q;
+        doubtful = doubtful || fs_doubtful(q);
+      }
+      if (doubtful)
+        for (int u = 0; u < V; u++) fs_settle(a, t, n + u, y + u);
     }
   }
 }

@@ -139,6 +139,39 @@ def test_gemm_f32_error(kind, K, T):
     assert float(off.pow(2).mean()) <= float(ref.pow(2).mean()) * (1 + 2.0 ** -6)
 
 
+@pytest.mark.parametrize("T", [1, 5, 40, 64, 203, 300])
+@pytest.mark.parametrize("N,K", [(256, 516), (1000, 1024)])
+def test_gemm_f32_ends_of_the_range(T, N, K):
+    """Infinities, NaN, numbers that bfloat16 would round to infinity and numbers below its range: what the FMA chain gives, bit for
+    bit (NaN for NaN), in the rows and columns that have them; the other results stay as they are."""
+    from qwen_decoder_b200 import kernels
+    inf, big, tiny = float("inf"), 3.4e38, 3e-37
+    g = torch.Generator(device=DEV).manual_seed(T)
+    x, w = torch.empty(T, K, device=DEV).normal_(generator=g), torch.empty(N, K, device=DEV).normal_(0.0, 0.05, generator=g)
+    b = torch.empty(N, device=DEV).normal_(generator=g)
+    w[:, 9] = 0.0
+    w[5, 9], w[6, 100], w[7, 3] = 2.0, -inf, float("nan")
+    plain = _product(x, w, b)
+    rows = {0: (inf, 2), T // 2: (-inf, 9), T - 1: (big, 9)}
+    for r, (v, k) in rows.items():
+        x[r, k] = v
+    for bias in (b, None):
+        got, chain = _product(x, w, bias), torch.empty(T, N, dtype=torch.float32, device=DEV)
+        kernels.gemm_generic(x, w, bias, chain)
+        odd = ~chain.isfinite()
+        assert bool(odd.any()) and torch.equal(got.isnan(), chain.isnan())
+        assert torch.equal(got[odd].nan_to_num(0.0, inf, -inf), chain[odd].nan_to_num(0.0, inf, -inf))
+        assert float((got - chain)[~odd].abs().max()) < 1e-5 * float(chain[~odd].abs().max())
+    if T > 3:
+        others = [r for r in range(T) if r not in rows]
+        assert torch.equal(_product(x, w, b)[others].nan_to_num(7.0), plain[others].nan_to_num(7.0))
+    x = torch.empty(T, K, device=DEV).normal_(generator=g) * tiny
+    chain = torch.empty(T, N, dtype=torch.float32, device=DEV)
+    w[6:8] = 0.01
+    kernels.gemm_generic(x, w, None, chain)
+    assert torch.equal(_product(x, w), chain)
+
+
 def _attend(q, out, kv, bt, tr, pos, cfg, splits):
     from qwen_decoder_b200 import kernels
     H, G, d, page_size, window = cfg
