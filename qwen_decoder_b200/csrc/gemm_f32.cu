@@ -17,13 +17,14 @@
 // The weights are the MMA's 128 rows, the tokens its columns.  Warps 0-7 cut W (float32) into tiles as the tensor cores read them
 // (K-major, 128-byte swizzle), warp 16 issues TMA loads, warp 17 the MMAs, warps 8-15 add up the blocks' sums (cutting and adding in
 // the same warps took turns: 2,500 cycles a block at 4 tokens, of which 1,300 were the sums').  Two forms:
-//  * up to 64 tokens, bound by shared memory (of the 2,000 cycles of a block at 4 tokens the MMAs' reads of W's pieces take 1,000, W
-//    itself, in and out, 500, its pieces 400): W comes by TMA, the first blocks before the wait for the kernel before; warps 0-7 read
-//    and cut the tokens too.
+//  * up to 64 tokens, bound by reading W (the projection over the vocabulary at 5.5 TB/s) and by ramps and tails where a run is short:
+//    W comes by TMA, the first blocks before the wait for the kernel before; its pieces go to tensor memory, from where the MMAs take
+//    them (in shared memory their 32 reads of a piece's 4 KB, the stores and W itself took 2,000 cycles a block: gate and up 48 us
+//    at 4 tokens, now 40); warps 0-7 read and cut the tokens too.
 //  * more tokens: W is read by warps 0-7, the tokens' pieces are made by a kernel beforehand and come by TMA, a piece a slot; bound by
 //    shared memory too (203 tokens: 3,300 cycles of MMAs a block, 4,200 of reads and writes, 5,100 taken).
-// Measured on a B200 at the 3B sizes, us a product, at 4 / 64 / 203 tokens: gate and up 48 / 60 / 127, output projection 9.3 / 13 / 27,
-// all products of a step 3,720 at 4 tokens, 9,800 at 203.  With kernels and shares of K chosen by the number of tokens, and six products
+// Measured on a B200 at the 3B sizes, us a product, at 4 / 64 / 203 tokens: gate and up 40 / 55 / 129, output projection 8.6 / 13 / 27,
+// all products of a step 3,200 at 4 tokens, 9,800 at 203.  With kernels and shares of K chosen by the number of tokens, and six products
 // of pieces that were cut off, they had been 34 / 96 / 165 and 4.9 / 17 / 27: the smallest steps pay for sums that do not go by the
 // batch.  Error against float64 1.2e-7 (gate and up; the FMA tiles of 9 to 32 tokens: 3.3e-7).
 // Every wait is bounded; after one has run out nothing new is asked for and what is in flight is waited for.
@@ -142,11 +143,17 @@ __device__ __forceinline__ void fs_store(const FsArgs& a, int run, int tile, int
     for (int t = t0; t < min(t0 + M, t_end); t++) fs_settle(a, t, n, o + t * ld);
 }
 
-// the product of two pieces over a block of k, by one thread: 4 MMAs into ``nt`` columns at d
+// the product of two pieces over a block of k, by one thread: 4 MMAs into the columns at d; W's piece in shared memory or in
+// tensor memory (the same sums)
 __device__ __forceinline__ void fs_product(unsigned d, unsigned long long w, unsigned long long x, unsigned idesc, bool fresh) {
   tc_mma_bf16(d, w, x, idesc, !fresh);
 #pragma unroll
   for (int k = 1; k < FS_BK / 16; k++) tc_mma_bf16(d, w + 2 * k, x + 2 * k, idesc, true);
+}
+__device__ __forceinline__ void fs_product(unsigned d, unsigned w, unsigned long long x, unsigned idesc, bool fresh) {
+  tc_mma_bf16_tmem(d, w, x, idesc, !fresh);
+#pragma unroll
+  for (int k = 1; k < FS_BK / 16; k++) tc_mma_bf16_tmem(d, w + 8 * k, x + 2 * k, idesc, true);
 }
 // What the small products' sum consists of, in this order in both forms, and then x1 w2, x1 w3 (P: from one piece of W to the next)
 #define FS_WITH_X2(small, w, x, idesc, fresh) \
@@ -198,21 +205,21 @@ __device__ __forceinline__ void fs_end(volatile int& dead, int warp, int lane, u
 }
 
 // ---------------------------------------------------------------------------------------------- up to 64 tokens
-// NT tokens (a multiple of 16); F blocks of W as they are (float32) on their way or in use, two blocks of pieces, each with its own
-// NT columns for the large products' sum
+// NT tokens (a multiple of 16); F blocks of W as they are (float32) on their way or in use, two blocks of pieces (W's in tensor
+// memory, 32 columns each, the tokens' in shared memory), each with its own NT columns for the large products' sum
 template <int NT, int F>
 __global__ void __launch_bounds__(FS_THREADS, 1)
 gemm_f32_few_kernel(const __grid_constant__ CUtensorMap map_w, const FsArgs a) {
-  constexpr int HALF = NT / 2, XP = NT / 16, XPIECE = NT * 128, STAGE = FS_WBLOCK + 3 * XPIECE, RAW = 128 * FS_BK * 4;
-  constexpr unsigned COLS = 3 * NT <= 64 ? 64 : 3 * NT <= 128 ? 128 : 256, P = FS_WPIECE >> 4;
-  static_assert(NT % 16 == 0 && STAGE % 1024 == 0 && 3 * NT <= 256, "");
+  constexpr int HALF = NT / 2, XP = NT / 16, XPIECE = NT * 128, RAW = 128 * FS_BK * 4;
+  constexpr unsigned P = FS_BK / 2, COLS = 6 * P + 3 * NT <= 256 ? 256 : 512;
+  static_assert(NT % 16 == 0 && 6 * P + 3 * NT <= 512, "");
   extern __shared__ unsigned char smem_raw[];
   __shared__ unsigned long long raw_full[F], raw_free[F], full[2], done[2], part_read;
   __shared__ unsigned tmem_slot;
   __shared__ int dead;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned char* ring = smem_raw + ((1024 - (tc_smem(smem_raw) & 1023)) & 1023);       // [2][W's pieces, the tokens' pieces]
-  unsigned char* raw = ring + 2 * STAGE;                                               // [F][128 rows][64 floats]
+  unsigned char* raw = smem_raw + ((1024 - (tc_smem(smem_raw) & 1023)) & 1023);        // [F][2 halves of k][128 rows][32 floats, swizzled]
+  unsigned char* ring = raw + F * RAW;                                                 // [2][3 pieces][tokens][128 bytes]
   if (threadIdx.x == 0) {
     dead = 0;
     // a block's pieces are there (warps 0-7) and the sums that lay in its columns are read (warps 8-15): one wait for the MMA warp,
@@ -229,6 +236,7 @@ gemm_f32_few_kernel(const __grid_constant__ CUtensorMap map_w, const FsArgs a) {
     const unsigned r = asked % F;
     tc_expect_tx(&raw_full[r], RAW);
     tc_load_2d(raw + r * RAW, &map_w, at.k * FS_BK, at.tile * 128, &raw_full[r]);
+    tc_load_2d(raw + r * RAW + RAW / 2, &map_w, at.k * FS_BK + FS_BK / 2, at.tile * 128, &raw_full[r]);
     at.next(a);
     asked++;
   };
@@ -240,22 +248,23 @@ gemm_f32_few_kernel(const __grid_constant__ CUtensorMap map_w, const FsArgs a) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const unsigned tmem = tmem_slot, small = tmem + 2 * NT;
+  const unsigned tmem = tmem_slot, main = tmem + 6 * P, small = main + 2 * NT;
   pdl_launch_dependents();
   if (warp < 8) {
     // ------------------------------------------------------------------ cut, store
-    const int row = threadIdx.x >> 4, chunk = threadIdx.x & 15;      // rows row + 16 j, floats 4 chunk .. + 3 of a block
-    const unsigned at = row * 128 + (((chunk >> 1) ^ (row & 7)) << 4) + (chunk & 1) * 8;
+    const int quarter = warp & 3, half = warp >> 2, w_row = quarter * 32 + lane;       // of W: a row, half of the block's k
+    const unsigned w_to = tmem + ((unsigned)quarter << 21) + half * (P / 2);
+    const int row = threadIdx.x >> 4, chunk = threadIdx.x & 15;      // of the tokens: rows row + 16 j, floats 4 chunk .. + 3
+    const unsigned at_x = row * 128 + (((chunk >> 1) ^ (row & 7)) << 4) + (chunk & 1) * 8;
     float4 x[XP];
-    FsAt ask(a);                                     // the block whose tokens are asked for next
     auto ask_x = [&]() {
-      const int k = ask.k * FS_BK + chunk * 4;
+      const int k = at.k * FS_BK + chunk * 4;
 #pragma unroll
       for (int j = 0; j < XP; j++) {
         const int t = row + 16 * j;
         x[j] = k < a.K && t < a.T ? __ldg(reinterpret_cast<const float4*>(a.X + (size_t)t * a.ldx + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      ask.next(a);
+      at.next(a);
     };
     pdl_wait();
     ask_x();
@@ -263,16 +272,29 @@ gemm_f32_few_kernel(const __grid_constant__ CUtensorMap map_w, const FsArgs a) {
       const int s = g & 1;
       if (!tc_wait(&raw_full[r], ph, &dead) && lane == 0) atomicExch(a.status, 1);
       float4 w[8];
-      const float4* from = reinterpret_cast<const float4*>(raw + r * RAW) + threadIdx.x;
 #pragma unroll
-      for (int j = 0; j < 8; j++) w[j] = from[256 * j];
+      for (int j = 0; j < 8; j++)
+        w[j] = *reinterpret_cast<const float4*>(raw + r * RAW + half * (RAW / 2) + w_row * 128 + ((j ^ (w_row & 7)) << 4));
       if (!tc_wait(&done[s], ((g >> 1) & 1) ^ 1, &dead) && lane == 0) atomicExch(a.status, 2);       // the stage is free
-      unsigned char* dst = ring + s * STAGE + at;
+      tc_fence_after();
 #pragma unroll
-      for (int j = 0; j < 8; j++) fs_put(dst + j * 2048, FS_WPIECE, w[j]);
+      for (int j = 0; j < XP; j++) fs_put(ring + s * 3 * XPIECE + at_x + j * 2048, XPIECE, x[j]);
 #pragma unroll
-      for (int j = 0; j < XP; j++) fs_put(dst + FS_WBLOCK + j * 2048, XPIECE, x[j]);
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // read by the tensor cores; the slot is written by TMA next
+      for (int j = 0; j < 8; j += 4) {               // 16 floats: 8 columns of each piece
+        unsigned p1[8], p2[8], p3[8];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          cut3(w[j + i].x, w[j + i].y, p1[2 * i], p2[2 * i], p3[2 * i]);
+          cut3(w[j + i].z, w[j + i].w, p1[2 * i + 1], p2[2 * i + 1], p3[2 * i + 1]);
+        }
+        __syncwarp();
+        tc_st8(w_to + s * 3 * P + 2 * j, p1);
+        tc_st8(w_to + s * 3 * P + P + 2 * j, p2);
+        tc_st8(w_to + s * 3 * P + 2 * P + 2 * j, p3);
+      }
+      tc_st_wait();
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tokens are read by the tensor cores
+      tc_fence_before();
       __syncwarp();
       if (lane == 0) { tc_arrive(&full[s]); tc_arrive(&raw_free[r]); }
       if (++r == F) { r = 0; ph ^= 1; }
@@ -293,7 +315,7 @@ gemm_f32_few_kernel(const __grid_constant__ CUtensorMap map_w, const FsArgs a) {
       tc_fence_after();
       const bool end = at.ends_part(a);
 #pragma unroll
-      for (int c = 0; c < HALF; c += 8) fs_add8(tmem + s * NT + mine + c, sum + c);
+      for (int c = 0; c < HALF; c += 8) fs_add8(main + s * NT + mine + c, sum + c);
       if (end) {
 #pragma unroll
         for (int c = 0; c < HALF; c += 8) fs_add8(small + mine + c, sum + c);
@@ -313,7 +335,7 @@ gemm_f32_few_kernel(const __grid_constant__ CUtensorMap map_w, const FsArgs a) {
       }
   } else if (warp == FS_MMA_WARP) {
     const unsigned idesc = tc_idesc_bf16(128, NT);
-    const unsigned long long d0 = tc_desc_sw128(tc_smem(ring));
+    const unsigned long long x0 = tc_desc_sw128(tc_smem(ring));
     const bool one = tc_elect();
     bool first = true;                               // of a part: the small products' sum begins anew
     unsigned parts = 0;
@@ -326,13 +348,14 @@ gemm_f32_few_kernel(const __grid_constant__ CUtensorMap map_w, const FsArgs a) {
       }
       tc_fence_after();
       __syncwarp();
-      const unsigned long long w = d0 + s * (STAGE >> 4), x = w + (FS_WBLOCK >> 4);
+      const unsigned w = tmem + s * 3 * P;
+      const unsigned long long x = x0 + s * (3 * XPIECE >> 4);
       if (one) {
         FS_WITH_X2(small, w, x + (XPIECE >> 4), idesc, first);
         FS_WITH_X3(small, w, x + 2 * (XPIECE >> 4), idesc);
         fs_product(small, w + P, x, idesc, false);
         fs_product(small, w + 2 * P, x, idesc, false);
-        fs_product(tmem + s * NT, w, x, idesc, true);
+        fs_product(main + s * NT, w, x, idesc, true);
         tc_commit(&done[s]);
       }
       first = at.ends_part(a);
@@ -609,7 +632,7 @@ static int fs_sms() {
 
 template <int NT, int F>
 static int launch_few(const FsArgs& a, int grid, cudaStream_t stream) {
-  constexpr int smem = 2 * (FS_WBLOCK + 3 * NT * 128) + F * 128 * FS_BK * 4 + 1024;
+  constexpr int smem = 2 * 3 * NT * 128 + F * 128 * FS_BK * 4 + 1024;
   CUtensorMap map;
   if (!tc_make_map(&map, a.W, false, a.N, a.K, 128)) return QD_ERR_UNSUPPORTED;
   const cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<NT, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -618,10 +641,9 @@ static int launch_few(const FsArgs& a, int grid, cudaStream_t stream) {
   return qd_last_error();
 }
 static int fs_few(const FsArgs& a, int grid, cudaStream_t stream) {
-  if (a.T <= 16) return launch_few<16, 3>(a, grid, stream);
-  if (a.T <= 32) return launch_few<32, 3>(a, grid, stream);
-  if (a.T <= 48) return launch_few<48, 2>(a, grid, stream);
-  return launch_few<64, 2>(a, grid, stream);
+  if (a.T <= 16) return launch_few<16, 5>(a, grid, stream);
+  if (a.T <= 32) return launch_few<32, 5>(a, grid, stream);
+  return launch_few<64, 4>(a, grid, stream);
 }
 
 template <int NT>

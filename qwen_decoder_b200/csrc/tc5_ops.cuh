@@ -20,7 +20,7 @@ __device__ __forceinline__ bool tc_wait(unsigned long long* bar, unsigned parity
                                         unsigned polls = TC_POLLS) {
   return qd_mbar_wait_bounded(tc_smem(bar), parity, dead, polls, 2000000000ull, backoff_ns);
 }
-// x: innermost coordinate in elements (a multiple of 64 here: 128 or 256 bytes), y: row
+// x: innermost coordinate in elements (of whole 128 bytes here), y: row
 __device__ __forceinline__ void tc_load_2d(void* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                ::"r"(tc_smem(dst)), "l"(map), "r"(tc_smem(bar)), "r"(x), "r"(y) : "memory");
@@ -38,6 +38,13 @@ __device__ __forceinline__ void tc_mma_bf16(unsigned d, unsigned long long a, un
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}\n"
       ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate ? 1u : 0u), "r"(0u) : "memory");
+}
+// the same with A in tensor memory: 128 lanes, two neighbouring k a column
+__device__ __forceinline__ void tc_mma_bf16_tmem(unsigned d, unsigned a, unsigned long long b, unsigned idesc, bool accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n}\n"
+      ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate ? 1u : 0u), "r"(0u) : "memory");
 }
 // true for one lane of a whole warp
 __device__ __forceinline__ bool tc_elect() {
@@ -60,6 +67,11 @@ __device__ __forceinline__ void tc_ld8(unsigned addr, unsigned (&v)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(addr));
 }
+__device__ __forceinline__ void tc_st8(unsigned addr, const unsigned (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n"
+               ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+__device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -78,15 +90,15 @@ static TcEncodeFn tc_encode_fn() {
   }
   return fn;
 }
-// rows x cols, contiguous; boxes of box_rows x 64 columns, zeros outside: bfloat16 with the 128-byte swizzle, or float32 as it lies
+// rows x cols bfloat16 or float32, contiguous; boxes of box_rows rows of 128 bytes, 128-byte swizzle, zeros outside
 static bool tc_make_map(CUtensorMap* map, const void* base, bool bfloat16, long long rows, long long cols, int box_rows) {
   TcEncodeFn fn = tc_encode_fn();
   if (!fn) return false;
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)cols * (bfloat16 ? 2 : 4)};
-  cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
+  cuuint32_t box[2] = {bfloat16 ? 64u : 32u, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   return fn(map, bfloat16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims,
-            strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, bfloat16 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+            strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
