@@ -1,4 +1,4 @@
-// tcgen05, tensor memory, TMA and mbarrier operations as the kernels that stream bfloat16 tiles use them.
+// tcgen05, tensor memory, TMA and mbarrier operations of gemm_f32.cu: operands of rows of 128 bytes, 128-byte swizzle.
 #pragma once
 #include "common.cuh"
 #include <cuda.h>

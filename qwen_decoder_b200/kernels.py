@@ -310,9 +310,12 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out
     _check(library("gemm_f32").qd_gemm_f32(
         _ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(pieces), _ptr(part), _I(T), _I(N), _I(K), _LL(x.stride(0)),
         _LL(out.stride(0)), _I(runs), _I(seg), _stream()), "gemm_f32")
+    # a segment: the tokens' pieces (more than 64 tokens), the product, the sums over runs
+    segments = [min(seg, T - t) for t in range(0, T, seg)] if T else [0]
+    _launch_count[0] += sum(1 + (n > F32_FEW_TOKENS) + (part is not None) for n in segments) - 1
 
 
-gemm_f32_split = gemm_f32
+gemm_f32_split = gemm_f32      # the name that products of more tokens had
 
 
 SKINNY_MAX_TOKENS = 64      # what the mma.sync few-token kernels take

@@ -220,3 +220,34 @@ def test_attention_f32_more_tokens_than_a_grid():
     _attend(q, out, kv, bt, tr, pos, cfg, 1)
     kernels.paged_attention_generic(q, 4, want, kv, bt, tr, pos, T, 1, 1, 4, page_size, 0.5, 24)
     assert float((out - want).abs().max()) < 2e-6 * float(want.abs().max())
+
+
+def test_f32_step_token_alone(tmp_path):
+    """Logits of the float32 engine, with matrices that ``gemm_f32`` takes, bit for bit: a prompt in one step, cut in several ways
+    (down to single tokens, replayed as a captured step), beside other requests."""
+    from qwen_decoder_b200.config import Qwen2Config
+    from qwen_decoder_b200.engine import ModelRunner, StepEntry
+    from qwen_decoder_b200.weights import write_random_model
+    cfg = {"architectures": ["Qwen2ForCausalLM"], "hidden_size": 512, "intermediate_size": 1280, "num_hidden_layers": 2,
+           "num_attention_heads": 8, "num_key_value_heads": 2, "vocab_size": 1000, "max_position_embeddings": 512,
+           "rope_theta": 10000.0, "rms_norm_eps": 1e-6, "tie_word_embeddings": False}
+    folder = write_random_model(Qwen2Config.from_dict(cfg), str(tmp_path), 4, dtype=torch.float32, std=0.08)
+    runner = ModelRunner.from_folder(folder, dtype="float32", device=DEV, num_pages=64)
+    g = torch.Generator().manual_seed(7)
+    tokens = torch.randint(0, 1000, (150,), generator=g).tolist()
+
+    def run(cuts, beside=()):
+        rc, others, at, got = runner.open("it"), [runner.open(f"o{i}") for i in range(len(beside))], 0, []
+        for n in cuts:
+            entries = [StepEntry(rc, tokens[at:at + n], list(range(n)))]
+            entries += [StepEntry(o, torch.randint(0, 1000, (k,), generator=g).tolist(), [k - 1]) for o, k in zip(others, beside)]
+            got.append(runner.step(entries)[:n].clone())
+            at += n
+        for r in [rc] + others:
+            runner.close(r)
+        return torch.cat(got)
+
+    want = run([150])
+    assert bool(want.isfinite().all())
+    for cuts, beside in [([1, 16, 17, 48, 68], ()), ([75, 75], (3, 20)), ([149, 1], (1, 1, 64)), ([140] + [1] * 10, ()), ([140] + [1] * 10, (1,) * 7)]:
+        assert torch.equal(run(cuts, beside), want), (cuts, beside)
