@@ -11,8 +11,9 @@
 //
 // A row's sums do not depend on the other rows or on their number.  The blocks of 64 k of all tiles of 128 features are cut into
 // ``runs`` equal runs, one per multiprocessor, by N and K alone; where a run ends inside a tile, the runs' sums of that tile are
-// added up in their order by a kernel of its own.  A result that is not finite, or so small that pieces may have left bfloat16's
-// range, is made again as one FMA chain over k, which is what gemm_generic.cu computes.
+// added up in their order by a kernel of its own.  A result that is not finite, or so small (2^-80) that pieces may have left
+// bfloat16's range, is made again as one FMA chain over k, which is what gemm_generic.cu computes.  (What that does not see: a row
+// whose terms are all a number below 2^-109 times one above 2^29; the lost bits are worth 2^-134 of the latter each.)
 //
 // The weights are the MMA's 128 rows, the tokens its columns.  Warps 0-7 cut W (float32) into tiles as the tensor cores read them
 // (K-major, 128-byte swizzle), warp 16 issues TMA loads, warp 17 the MMAs, warps 8-15 add up the blocks' sums (cutting and adding in

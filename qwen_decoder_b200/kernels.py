@@ -264,10 +264,11 @@ def gemm_generic(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor],
 F32_FEW_TOKENS = 64        # up to here the warps that read a float32 product's weights also cut its tokens
 F32_SEGMENT = 448          # tokens of a float32 product that are worked on at once: bounds its scratch memory
 
-# Smaller matrices stay with ``gemm_generic``: a few microseconds either way; and so do shorter rows, where one FMA chain is at
-# least as close to the exact sum (all terms of one sign with all lower bits set: 64 of k 0.8e-7 root mean square against 1.0e-7,
-# 128 0.96e-7 against 0.98e-7, 256 3.5e-7 against 1.0e-7).  (Which of the two takes a product must not depend on the number of
-# tokens: a token's result would.)
+# Smaller matrices (routers, gates, small models) stay with ``gemm_generic``, whose results they had before there was another kernel;
+# it is not the faster one there (256 x 512 at 4 / 203 tokens 35 / 39 us, ``gemm_f32`` 5 / 18).  So do shorter rows, where one FMA
+# chain is at least as close to the exact sum (all terms of one sign with all lower bits set: 64 of k 0.8e-7 root mean square
+# against 1.0e-7, 128 0.96e-7 against 0.98e-7, 256 3.5e-7 against 1.0e-7).  (Which of the two takes a product must not depend on the
+# number of tokens: a token's result would.)
 F32_MIN_WEIGHTS, F32_MIN_K = 1 << 17, 256
 
 

@@ -251,3 +251,16 @@ def test_f32_step_token_alone(tmp_path):
     assert bool(want.isfinite().all())
     for cuts, beside in [([1, 16, 17, 48, 68], ()), ([75, 75], (3, 20)), ([149, 1], (1, 1, 64)), ([140] + [1] * 10, ()), ([140] + [1] * 10, (1,) * 7)]:
         assert torch.equal(run(cuts, beside), want), (cuts, beside)
+
+
+def test_gemm_f32_wait_that_runs_out_is_reported_once():
+    """The library's own bounded wait, on an mbarrier nobody arrives at, with a limit of a few thousand polls; products go on."""
+    from qwen_decoder_b200 import kernels
+    kernels.check_status()
+    kernels.wait_probe("gemm_f32", 4096)
+    torch.cuda.synchronize()
+    with pytest.raises(kernels.KernelError, match="gemm_f32"):
+        kernels.check_status()
+    kernels.check_status()
+    x, w = torch.ones(3, 512, device=DEV), torch.ones(300, 512, device=DEV)
+    assert bool((_product(x, w) == 512.0).all())
