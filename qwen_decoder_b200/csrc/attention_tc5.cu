@@ -199,7 +199,7 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap kv_map, const A
   // Slot i (i = -2 .. n_kt - 1, stage (i + 2) % NS) holds K of tile i + 2 and V of tile i, the two tiles the MMA
   // thread reads in its step i, under one pair of barriers: each wait of that one thread is time in which no
   // MMA is issued.  Both producers arrive at kv_full (with their bytes, or bare where a slot lacks their tile).
-  __shared__ unsigned long long kv_full[NS], kv_empty[NS], s_full[2], p_full[2], o_done, q_full;
+  __shared__ unsigned long long kv_full[NS], kv_empty[NS], s_full[2], p_full[2], o_done, o_last, q_full;
   __shared__ float mx_s[2][TPR][AT_ROWS];           // [tile parity][share of the keys][row]: the shares' maxima
   __shared__ float l_s[TPR][AT_ROWS];               // the shares' sums, at the end
   __shared__ unsigned tmem_slot;
@@ -212,7 +212,11 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap kv_map, const A
     dead = 0;
     for (int s = 0; s < NS; s++) { at_mbar_init(&kv_full[s], 2); at_mbar_init(&kv_empty[s], 1); }
     for (int s = 0; s < 2; s++) at_mbar_init(&s_full[s], 1);
-    at_mbar_init(&o_done, 1);
+    // o_done: a product but the last is complete.  Who waits for product j - 1 has the scores of tile j, so product j - 2 is
+    // complete and the parity says which of two phases it is.  The last product has no scores behind it: after the last tile the
+    // product before it may still be under way, whose phase has the other parity, and a wait on o_done would pass at once
+    // (rows of two key tiles or more whose last V came late were stored without them).  It has a barrier of its own.
+    at_mbar_init(&o_done, 1); at_mbar_init(&o_last, 1);
     // P of tile j + 1 may be ready before the MMA thread has looked at tile j's barrier (the softmax threads
     // hand P over before they wait for the product of the tile before): two barriers, used in turn
     at_mbar_init(&p_full[0], AT_SOFTMAX_THREADS); at_mbar_init(&p_full[1], AT_SOFTMAX_THREADS);
@@ -356,7 +360,7 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap kv_map, const A
                       idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
         }
         if (mstamp) p.timeline[128 + j * 4 + 2] = at_now();
-        at_commit(&o_done);
+        at_commit(j + 1 < n_kt ? &o_done : &o_last);
         if (j + 2 < n_kt) scores(j + 2);
         at_commit(&kv_empty[s]);
         if (j + 2 < n_kt) at_commit(&s_full[j & 1]);
@@ -472,7 +476,7 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap kv_map, const A
     }
     if (n_kt > 0) {
       if (stamp) p.timeline[32 + 7] = at_now();
-      if (!at_mbar_wait(&o_done, (n_kt - 1) & 1, &dead) && lane == 0) atomicCAS(p.status, 0, 9);
+      if (!at_mbar_wait(&o_last, 0, &dead) && lane == 0) atomicCAS(p.status, 0, 9);
       if (stamp) p.timeline[40 + 7] = at_now();
       at_fence_after();
     }
