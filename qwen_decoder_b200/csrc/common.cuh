@@ -110,9 +110,9 @@ static inline void qd_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
 // waiter sets ``*dead`` (no wait of its CTA spins again), the caller records which wait it was in the
 // library's status word, and the kernel runs on to its end with void results: the host reads the
 // status word (qd_<library>_status) and raises.  A kernel never hangs on a copy that did not arrive.
-__device__ __forceinline__ bool qd_mbar_wait_bounded(unsigned bar_smem_addr, unsigned parity, volatile int* dead,
-                                                     unsigned poll_limit, unsigned long long time_limit_ns,
-                                                     unsigned backoff_ns = 0) {
+__device__ __forceinline__ bool qd_mbar_wait_loop(unsigned bar_smem_addr, unsigned parity, volatile int* dead,
+                                                  unsigned poll_limit, unsigned long long time_limit_ns,
+                                                  unsigned backoff_ns = 0) {
   unsigned long long start = 0;
   for (unsigned spin = 0; spin < poll_limit; spin++) {
     if (backoff_ns && spin) __nanosleep(backoff_ns);     // long waits of many threads: leave the issue slots alone
@@ -131,6 +131,23 @@ __device__ __forceinline__ bool qd_mbar_wait_bounded(unsigned bar_smem_addr, uns
   }
   *dead = 1;
   return false;
+}
+// The same with the loop as a function that is called when the first try fails.  With the loop, its clock and its limits inlined
+// at every wait, the threads that issue copies and MMAs spent 36 to 250 cycles more on waits most of which wait for nothing (a
+// float32 step of 4 requests at the 3B sizes: 4.07 ms with the loop inlined, 3.99 with the call).  Where a thread holds more
+// registers than a call leaves it (the sums of gemm_f32.cu's second form), the loop stays.
+static __device__ __noinline__ bool qd_mbar_wait_long(unsigned bar_smem_addr, unsigned parity, volatile int* dead,
+                                                      unsigned poll_limit, unsigned long long time_limit_ns, unsigned backoff_ns) {
+  return qd_mbar_wait_loop(bar_smem_addr, parity, dead, poll_limit, time_limit_ns, backoff_ns);
+}
+__device__ __forceinline__ bool qd_mbar_wait_bounded(unsigned bar_smem_addr, unsigned parity, volatile int* dead,
+                                                     unsigned poll_limit, unsigned long long time_limit_ns,
+                                                     unsigned backoff_ns = 0) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok) : "r"(bar_smem_addr), "r"(parity) : "memory");
+  return ok || qd_mbar_wait_long(bar_smem_addr, parity, dead, poll_limit, time_limit_ns, backoff_ns);
 }
 
 // A probe of a library's wait, for tests: one warp waits, with ``poll_limit`` polls, on an mbarrier that

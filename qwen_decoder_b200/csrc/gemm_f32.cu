@@ -193,10 +193,10 @@ __device__ __forceinline__ void fs_end(volatile int& dead, int warp, int lane, u
       tc_bar_init(&fin, 1);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       tc_commit(&fin);
-      tc_wait(&fin, 0, &late);
+      tc_wait_inline(&fin, 0, &late);
     }
     if (warp == FS_TMA_WARP && lane == 0)
-      for (unsigned i = asked > slots ? asked - slots : 0; i < asked; i++) tc_wait(&loaded[i % slots], (i / slots) & 1, &late);
+      for (unsigned i = asked > slots ? asked - slots : 0; i < asked; i++) tc_wait_inline(&loaded[i % slots], (i / slots) & 1, &late);
     __syncthreads();
   }
   if (warp == FS_MMA_WARP) {
@@ -428,7 +428,7 @@ gemm_f32_many_kernel(const __grid_constant__ CUtensorMap map_x, const FsArgs a) 
     };
     ask_w();
     for (int g = 0; g < blocks; g++) {
-      if (!tc_wait(&wfree[g & 1], ((g >> 1) & 1) ^ 1, &dead, 32) && lane == 0) atomicExch(a.status, 1);
+      if (!tc_wait_inline(&wfree[g & 1], ((g >> 1) & 1) ^ 1, &dead, 32) && lane == 0) atomicExch(a.status, 1);
       unsigned char* dst = wring + (g & 1) * FS_WBLOCK + at;
 #pragma unroll
       for (int j = 0; j < 8; j++) fs_put(dst + j * 2048, FS_WPIECE, w[j]);
@@ -448,7 +448,7 @@ gemm_f32_many_kernel(const __grid_constant__ CUtensorMap map_x, const FsArgs a) 
     FsAt at(a);
     pdl_wait();
     for (int g = 0; g < blocks; g++, at.next(a)) {
-      if (!tc_wait(&done, g & 1, &dead, 32) && lane == 0) atomicExch(a.status, 2);
+      if (!tc_wait_inline(&done, g & 1, &dead, 32) && lane == 0) atomicExch(a.status, 2);
       tc_fence_after();
       const bool end = at.ends_part(a);
 #pragma unroll
@@ -475,7 +475,7 @@ gemm_f32_many_kernel(const __grid_constant__ CUtensorMap map_x, const FsArgs a) 
         unsigned s = 0, ph = 0;
         for (int g = 0; g < blocks; g++, at.next(a))
           for (int i = 0; i < 3; i++) {
-            if (!tc_wait(&xfree[s], ph ^ 1, &dead)) { atomicExch(a.status, 3); g = blocks; break; }
+            if (!tc_wait_inline(&xfree[s], ph ^ 1, &dead)) { atomicExch(a.status, 3); g = blocks; break; }
             tc_expect_tx(&xfull[s], a.n_cols * 128);
             tc_load_2d(xring + s * XPIECE, &map_x, at.k * FS_BK, (i == 2 ? 0 : i + 1) * a.T + at.tt * a.t_rows, &xfull[s]);
             asked++;
@@ -492,7 +492,7 @@ gemm_f32_many_kernel(const __grid_constant__ CUtensorMap map_x, const FsArgs a) 
       FsAt at(a);
       unsigned s = 0, ph = 0;
       auto x_there = [&](unsigned code) {
-        if (!tc_wait(&xfull[s], ph, &dead) && one) atomicExch(a.status, code);
+        if (!tc_wait_inline(&xfull[s], ph, &dead) && one) atomicExch(a.status, code);
         const unsigned long long x = dx0 + s * (XPIECE >> 4);
         return x;
       };
@@ -502,10 +502,10 @@ gemm_f32_many_kernel(const __grid_constant__ CUtensorMap map_x, const FsArgs a) 
       };
       auto go = [&]() { tc_fence_after(); __syncwarp(); };
       auto w_there = [&](int g) {
-        if (!tc_wait(&wfull[g & 1], (g >> 1) & 1, &dead) && one) atomicExch(a.status, 4);
+        if (!tc_wait_inline(&wfull[g & 1], (g >> 1) & 1, &dead) && one) atomicExch(a.status, 4);
       };
       auto sums_read = [&](int g) {                  // of the block before
-        if (g > 0 && !tc_wait(&sfree, (g - 1) & 1, &dead) && one) atomicExch(a.status, 8);
+        if (g > 0 && !tc_wait_inline(&sfree, (g - 1) & 1, &dead) && one) atomicExch(a.status, 8);
       };
       w_there(0);
       unsigned long long x = x_there(5);

@@ -20,6 +20,10 @@ __device__ __forceinline__ bool tc_wait(unsigned long long* bar, unsigned parity
                                         unsigned polls = TC_POLLS) {
   return qd_mbar_wait_bounded(tc_smem(bar), parity, dead, polls, 2000000000ull, backoff_ns);
 }
+// the same without a call
+__device__ __forceinline__ bool tc_wait_inline(unsigned long long* bar, unsigned parity, volatile int* dead, unsigned backoff_ns = 0) {
+  return qd_mbar_wait_loop(tc_smem(bar), parity, dead, TC_POLLS, 2000000000ull, backoff_ns);
+}
 // x: innermost coordinate in elements (of whole 128 bytes here), y: row
 __device__ __forceinline__ void tc_load_2d(void* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -90,12 +94,14 @@ static TcEncodeFn tc_encode_fn() {
   }
   return fn;
 }
-// rows x cols bfloat16 or float32, contiguous; boxes of box_rows rows of 128 bytes, 128-byte swizzle, zeros outside
-static bool tc_make_map(CUtensorMap* map, const void* base, bool bfloat16, long long rows, long long cols, int box_rows) {
+// rows x cols bfloat16 or float32, rows ``ld`` elements apart (0: contiguous); boxes of box_rows rows of 128 bytes, 128-byte
+// swizzle, zeros outside
+static bool tc_make_map(CUtensorMap* map, const void* base, bool bfloat16, long long rows, long long cols, int box_rows,
+                        long long ld = 0) {
   TcEncodeFn fn = tc_encode_fn();
   if (!fn) return false;
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)cols * (bfloat16 ? 2 : 4)};
+  cuuint64_t strides[1] = {(cuuint64_t)(ld ? ld : cols) * (bfloat16 ? 2 : 4)};
   cuuint32_t box[2] = {bfloat16 ? 64u : 32u, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   return fn(map, bfloat16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims,
