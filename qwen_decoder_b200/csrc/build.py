@@ -36,6 +36,7 @@ LIBRARIES: Dict[str, str] = {
     "gemm_skinny": "gemm_skinny.cu",
     "gemm_stream": "gemm_stream.cu",
     "gemm_tc5": "gemm_tc5.cu",
+    "gemm_pair": "gemm_pair.cu",
     "attention_generic": "attention_generic.cu",
     "attention_f32": "attention_f32.cu",
     "attention_flash": "attention_flash.cu",
@@ -61,6 +62,7 @@ HEADERS = ["common.cuh", "entry_points.h"]
 EXTRA_DEPS: Dict[str, List[str]] = {
     "decode_attention_noalloc": ["attention_flash.cu", "decode_attention_noalloc.h"],
     "gemm_f32": ["tc5_ops.cuh"],
+    "gemm_pair": ["tc5_ops.cuh"],
     "gated_block": ["short_conv.cuh"],
     "attention_diff": ["short_conv.cuh", "mma_sync.cuh"],
     "qkv_prep": ["short_conv.cuh"],

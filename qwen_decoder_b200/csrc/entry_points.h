@@ -11,6 +11,9 @@ int qd_add_rmsnorm(float* x, const void* delta, int delta_dtype, const float* w,
 int qd_rope_kv_write_biased(void* qkv, const float* bias, int T, int H, int G, int d, int rotary_dim, int pairing,
                             const float* cos_t, const float* sin_t, const int* positions, void* kv,
                             const int* slot_map, int page_size, int write_kv, cudaStream_t stream);
+int qd_gemm_pair(const void* W, const void* X, long long ldx, const float* bias, void* out, int out_dtype, long long ldo, int T,
+                 int N, int K, int cg, int bn, int splits, int epi, int sms, cudaStream_t stream);
+int qd_gemm_pair_plan(int T, int N, int K, int epi, int sms, int* cg_out, int* bn_out, int* splits_out);
 int qd_swiglu(const void* gate_up, void* out, int dtype, int T, int F, cudaStream_t stream);
 void qd_elementwise_plain_next();
 int qd_decode_attention(const void* q, long long q_stride, void* out, const void* kv, const int* block_table,

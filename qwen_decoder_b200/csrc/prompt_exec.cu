@@ -9,12 +9,12 @@
 //
 //   per layer:  h = rmsnorm(x += delta) ; qkv = h Wqkv^T ; bias, rotation, cache write ; attention over
 //               the pages (the decode kernel for the single tokens of a mixed step, a prompt kernel for the
-//               rest) ; delta = attn Wo^T ; h = rmsnorm(x += delta) ; gu = h Wgu^T ; act = silu(gate) * up ;
-//               delta = act Wd^T
+//               rest) ; delta = attn Wo^T ; h = rmsnorm(x += delta) ; gu = h Wgu^T ; act = silu(gate) * up (one kernel
+//               where gemm_pair.cu takes it) ; delta = act Wd^T
 //   at the end: hrows = rmsnorm(x += delta) at the wanted rows          (the output projection stays outside)
 //
-// It holds no kernel of its own.  The launchers live in the other libraries of this directory and the
-// matrix products in cuBLAS (as the reference's do, gpu_kernels.cu:431-436); the caller hands over their
+// It holds no kernel of its own.  The launchers live in the other libraries of this directory and the matrix
+// products that gemm_pair.cu does not take in cuBLAS (as the reference's do, gpu_kernels.cu:431-436); the caller hands over their
 // addresses, so this library links against none of them and uses whatever cuBLAS the process has loaded.
 // The reference launches its layers from C++ as well (gpu_decoder.cu:321-497).
 #include "common.cuh"
@@ -52,7 +52,11 @@ struct PeFns {
   cublasHandle_t blas;             // the caller's handle, bound to ``stream``
   PeGemmBatched gemm_batched;
   decltype(&qd_elementwise_plain_next) plain_next;      // the elementwise library's next launch without the attribute
+  decltype(&qd_gemm_pair) gemm_pair;                    // products on pairs of multiprocessors, where a plan below says so
 };
+
+// How a product is cut (``qd_gemm_pair_plan``); cg 0: the library's product
+struct PePlan { int cg, bn, splits; };
 
 struct PeParams {
   PeFns fn;
@@ -74,6 +78,11 @@ struct PeParams {
   // sums [down_shares, T, D] in ``down_part`` for the next norm's kernel (0: the plain product into ``delta``).
   // With few tokens, a long K and few output features the plain product fills the GPU with too few CTAs.
   float* down_part; int down_shares, pad2;
+  // the output projection, gate and up with the activation, the down projection; their partial sums go to ``o_part`` [splits, T, D]
+  // and ``down_part``
+  PePlan wo_plan, wgu_plan, wd_plan;
+  int sms;
+  float* o_part;
 };
 
 extern "C" int qd_prompt_exec_struct_sizes(int* layer_bytes, int* params_bytes) {
@@ -100,6 +109,16 @@ static int product_shares(const PeParams& p, const void* W, const void* X, float
   return st == CUBLAS_STATUS_SUCCESS ? 0 : 20000 + (int)st;
 }
 
+// The same into ``Y`` or, in shares, into ``part``; what was left: the tensor, its dtype and its parts.
+static int product_for_norm(const PeParams& p, const PePlan& plan, const void* W, const void* X, void* Y, float* part, int T, int N,
+                            int K, const void** left, int* dtype, int* parts, cudaStream_t stream) {
+  *left = Y; *dtype = QD_BF16; *parts = 1;
+  if (!plan.cg) return product(p, W, X, Y, T, N, K);
+  if (plan.splits == 1) return p.fn.gemm_pair(W, X, K, nullptr, Y, QD_BF16, N, T, N, K, plan.cg, plan.bn, 1, 0, p.sms, stream);
+  *left = part; *dtype = QD_F32; *parts = plan.splits;
+  return p.fn.gemm_pair(W, X, K, nullptr, part, QD_F32, N, T, N, K, plan.cg, plan.bn, plan.splits, 1, p.sms, stream);
+}
+
 #define PE_TRY(call)            \
   do {                          \
     int rc_ = (call);           \
@@ -113,14 +132,18 @@ extern "C" int qd_prompt_exec(const PeParams* pp, cudaStream_t stream) {
   if (shares < 0 || shares == 1 ||
       (shares > 1 && (!p.down_part || !p.fn.gemm_batched || !p.fn.plain_next || p.F % (8 * shares))))
     return QD_ERR_UNSUPPORTED;
+  if ((p.wo_plan.cg || p.wgu_plan.cg || p.wd_plan.cg) && !p.fn.gemm_pair) return QD_ERR_UNSUPPORTED;
+  if ((p.wo_plan.cg && p.wo_plan.splits > 1 && !p.o_part) || (p.wd_plan.cg && p.wd_plan.splits > 1 && !p.down_part)) return QD_ERR_UNSUPPORTED;
   const int T = p.T, D = p.D, H = p.H, G = p.G, d = p.d, F = p.F;
   const int n_qkv = (H + 2 * G) * d;
   const long long xn = (long long)T * D;
   const void* delta = p.delta0;
   int delta_dtype = QD_BF16, delta_parts = 1;          // what the previous layer's down projection left
+  const void* o;
+  int o_dtype, o_parts;
   for (int l = 0; l < p.n_layers; l++) {
     const PeLayer& L = p.layers[l];
-    if (delta_parts > 1) p.fn.plain_next();            // the norm that reads the batched product waits for all of it
+    if (shares > 1 && delta_parts > 1) p.fn.plain_next();     // the norm that reads the batched product waits for all of it
     PE_TRY(p.fn.add_rmsnorm(p.x, delta, delta ? delta_dtype : -1, L.norm1_w, p.h, QD_BF16, nullptr, T, D, L.eps1, 1,
                             delta_parts, xn, stream));
     PE_TRY(product(p, L.wqkv, p.h, p.qkv, T, n_qkv, D));
@@ -143,19 +166,22 @@ extern "C" int qd_prompt_exec(const PeParams* pp, cudaStream_t stream) {
     else
       PE_TRY(p.fn.attention_regs(p.qkv, n_qkv, p.attn, L.kv, bt, p.max_blocks, p.cu_tokens + nd, p.start_pos + nd,
                                  p.R - nd, T - nd, H, G, d, p.page_size, p.scale, p.window, stream));
-    PE_TRY(product(p, L.wo, p.attn, p.delta, T, D, H * d));
-    PE_TRY(p.fn.add_rmsnorm(p.x, p.delta, QD_BF16, L.norm2_w, p.h, QD_BF16, nullptr, T, D, L.eps2, 1, 1, xn, stream));
-    PE_TRY(product(p, L.wgu, p.h, p.gu, T, 2 * F, D));
-    PE_TRY(p.fn.swiglu(p.gu, p.act, QD_BF16, T, F, stream));
+    PE_TRY(product_for_norm(p, p.wo_plan, L.wo, p.attn, p.delta, p.o_part, T, D, H * d, &o, &o_dtype, &o_parts, stream));
+    PE_TRY(p.fn.add_rmsnorm(p.x, o, o_dtype, L.norm2_w, p.h, QD_BF16, nullptr, T, D, L.eps2, 1, o_parts, xn, stream));
+    if (p.wgu_plan.cg) {
+      PE_TRY(p.fn.gemm_pair(L.wgu, p.h, D, nullptr, p.act, QD_BF16, F, T, 2 * F, D, p.wgu_plan.cg, p.wgu_plan.bn, 1, 2, p.sms, stream));
+    } else {
+      PE_TRY(product(p, L.wgu, p.h, p.gu, T, 2 * F, D));
+      PE_TRY(p.fn.swiglu(p.gu, p.act, QD_BF16, T, F, stream));
+    }
     if (shares > 1) {
       PE_TRY(product_shares(p, L.wd, p.act, p.down_part, T, D, F, shares));
       delta = p.down_part; delta_dtype = QD_F32; delta_parts = shares;
     } else {
-      PE_TRY(product(p, L.wd, p.act, p.delta, T, D, F));
-      delta = p.delta;
+      PE_TRY(product_for_norm(p, p.wd_plan, L.wd, p.act, p.delta, p.down_part, T, D, F, &delta, &delta_dtype, &delta_parts, stream));
     }
   }
-  if (p.n_wanted > 0 && delta_parts > 1) p.fn.plain_next();
+  if (p.n_wanted > 0 && shares > 1 && delta_parts > 1) p.fn.plain_next();
   if (p.n_wanted > 0)
     PE_TRY(p.fn.add_rmsnorm(p.x, delta, delta ? delta_dtype : -1, p.final_w, p.hrows, QD_BF16, p.logit_rows, p.n_wanted,
                             D, p.final_eps, 0, delta_parts, xn, stream));     // only the wanted rows: x itself stays as it is

@@ -7,6 +7,7 @@ on a CUDA device, or a kernel library that cannot be built or loaded, is an erro
 from __future__ import annotations
 
 import ctypes
+import functools
 import os as _os
 from typing import Optional
 
@@ -501,6 +502,43 @@ def _skinny_call(x, w, bias, out, part, T, N, K, splits, epi, what, w_tiled=Fals
             _I(T), _I(N), _I(K), _I(splits), _I(epi), _stream()), what)
 
 
+@functools.lru_cache(maxsize=4096)
+def gemm_pair_sizes_plan(T: int, N: int, K: int, epi: int, sms: int):
+    a, b, c = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
+    fast = library("gemm_pair").qd_gemm_pair_plan(_I(T), _I(N), _I(K), _I(epi), _I(sms), ctypes.byref(a), ctypes.byref(b),
+                                                  ctypes.byref(c))
+    return (a.value, b.value, c.value) if fast else None
+
+
+def gemm_pair_plan(x: torch.Tensor, w: torch.Tensor, epi: int):
+    """(cg, bn, splits) for ``gemm_pair`` of more tokens than the few-token kernels take, or None where it does not take the
+    product or the library's is the faster one."""
+    T, K = x.shape
+    if not (x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and not few_token_impl(T) and K % 8 == 0 and x.stride(1) == 1
+            and x.stride(0) % 8 == 0 and x.stride(0) >= K and w.is_contiguous() and x.data_ptr() % 16 == 0
+            and w.data_ptr() % 16 == 0):
+        return None
+    return gemm_pair_sizes_plan(T, w.shape[0], K, epi, sm_count())
+
+
+def gemm_pair(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, cg: int, bn: int,
+              splits: int = 1, epi: int = EPI_STORE) -> None:
+    """out = x @ w^T on pairs of multiprocessors, in tiles of ``bn`` rows of w; out as ``epi`` says: [T, N] bfloat16 or float32
+    (+ bias), float32 partial sums [splits, T, N], or the gated activation [T, N / 2] bfloat16 (+ 256 * activation)."""
+    T, K = x.shape
+    N = w.shape[0]
+    _contig(w, "w")
+    assert x.dtype == w.dtype == torch.bfloat16 and x.stride(1) == 1 and w.shape[1] == K and out.stride(-1) == 1
+    if epi == EPI_PARTIAL:
+        assert tuple(out.shape) == (splits, T, N) and out.is_contiguous()
+    else:
+        assert tuple(out.shape) == (T, N if epi == EPI_STORE else N // 2)
+    assert bias is None or (bias.dtype == torch.float32 and bias.numel() == N and bias.is_contiguous())
+    _check(library("gemm_pair").qd_gemm_pair(
+        _ptr(w), _ptr(x), _LL(x.stride(0)), _ptr(bias), _ptr(out), _I(dtype_code(out.dtype)), _LL(out.stride(-2)), _I(T), _I(N),
+        _I(K), _I(cg), _I(bn), _I(splits), _I(epi), _I(sm_count()), _stream()), "gemm_pair")
+
+
 def gemm_stream_status() -> int:
     """0 unless a bounded wait inside the streaming kernel ran out on the current device."""
     return int(library("gemm_stream").qd_gemm_stream_status())
@@ -775,6 +813,7 @@ def prefill_attention_tc5_status() -> int:
 # library -> (its status function, its wait probe): the kernels with bounded waits on mbarriers or a grid barrier
 _STATUS = {"gemm_stream": ("qd_gemm_stream_status", "qd_gemm_stream_wait_probe"),
            "gemm_tc5": ("qd_gemm_tc5_status", "qd_gemm_tc5_wait_probe"),
+           "gemm_pair": ("qd_gemm_pair_status", "qd_gemm_pair_wait_probe"),
            "gemm_f32": ("qd_gemm_f32_status", "qd_gemm_f32_wait_probe"),
            "attention_tc5": ("qd_prefill_attention_tc5_status", "qd_prefill_attention_tc5_wait_probe"),
            "attention_flash": ("qd_decode_attention_tma_status", "qd_decode_attention_tma_wait_probe")}
@@ -1739,7 +1778,12 @@ class PromptFns(ctypes.Structure):
     """Addresses of the launchers and of the library product that the native prompt step calls."""
     _fields_ = [(n, ctypes.c_void_p) for n in ("add_rmsnorm", "rope_kv_write", "swiglu", "attention_regs",
                                                "attention_tc5", "attention_decode", "attention_decode_tma", "gemm_ex",
-                                               "blas", "gemm_batched", "plain_next")]
+                                               "blas", "gemm_batched", "plain_next", "gemm_pair")]
+
+
+class PromptPlan(ctypes.Structure):
+    """How a product of the native prompt step is cut (PePlan in csrc/prompt_exec.cu)."""
+    _fields_ = [(n, ctypes.c_int) for n in ("cg", "bn", "splits")]
 
 
 class PromptParams(ctypes.Structure):
@@ -1753,7 +1797,8 @@ class PromptParams(ctypes.Structure):
                                         "attn", "delta", "gu", "act", "hrows")] + \
         [("n_decode", ctypes.c_int), ("decode_splits", ctypes.c_int)] + \
         [(n, ctypes.c_void_p) for n in ("token_req", "part_o", "part_ml", "tickets", "down_part")] + \
-        [("down_shares", ctypes.c_int), ("pad2", ctypes.c_int)]
+        [("down_shares", ctypes.c_int), ("pad2", ctypes.c_int)] + \
+        [(n, PromptPlan) for n in ("wo_plan", "wgu_plan", "wd_plan")] + [("sms", ctypes.c_int), ("o_part", ctypes.c_void_p)]
 
 
 def prompt_exec_struct_sizes_match() -> bool:
@@ -1799,6 +1844,7 @@ def prompt_fns(use_tc5: bool, with_decode: bool = False, decode_tma: bool = Fals
         fns.gemm_ex = addr(_loaded_cublas().cublasGemmEx)
         fns.gemm_batched = addr(_loaded_cublas().cublasGemmStridedBatchedEx)
         fns.plain_next = addr(ew.qd_elementwise_plain_next)
+        fns.gemm_pair = addr(library("gemm_pair").qd_gemm_pair)
         _prompt_fns[(use_tc5, with_decode, decode_tma)] = fns
     return fns
 

@@ -68,7 +68,7 @@ class Linear:
 
     def forward_partial(self, x: torch.Tensor, with_bias: bool = True) -> torch.Tensor:
         """The product as something a residual stream can take: [T, N] in x's dtype, or -- from the
-        few-token kernel -- float32 partial sums [n_parts, T, N] (bias not added) that the next
+        kernels that share K -- float32 partial sums [n_parts, T, N] (bias not added) that the next
         norm's kernel adds up.  ``with_bias`` False leaves the bias to the caller."""
         bias = self.bias if with_bias else None
         if bias is None and matmul_backend.use_skinny(x, self.weight):
@@ -78,6 +78,9 @@ class Linear:
             shares = matmul_backend.library_shares(x.shape[0], self.out_features, self.in_features)
             if shares:
                 return matmul_backend.linear_partial_library(x, self.weight, shares)
+            out = matmul_backend.linear_partial_pair(x, self.weight)
+            if out is not None:
+                return out
         if bias is not self.bias:
             out = torch.empty((x.shape[0], self.out_features), dtype=x.dtype, device=x.device)
             matmul_backend.linear(x, self.weight, None, out)

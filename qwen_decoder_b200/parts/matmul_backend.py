@@ -4,9 +4,9 @@ float32: the tensor cores on operands cut into three bfloat16 pieces that sum to
 matrices, short rows and rows that are no whole 16-byte pieces float32 FMA (``csrc/gemm_generic.cu``); no TF32 anywhere.  Which of
 the two goes by the matrix, never by the number of tokens, and in neither does a row's result depend on the other rows.
 bfloat16: ``mode`` chooses.
-  * ``auto``    few tokens (<= 64): the hand-written weight-streaming tensor-core kernel
-                (``csrc/gemm_skinny.cu``); more tokens: cuBLAS for products large enough to
-                matter, else the generic kernel;
+  * ``auto``    up to 16 tokens: the hand-written weight-streaming kernels (``csrc/gemm_stream.cu``,
+                ``csrc/gemm_skinny.cu``); more tokens: ``csrc/gemm_pair.cu`` where its plan says that it is the faster
+                one, else cuBLAS for products large enough to matter, else the generic kernel;
   * ``generic`` always the generic kernel (any size);
   * ``cublas``  the library product through torch, as the reference calls cublasHgemm
                 (gpu_kernels.cu:431-436), for every bfloat16 product.
@@ -71,7 +71,11 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: 
         kernels.gemm_skinny(x, w, bias, out)
         counters["own"] += 1
         return
-    if K % 8 == 0 and N % 8 == 0 and N * K >= 256 * 256:
+    plan = kernels.gemm_pair_plan(x, w, kernels.EPI_STORE) if out.stride(1) == 1 else None
+    if plan is not None:
+        kernels.gemm_pair(x, w, bias, out, *plan)
+        counters["own"] += 1
+    elif K % 8 == 0 and N % 8 == 0 and N * K >= 256 * 256:
         _cublas(x, w, bias, out)
     else:
         kernels.gemm_generic(x, w, bias, out)
@@ -115,6 +119,23 @@ def linear_partial_library(x: torch.Tensor, w: torch.Tensor, shares: int) -> tor
     part = torch.bmm(xs, ws, out_dtype=torch.float32)
     kernels.elementwise_plain_next()          # whoever adds these sums up waits for the whole batched product
     return part
+
+
+def linear_partial_pair(x: torch.Tensor, w: torch.Tensor) -> Optional[torch.Tensor]:
+    """x @ w^T from ``csrc/gemm_pair.cu`` for a caller that takes float32 partial sums [shares, T, N] as well as [T, N] in
+    bfloat16, or None where that kernel is not the choice."""
+    plan = kernels.gemm_pair_plan(x, w, kernels.EPI_PARTIAL) if mode == "auto" else None
+    if plan is None:
+        return None
+    T, N, shares = x.shape[0], w.shape[0], plan[2]
+    counters["own"] += 1
+    if shares == 1:
+        out = torch.empty((T, N), dtype=torch.bfloat16, device=x.device)
+        kernels.gemm_pair(x, w, None, out, *plan)
+    else:
+        out = torch.empty((shares, T, N), dtype=torch.float32, device=x.device)
+        kernels.gemm_pair(x, w, None, out, *plan, epi=kernels.EPI_PARTIAL)
+    return out
 
 
 def use_skinny(x: torch.Tensor, w: torch.Tensor) -> bool:

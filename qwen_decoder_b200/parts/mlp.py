@@ -102,7 +102,12 @@ class SwiGLU(FeedForward):
                 kernels.gemm_skinny_swiglu(x, self.gate_up.weight, h, self.gate_up.bias, act)       # gate, up and the activation in one kernel
             matmul_backend.counters["own"] += 1
         else:
-            kernels.swiglu(self.gate_up.forward(x), h, act)
+            plan = kernels.gemm_pair_plan(x, self.gate_up.weight, kernels.EPI_SWIGLU) if matmul_backend.mode == "auto" else None
+            if plan is not None:                             # gate, up and the activation in one kernel
+                kernels.gemm_pair(x, self.gate_up.weight, self.gate_up.bias, h, *plan, epi=kernels.EPI_SWIGLU + 256 * act)
+                matmul_backend.counters["own"] += 1
+            else:
+                kernels.swiglu(self.gate_up.forward(x), h, act)
         return self._down(h)
 
 

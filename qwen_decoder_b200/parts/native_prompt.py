@@ -34,7 +34,7 @@ _MIN_TOKENS = 1       # measured faster at every length: 4 tokens 3.2 against 4.
 # the one arrangement of parts whose order of kernels csrc/prompt_exec.cu restates: a block that answers
 # ``native_params()`` with any other ``composition`` (another order, another part) keeps the parts' own path
 COMPOSITION = "pre_norm/gq_attention/swiglu/rmsnorm/rmsnorm"
-OWN_LAUNCHES_PER_LAYER = 5    # norm, rotation, attention, norm, SwiGLU; the four products are the library's
+OWN_LAUNCHES_PER_LAYER = 4    # norm, rotation, attention, norm; SwiGLU or a product with it; products as ``_plans`` says
 
 
 class NativePrompt:
@@ -102,6 +102,16 @@ class NativePrompt:
                 and len(layout.groups) == 1 and not layout.fixed and ctx.cache.dtype == torch.bfloat16
                 and self.attention_impl(ctx.cache.page_size) is not None)
 
+    def _plans(self, T: int):
+        """(output projection, gate and up, down projection): how ``csrc/gemm_pair.cu`` cuts them at ``T`` tokens, None: the
+        library's product."""
+        c = self.common
+        if matmul_backend.mode != "auto" or any(a[n].data_ptr() % 16 for a in self.entries for n in ("wo", "wgu", "wd")):
+            return None, None, None
+        plan = lambda N, K, epi: kernels.gemm_pair_sizes_plan(T, N, K, epi, kernels.sm_count())
+        return (plan(c["D"], c["H"] * c["d"], kernels.EPI_PARTIAL), plan(2 * c["F"], c["D"], kernels.EPI_SWIGLU),
+                None if matmul_backend.library_shares(T, c["D"], c["F"]) else plan(c["D"], c["F"], kernels.EPI_PARTIAL))
+
     # ---- the step --------------------------------------------------------------
     def _layer_array(self, cache):
         if self._cache_id != id(cache):
@@ -126,8 +136,9 @@ class NativePrompt:
         T, D, H, G, d, F = ctx.num_tokens, c["D"], c["H"], c["G"], c["d"], c["F"]
         bf = torch.bfloat16
         n_qkv = (H + 2 * G) * d
+        wo_plan, wgu_plan, wd_plan = plans = self._plans(T)
         # one scratch buffer for the step, carved into the six activations (all offsets 16-byte aligned)
-        sizes = [T * D, T * n_qkv, T * H * d, T * D, T * 2 * F, T * F]
+        sizes = [T * D, T * n_qkv, T * H * d, T * D, 0 if wgu_plan else T * 2 * F, T * F]
         offs, total = [], 0
         for n in sizes:
             offs.append(total)
@@ -173,11 +184,20 @@ class NativePrompt:
         p.h, p.qkv, p.attn, p.delta, p.gu, p.act = (base + 2 * o for o in offs)
         p.hrows = hrows.data_ptr() if hrows is not None else None
         shares = matmul_backend.library_shares(T, D, F)
-        down_part = torch.empty((shares, T, D), dtype=torch.float32, device=dev) if shares else None
         p.down_shares = shares
-        p.down_part = down_part.data_ptr() if shares else None
-        n_launches = len(self.entries) * (OWN_LAUNCHES_PER_LAYER + (1 if nd else 0)) + (1 if ctx.num_wanted else 0)
+        for field, plan in zip((p.wo_plan, p.wgu_plan, p.wd_plan), plans):
+            field.cg, field.bn, field.splits = plan or (0, 0, 0)
+        p.sms = kernels.sm_count()
+        parts = lambda n: torch.empty((n, T, D), dtype=torch.float32, device=dev) if n > 1 else None
+        down_part = parts(shares or (wd_plan[2] if wd_plan else 0))
+        o_part = parts(wo_plan[2] if wo_plan else 0)
+        p.down_part = down_part.data_ptr() if down_part is not None else None
+        p.o_part = o_part.data_ptr() if o_part is not None else None
+        own = sum(1 for plan in plans if plan)
+        n_launches = len(self.entries) * (OWN_LAUNCHES_PER_LAYER + own + (0 if wgu_plan else 1) + (1 if nd else 0)) \
+            + (1 if ctx.num_wanted else 0)
         kernels.prompt_exec(p, n_launches)
         self.steps += 1
-        matmul_backend.counters["library"] += 4 * len(self.entries)
+        matmul_backend.counters["library"] += (4 - own) * len(self.entries)
+        matmul_backend.counters["own"] += own * len(self.entries)
         return hrows
