@@ -66,7 +66,7 @@ EXTRA_DEPS: Dict[str, List[str]] = {
     "gated_block": ["short_conv.cuh"],
     "attention_diff": ["short_conv.cuh", "mma_sync.cuh"],
     "qkv_prep": ["short_conv.cuh"],
-    "linear_scan": ["short_conv.cuh"],
+    "linear_scan": ["short_conv.cuh", "linear_chunk.cuh", "mma_sync.cuh"],
     "attention_sink": ["mma_sync.cuh"],
 }
 

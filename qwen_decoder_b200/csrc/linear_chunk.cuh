@@ -1,0 +1,868 @@
+// Linear attention over portions in chunks of LC tokens, on the tensor cores (the general kernels of linear_scan.cu go token by
+// token, or four at a time: a serial chain of 0.1 to 0.2 us a token that leaves most of the GPU waiting).  For heads of 64 x 64 or
+// 128 x 128 (keys x values).  With S0 the state before a chunk, g_i the decays, G_p = g_0 .. g_p, d(s, p) = g_(s+1) .. g_p:
+//
+//   plain       o_p = G_p S0^T q_p + sum_(s <= p) d(s, p) (k_s . q_p) x_s,   S <- G S0 + sum_s d(s, last) k_s x_s^T,   x = v
+//   delta rule  the same with x the solution of (1 + A) X = beta (V - G K S0), A[p, s] = beta_p d(s, p) (k_s . k_p) for s < p:
+//               with T = (1 + A)^-1,  X = U - W S0,  U = T (beta V),  W = T (beta G K)
+//
+// Three launches: what a chunk contributes by itself (plain: sum_s d(s, last) k_s v_s^T; delta rule: U and W), all chunks at once;
+// the states before the chunks, one after the other (plain: a sum; delta rule: X = U - W S0 and the state's product, with the state
+// in registers); the outputs with norm and gate, all chunks at once.
+//
+// Numbers stay float32: every operand is cut into three bfloat16 pieces that sum to it exactly, and of the nine products of pieces
+// the six above 2^-24 are taken, the large one and the five small ones in sums of their own.  (T is made by float32 FMA.)  A chunk
+// that holds an infinity, NaN or a number beyond bfloat16's range takes its triangular products by FMA over s <= p only, so that
+// tokens before it stay as they are.
+#pragma once
+#include "common.cuh"
+#include "mma_sync.cuh"
+
+#define LC 64                 // tokens of a chunk
+#define LC_THREADS 256
+#define LC_DEC 68             // numbers per (chunk, head): d(s, last) of the LC tokens, then the chunk's whole decay
+
+struct LinearChunk {
+  const float *q, *k;                     // [T, G, D]
+  const float* v; long long ldv;
+  const float* g; int g_ld; const float* beta;
+  int T, R, H, G;
+  float* state; long long state_stride, s_off;
+  const int *cu_tokens, *slots; int write_state;
+  float* dec;                             // [chunk, H, LC_DEC]
+  float* x;                               // delta rule: [chunk, H, LC, DV]: U, then X
+  bf16* w;                                // delta rule: pieces of W [chunk, H, 3, LC, D]
+  bf16* kp;                               // delta rule: pieces of K [chunk, G, 3, LC, D]
+  float* s0;                              // [chunk, H, DV, D]: what the chunk adds to the state (plain), then the state before it
+  // norm, gate and result, as LinearFinish in linear_scan.cu
+  const float* gate; long long gate_ld; const float* norm; int norm_ld; float eps, out_scale; int gate_kind;
+  void* out; int out_dtype; long long out_stride;
+};
+
+// Chunk ``b`` of all: its request, its first token and how many it has; false past the last one.
+__device__ __forceinline__ bool lc_find(const LinearChunk& a, int b, int& r, int& t0, int& n) {
+  int at = 0;
+  for (r = 0; r < a.R; r++) {
+    const int begin = a.cu_tokens[r], end = a.cu_tokens[r + 1], chunks = (end - begin + LC - 1) / LC;
+    if (b < at + chunks) {
+      t0 = begin + (b - at) * LC;
+      n = min(LC, end - t0);
+      return true;
+    }
+    at += chunks;
+  }
+  return false;
+}
+
+__device__ __forceinline__ unsigned lc_round2(float lo, float hi) {
+  unsigned r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+// the pieces of (x, y) as bfloat16 pairs
+__device__ __forceinline__ void lc_cut(float x, float y, unsigned (&p)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    p[i] = lc_round2(x, y);
+    x -= __uint_as_float(p[i] << 16);
+    y -= __uint_as_float(p[i] & 0xFFFF0000u);
+  }
+}
+__device__ __forceinline__ bool lc_odd(float x) { return !(fabsf(x) <= 3.38e38f); }
+
+// A tile of pieces in shared memory: [3][ROWS][W + 8] bfloat16 (eight rows of a matrix of ldmatrix fall on different banks)
+template <int ROWS, int W>
+struct LcTile {
+  static constexpr int LD = W + 8, PIECE = ROWS * LD, ELEMS = 3 * PIECE;
+};
+// Rows of W numbers ``ld`` apart on their way into registers, the rows from ``n`` on zero, and from there into a tile; true if one of
+// this thread's is odd.
+template <int ROWS, int W, int THREADS>
+__device__ __forceinline__ void lc_ask(float4 (&x)[ROWS * W / 4 / THREADS], const float* src, long long ld, int n) {
+#pragma unroll
+  for (int i = 0; i < ROWS * W / 4 / THREADS; i++) {
+    const int e = threadIdx.x + i * THREADS, row = e / (W / 4), c = (e - row * (W / 4)) * 4;
+    x[i] = row < n ? *reinterpret_cast<const float4*>(src + row * ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+template <int ROWS, int W, int THREADS>
+__device__ __forceinline__ bool lc_put(bf16* tile, const float4 (&x)[ROWS * W / 4 / THREADS]) {
+  using L = LcTile<ROWS, W>;
+  bool odd = false;
+#pragma unroll
+  for (int k = 0; k < ROWS * W / 4 / THREADS; k++) {
+    const int e = threadIdx.x + k * THREADS, row = e / (W / 4), c = (e - row * (W / 4)) * 4;
+    odd = odd || lc_odd(x[k].x) || lc_odd(x[k].y) || lc_odd(x[k].z) || lc_odd(x[k].w);
+    unsigned lo[3], hi[3];
+    lc_cut(x[k].x, x[k].y, lo);
+    lc_cut(x[k].z, x[k].w, hi);
+#pragma unroll
+    for (int i = 0; i < 3; i++) *reinterpret_cast<uint2*>(tile + i * L::PIECE + row * L::LD + c) = make_uint2(lo[i], hi[i]);
+  }
+  return odd;
+}
+// both at once, eight pieces of 16 bytes a thread at a time
+template <int ROWS, int W, int THREADS = LC_THREADS>
+__device__ __forceinline__ bool lc_fill(bf16* tile, const float* src, long long ld, int n) {
+  constexpr int TURN = ROWS * W / 4 / THREADS < 8 ? ROWS * W / 4 / THREADS : 8, STEP = TURN * THREADS * 4 / W;      // rows a turn
+  static_assert(ROWS % STEP == 0 && TURN * THREADS * 4 % W == 0, "whole turns");
+  bool odd = false;
+#pragma unroll 1
+  for (int row = 0; row < ROWS; row += STEP) {
+    float4 x[TURN];
+#pragma unroll
+    for (int i = 0; i < TURN; i++) {
+      const int e = threadIdx.x + i * THREADS, r = row + e / (W / 4), c = e % (W / 4) * 4;
+      x[i] = r < n ? *reinterpret_cast<const float4*>(src + r * ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    using L = LcTile<ROWS, W>;
+#pragma unroll
+    for (int k = 0; k < TURN; k++) {
+      const int e = threadIdx.x + k * THREADS, r = row + e / (W / 4), c = e % (W / 4) * 4;
+      odd = odd || lc_odd(x[k].x) || lc_odd(x[k].y) || lc_odd(x[k].z) || lc_odd(x[k].w);
+      unsigned lo[3], hi[3];
+      lc_cut(x[k].x, x[k].y, lo);
+      lc_cut(x[k].z, x[k].w, hi);
+#pragma unroll
+      for (int i = 0; i < 3; i++) *reinterpret_cast<uint2*>(tile + i * L::PIECE + r * L::LD + c) = make_uint2(lo[i], hi[i]);
+    }
+  }
+  return odd;
+}
+
+// Fragments of one piece.  A: 16 x 16 at (m, k), B: 16 (k) x 16 (n, two tiles of the MMA), from tiles whose rows run over the other
+// index of the matrix (_t) or not.
+__device__ __forceinline__ void lc_a(unsigned (&r)[4], const bf16* t, int ld, int m, int k, int lane) {        // rows m
+  ts_ldmatrix_x4(r, t + (m + (lane & 7) + 8 * ((lane >> 3) & 1)) * ld + k + 8 * (lane >> 4));
+}
+__device__ __forceinline__ void lc_a_t(unsigned (&r)[4], const bf16* t, int ld, int m, int k, int lane) {      // rows k
+  ts_ldmatrix_x4_trans(r, t + (k + (lane & 7) + 8 * (lane >> 4)) * ld + m + 8 * ((lane >> 3) & 1));
+}
+__device__ __forceinline__ void lc_b(unsigned (&r)[4], const bf16* t, int ld, int k, int n, int lane) {        // rows n
+  ts_ldmatrix_x4(r, t + (n + (lane & 7) + 8 * (lane >> 4)) * ld + k + 8 * ((lane >> 3) & 1));
+}
+__device__ __forceinline__ void lc_b_t(unsigned (&r)[4], const bf16* t, int ld, int k, int n, int lane) {      // rows k
+  ts_ldmatrix_x4_trans(r, t + (k + (lane & 7) + 8 * ((lane >> 3) & 1)) * ld + n + 8 * (lane >> 4));
+}
+// Two tiles of 16 x 8: the large products into ``c``, the small ones into ``s`` (an MMA waits for the one before it into the same sum:
+// the two tiles' take turns).
+__device__ __forceinline__ void lc_mma(float (&c)[2][4], float (&s)[2][4], const unsigned (&a)[3][4], const unsigned (&b)[3][4]) {
+  auto both = [&](float (&d)[2][4], int i, int j) {
+#pragma unroll
+    for (int n = 0; n < 2; n++) ts_mma(d[n], a[i], b[j][2 * n], b[j][2 * n + 1]);
+  };
+  both(s, 0, 1);
+  both(c, 0, 0);
+  both(s, 1, 0);
+  both(s, 1, 1);
+  both(s, 0, 2);
+  both(s, 2, 0);
+}
+__device__ __forceinline__ void lc_zero(float (&c)[2][4]) {
+#pragma unroll
+  for (int n = 0; n < 2; n++) c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.f;
+}
+
+// dm[p][s] = d(s, p) for s <= p < LC from the chunk's decays (1 past its end), dm's rows LC_DM apart
+#define LC_DM (LC + 2)
+__device__ __forceinline__ void lc_decays(const LinearChunk& a, int t0, int n, int h, float* gs, float* dm) {
+  if (threadIdx.x < LC) gs[threadIdx.x] = (int)threadIdx.x < n ? a.g[(a.g_ld ? (size_t)(t0 + threadIdx.x) * a.g_ld : 0) + h] : 1.f;
+  __syncthreads();
+  if (threadIdx.x < 4 * LC) {                         // four threads a column: a quarter of its rows each
+    const int s = threadIdx.x & (LC - 1), p0 = (threadIdx.x / LC) * (LC / 4);
+    float d = 1.f;
+    for (int p = s + 1; p < p0; p++) d *= gs[p];
+#pragma unroll
+    for (int p1 = 0; p1 < LC / 4; p1 += 8) {
+      float x[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) x[i] = gs[p0 + p1 + i];
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const int p = p0 + p1 + i;
+        if (p > s) d *= x[i];
+        dm[p * LC_DM + s] = p >= s ? d : 0.f;
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// ------------------------------------------------------------------------------------- what a chunk contributes
+// Plain: s0[chunk, h, j, i] = sum_s d(s, last) v_s[j] k_s[i].  grid (chunks, H)
+template <int D, int DV>
+__global__ void __launch_bounds__(LC_THREADS)
+linear_chunk_add_kernel(LinearChunk a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  extern __shared__ __align__(16) unsigned char lc_sm[];
+  using TK = LcTile<LC, D>;
+  using TV = LcTile<LC, DV>;
+  bf16* ks = reinterpret_cast<bf16*>(lc_sm);
+  bf16* vs = ks + TK::ELEMS;
+  __shared__ float gs[LC], dl[LC];
+  int r, t0, n;
+  if (!lc_find(a, blockIdx.x, r, t0, n)) return;
+  const int h = blockIdx.y, gk = h / (a.H / a.G), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid < LC) gs[tid] = tid < n ? a.g[(a.g_ld ? (size_t)(t0 + tid) * a.g_ld : 0) + h] : 1.f;
+  lc_fill<LC, D>(ks, a.k + ((size_t)t0 * a.G + gk) * D, (long long)a.G * D, n);
+  __syncthreads();
+  float* dec = a.dec + ((size_t)blockIdx.x * a.H + h) * LC_DEC;
+  if (tid <= LC) {                                    // d(s, last); thread LC: the whole decay
+    float d = 1.f;
+    for (int p = LC - 1; p > (tid < LC ? tid : -1); p--) d *= gs[p];
+    if (tid < LC) dl[tid] = d;
+    dec[tid] = d;
+  }
+  __syncthreads();
+  const float* v = a.v + (size_t)t0 * a.ldv + (size_t)h * DV;
+  for (int e = tid; e < LC * (DV / 4); e += LC_THREADS) {
+    const int row = e / (DV / 4), c = (e - row * (DV / 4)) * 4;
+    const float4 x = row < n ? *reinterpret_cast<const float4*>(v + row * a.ldv + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float d = dl[row];
+    unsigned lo[3], hi[3];
+    lc_cut(d * x.x, d * x.y, lo);
+    lc_cut(d * x.z, d * x.w, hi);
+#pragma unroll
+    for (int i = 0; i < 3; i++) *reinterpret_cast<uint2*>(vs + i * TV::PIECE + row * TV::LD + c) = make_uint2(lo[i], hi[i]);
+  }
+  __syncthreads();
+  // a warp: 16 rows (j) at a time by a share of the columns (i)
+  constexpr int MT = DV / 16, NW = 8 / (MT < 8 ? MT : 8), NP = D / 16 / NW;      // warps to a row of tiles; pairs of tiles a warp
+  float* out = a.s0 + ((size_t)blockIdx.x * a.H + h) * DV * D;
+  const int m = (warp / NW) * 16, n0 = (warp % NW) * NP * 16;
+#pragma unroll
+  for (int np = 0; np < NP; np++) {
+    float c[2][4], s[2][4];
+    lc_zero(c);
+    lc_zero(s);
+#pragma unroll
+    for (int kk = 0; kk < LC / 16; kk++) {
+      unsigned fa[3][4], fb[3][4];
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        lc_a_t(fa[i], vs + i * TV::PIECE, TV::LD, m, kk * 16, lane);
+        lc_b_t(fb[i], ks + i * TK::PIECE, TK::LD, kk * 16, n0 + np * 16, lane);
+      }
+      lc_mma(c, s, fa, fb);
+    }
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+      float* o = out + (size_t)(m + (lane >> 2)) * D + n0 + np * 16 + t * 8 + (lane & 3) * 2;
+      *reinterpret_cast<float2*>(o) = make_float2(c[t][0] + s[t][0], c[t][1] + s[t][1]);
+      *reinterpret_cast<float2*>(o + 8 * D) = make_float2(c[t][2] + s[t][2], c[t][3] + s[t][3]);
+    }
+  }
+}
+
+// Delta rule: U, the pieces of W, of K and the decays.  grid (chunks, H)
+template <int D, int DV>
+__global__ void __launch_bounds__(LC_THREADS, 2)
+linear_chunk_solve_kernel(LinearChunk a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  static_assert(D == DV, "the values take the keys' place in shared memory");
+  extern __shared__ __align__(16) unsigned char lc_sm[];
+  using TK = LcTile<LC, D>;
+  bf16* ks = reinterpret_cast<bf16*>(lc_sm);
+  float* dm = reinterpret_cast<float*>(ks + TK::ELEMS);                 // [LC][LC_DM]: decays, then M of the inverse's steps
+  float* am = dm + LC * LC_DM;                                          // A, lower triangle
+  float* tm = am + LC * LC_DM;                                          // T
+  __shared__ float gs[LC], bs[LC], bg[LC];
+  int r, t0, n;
+  if (!lc_find(a, blockIdx.x, r, t0, n)) return;
+  const int h = blockIdx.y, per = a.H / a.G, gk = h / per, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const float* kg = a.k + ((size_t)t0 * a.G + gk) * D;
+  const float* vg = a.v + (size_t)t0 * a.ldv + (size_t)h * DV;
+  if (tid < LC) bs[tid] = tid < n ? a.beta[(size_t)(t0 + tid) * a.H + h] : 0.f;
+  bool odd = lc_fill<LC, D>(ks, kg, (long long)a.G * D, n);
+  lc_decays(a, t0, n, h, gs, dm);
+  if (tid < LC) {
+    bg[tid] = bs[tid] * (dm[tid * LC_DM] * gs[0]);
+    odd = odd || lc_odd(bs[tid]) || lc_odd(bg[tid]);
+    float* dec = a.dec + ((size_t)blockIdx.x * a.H + h) * LC_DEC;
+    dec[tid] = dm[(LC - 1) * LC_DM + tid];
+    if (tid == 0) dec[LC] = dm[(LC - 1) * LC_DM] * gs[0];
+  }
+  // (a scheduler's two warps have rows whose triangular products are five blocks together)
+  const int part = warp >> 2, m = (part ? 3 - (warp & 3) : warp & 3) * 16, g = lane >> 2, t2 = (lane & 3) * 2;
+  // A: a warp has 16 rows by every other pair of column tiles up to the diagonal
+  for (int np = part; np * 16 <= m; np += 2) {
+    float c[2][4], s[2][4];
+    lc_zero(c);
+    lc_zero(s);
+#pragma unroll 2
+    for (int kk = 0; kk < D / 16; kk++) {
+      unsigned fa[3][4], fb[3][4];
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        lc_a(fa[i], ks + i * TK::PIECE, TK::LD, m, kk * 16, lane);
+        lc_b(fb[i], ks + i * TK::PIECE, TK::LD, kk * 16, np * 16, lane);
+      }
+      lc_mma(c, s, fa, fb);
+    }
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const int p = m + g + 8 * (e >> 1), q = np * 16 + t * 8 + t2 + (e & 1);
+        am[p * LC_DM + q] = q < p ? bs[p] * (dm[p * LC_DM + q] * (c[t][e] + s[t][e])) : 0.f;
+      }
+  }
+  for (int e = tid; e < LC * LC_DM; e += LC_THREADS) tm[e] = 0.f;
+  // the pieces of K, once for the value heads that share it
+  if (h == gk * per) {
+    bf16* to = a.kp + ((size_t)blockIdx.x * a.G + gk) * 3 * LC * D;
+    for (int e = tid; e < 3 * LC * (D / 8); e += LC_THREADS) {
+      const int row = e / (D / 8), c = (e - row * (D / 8)) * 8;
+      *reinterpret_cast<uint4*>(to + row * D + c) = *reinterpret_cast<const uint4*>(ks + row * TK::LD + c);
+    }
+  }
+  __syncthreads();
+  // T: blocks of 16 on the diagonal a column a thread, then blocks of 16 and of 32 below them: T21 = -T22 (A21 T11)
+  if (tid < LC) {
+    const int b = tid & ~15, col = tid & 15;
+    float t[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) t[i] = i == col ? 1.f : 0.f;
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+      if (k < col) t[k] = 0.f;                        // (above the diagonal, whatever A holds there)
+#pragma unroll
+      for (int i = k + 1; i < 16; i++) t[i] = fmaf(-am[(b + i) * LC_DM + b + k], t[k], t[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 16; i++) tm[(b + i) * LC_DM + b + col] = t[i];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int half = 16; half < LC; half *= 2) {         // four neighbouring numbers a thread
+    const int blocks = LC / (2 * half), per_block = half * half / 4;
+    const int b = tid / per_block * 2 * half, i = tid % per_block / (half / 4), j = tid % (half / 4) * 4;
+    const bool mine = tid < blocks * per_block;
+    if (mine) {
+      float y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+      for (int k = 0; k < half; k++) {
+        const float w = am[(b + half + i) * LC_DM + b + k];
+        const float2 lo = *reinterpret_cast<const float2*>(tm + (b + k) * LC_DM + b + j), hi = *reinterpret_cast<const float2*>(tm + (b + k) * LC_DM + b + j + 2);
+        y[0] = fmaf(w, lo.x, y[0]);
+        y[1] = fmaf(w, lo.y, y[1]);
+        y[2] = fmaf(w, hi.x, y[2]);
+        y[3] = fmaf(w, hi.y, y[3]);
+      }
+#pragma unroll
+      for (int c = 0; c < 4; c++) dm[(b + i) * LC_DM + j + c] = y[c];
+    }
+    __syncthreads();
+    if (mine) {
+      float y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+      for (int k = 0; k < half; k++) {
+        if (k > i) break;                             // (rows behind this one may not be numbers)
+        const float w = -tm[(b + half + i) * LC_DM + b + half + k];
+        const float2 lo = *reinterpret_cast<const float2*>(dm + (b + k) * LC_DM + j), hi = *reinterpret_cast<const float2*>(dm + (b + k) * LC_DM + j + 2);
+        y[0] = fmaf(w, lo.x, y[0]);
+        y[1] = fmaf(w, lo.y, y[1]);
+        y[2] = fmaf(w, hi.x, y[2]);
+        y[3] = fmaf(w, hi.y, y[3]);
+      }
+#pragma unroll
+      for (int c = 0; c < 4; c++) tm[(b + half + i) * LC_DM + b + j + c] = y[c];
+    }
+    __syncthreads();
+  }
+  // T (f_s rows): 16 rows by half of the columns of a warp; ``put`` takes a pair of neighbouring results
+  odd = __syncthreads_or(odd);
+  constexpr int NP = D / 32;
+  auto scalar = [&](const float* f, const float* src, long long ld, auto&& put) {      // only what lies at or before a token joins its sum
+    for (int e = tid; e < LC * (D / 2); e += LC_THREADS) {
+      const int p = e / (D / 2), c = (e - p * (D / 2)) * 2;
+      float x = 0.f, y = 0.f;
+      for (int s = 0; s <= p && s < n; s++) {
+        const float w = tm[p * LC_DM + s] * f[s];
+        x = fmaf(w, src[s * ld + c], x);
+        y = fmaf(w, src[s * ld + c + 1], y);
+      }
+      put(p, c, x, y);
+    }
+  };
+  auto product = [&](const float* f, auto&& before, auto&& put) {
+    float c[NP][2][4], s[NP][2][4];
+#pragma unroll
+    for (int i = 0; i < NP; i++) { lc_zero(c[i]); lc_zero(s[i]); }
+#pragma unroll 1
+    for (int kk = 0; kk * 16 <= m; kk++) {
+      unsigned fa[3][4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int p = m + g + 8 * (i & 1), q = kk * 16 + t2 + 8 * (i >> 1);
+        const float2 x = *reinterpret_cast<const float2*>(tm + p * LC_DM + q);
+        unsigned cut[3];
+        lc_cut(x.x * f[q], x.y * f[q + 1], cut);
+        fa[0][i] = cut[0]; fa[1][i] = cut[1]; fa[2][i] = cut[2];
+      }
+#pragma unroll
+      for (int np = 0; np < NP; np++) {
+        unsigned fb[3][4];
+#pragma unroll
+        for (int i = 0; i < 3; i++) lc_b_t(fb[i], ks + i * TK::PIECE, TK::LD, kk * 16, part * (D / 2) + np * 16, lane);
+        lc_mma(c[np], s[np], fa, fb);
+      }
+    }
+    before();
+#pragma unroll
+    for (int np = 0; np < NP; np++)
+#pragma unroll
+      for (int t = 0; t < 2; t++)
+#pragma unroll
+        for (int e = 0; e < 4; e += 2)
+          put(m + g + 4 * e, part * (D / 2) + np * 16 + t * 8 + t2, c[np][t][e] + s[np][t][e], c[np][t][e + 1] + s[np][t][e + 1]);
+  };
+  // W's pieces take K's place and go out in whole rows
+  auto w_put = [&](int p, int c, float x, float y) {
+    unsigned cut[3];
+    lc_cut(x, y, cut);
+#pragma unroll
+    for (int i = 0; i < 3; i++) *reinterpret_cast<unsigned*>(ks + (i * LC + p) * TK::LD + c) = cut[i];
+  };
+  if (odd) scalar(bg, kg, (long long)a.G * D, w_put);
+  else product(bg, [] { __syncthreads(); }, w_put);
+  __syncthreads();
+  bf16* wp = a.w + ((size_t)blockIdx.x * a.H + h) * 3 * LC * D;
+  for (int e = tid; e < 3 * LC * (D / 8); e += LC_THREADS) {
+    const int row = e / (D / 8), c = (e - row * (D / 8)) * 8;
+    *reinterpret_cast<uint4*>(wp + row * D + c) = *reinterpret_cast<const uint4*>(ks + row * TK::LD + c);
+  }
+  __syncthreads();
+  odd = __syncthreads_or(lc_fill<LC, DV>(ks, vg, a.ldv, n)) || odd;
+  float* u = a.x + ((size_t)blockIdx.x * a.H + h) * LC * DV;
+  auto u_put = [&](int p, int c, float x, float y) { *reinterpret_cast<float2*>(u + p * DV + c) = make_float2(x, y); };
+  if (odd) scalar(bs, vg, a.ldv, u_put);
+  else product(bs, [] {}, u_put);
+}
+
+// ----------------------------------------------------------------------------------- the states before the chunks
+// Plain.  grid (DV D / 4 / LC_THREADS, H, requests)
+template <int D, int DV>
+__global__ void __launch_bounds__(LC_THREADS)
+linear_chunk_states_kernel(LinearChunk a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int h = blockIdx.y, req = blockIdx.z, e = blockIdx.x * LC_THREADS + threadIdx.x;
+  int first = 0;
+  for (int r = 0; r < req; r++) first += (a.cu_tokens[r + 1] - a.cu_tokens[r] + LC - 1) / LC;
+  const int chunks = (a.cu_tokens[req + 1] - a.cu_tokens[req] + LC - 1) / LC;
+  float4* S = reinterpret_cast<float4*>(a.state + (size_t)a.slots[req] * a.state_stride + a.s_off + (size_t)h * DV * D) + e;
+  float4 s = *S;
+  constexpr int AHEAD = 8;
+  for (int c0 = 0; c0 < chunks; c0 += AHEAD) {
+    float4 add[AHEAD];
+    float G[AHEAD];
+#pragma unroll
+    for (int i = 0; i < AHEAD; i++)
+      if (c0 + i < chunks) {
+        const size_t at = (size_t)(first + c0 + i) * a.H + h;
+        add[i] = reinterpret_cast<const float4*>(a.s0 + at * DV * D)[e];
+        G[i] = a.dec[at * LC_DEC + LC];
+      }
+#pragma unroll
+    for (int i = 0; i < AHEAD; i++)
+      if (c0 + i < chunks) {
+        reinterpret_cast<float4*>(a.s0 + ((size_t)(first + c0 + i) * a.H + h) * DV * D)[e] = s;
+        s = make_float4(fmaf(G[i], s.x, add[i].x), fmaf(G[i], s.y, add[i].y), fmaf(G[i], s.z, add[i].z), fmaf(G[i], s.w, add[i].w));
+      }
+  }
+  if (a.write_state) *S = s;
+}
+
+// Delta rule.  grid (DV / 32, H, requests): a CTA takes 32 value columns of a head through the request's chunks.  S [j][i] is 32 x D:
+// a warp has D / 8 of the i.
+#define LC_COLS 32
+template <int D, int DV>
+__global__ void __launch_bounds__(LC_THREADS)
+linear_chunk_delta_kernel(LinearChunk a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  extern __shared__ __align__(16) unsigned char lc_sm[];
+  using TW = LcTile<LC, D>;
+  using TS = LcTile<LC_COLS, D>;
+  using TX = LcTile<LC, LC_COLS>;
+  bf16* wbuf = reinterpret_cast<bf16*>(lc_sm);                          // two chunks' pieces of W: the next one's are long on their way
+  bf16* ks = wbuf + 2 * TW::ELEMS;
+  bf16* ss = ks + TW::ELEMS;
+  bf16* xs = ss + TS::ELEMS;
+  float* ubuf = reinterpret_cast<float*>(xs + TX::ELEMS);               // two of [LC][LC_COLS + 4]
+  constexpr int LU = LC_COLS + 4, IW = D / 8, NP = IW / 16;             // a warp's columns of S; pairs of tiles among them
+  static_assert(IW % 16 == 0, "a warp has whole pairs of tiles");
+  const int h = blockIdx.y, req = blockIdx.z, j0 = blockIdx.x * LC_COLS, gk = h / (a.H / a.G);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t2 = (lane & 3) * 2;
+  int first = 0;
+  for (int r = 0; r < req; r++) first += (a.cu_tokens[r + 1] - a.cu_tokens[r] + LC - 1) / LC;
+  const int chunks = (a.cu_tokens[req + 1] - a.cu_tokens[req] + LC - 1) / LC;
+  if (!chunks) return;
+  auto pieces = [&](bf16* tile, const bf16* src) {
+    for (int e = tid; e < 3 * LC * (D / 8); e += LC_THREADS) {
+      const int row = e / (D / 8), c = (e - row * (D / 8)) * 8;
+      ts_cp_async16(tile + row * TW::LD + c, src + row * D + c, 16);
+    }
+  };
+  auto ask_w = [&](int c) {
+    const size_t at = (size_t)(first + c) * a.H + h;
+    float* us = ubuf + (c & 1) * LC * LU;
+    pieces(wbuf + (c & 1) * TW::ELEMS, a.w + at * 3 * LC * D);
+    for (int e = tid; e < LC * (LC_COLS / 4); e += LC_THREADS) {
+      const int row = e / (LC_COLS / 4), col = (e - row * (LC_COLS / 4)) * 4;
+      ts_cp_async16(us + row * LU + col, a.x + (at * LC + row) * DV + j0 + col, 16);
+    }
+  };
+  auto ask_k = [&](int c) { pieces(ks, a.kp + ((size_t)(first + c) * a.G + gk) * 3 * LC * D); };
+  ask_w(0);
+  ts_commit();
+  ask_k(0);
+  ts_commit();
+  if (chunks > 1) ask_w(1);
+  ts_commit();
+  // S: rows j of both tiles of 16, columns i of this warp
+  float* state = a.state + (size_t)a.slots[req] * a.state_stride + a.s_off + ((size_t)h * DV + j0) * D;
+  float S[2][NP][2][4];
+  const int i0 = warp * IW;
+  auto each = [&](auto&& f) {                         // f(pair of numbers, j, i)
+#pragma unroll
+    for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+      for (int np = 0; np < NP; np++)
+#pragma unroll
+        for (int t = 0; t < 2; t++)
+#pragma unroll
+          for (int e = 0; e < 4; e += 2) f(S[mt][np][t][e], S[mt][np][t][e + 1], mt * 16 + g + 4 * e, i0 + np * 16 + t * 8 + t2);
+  };
+  each([&](float& x, float& y, int j, int i) {
+    const float2 v = *reinterpret_cast<const float2*>(state + (size_t)j * D + i);
+    x = v.x;
+    y = v.y;
+  });
+  for (int c = 0; c < chunks; c++) {
+    const size_t at = (size_t)(first + c) * a.H + h;
+    float* s0 = a.s0 + (at * DV + j0) * D;
+    each([&](float& x, float& y, int j, int i) {      // the state before the chunk: for the outputs, and as pieces
+      *reinterpret_cast<float2*>(s0 + (size_t)j * D + i) = make_float2(x, y);
+      unsigned cut[3];
+      lc_cut(x, y, cut);
+#pragma unroll
+      for (int q = 0; q < 3; q++) *reinterpret_cast<unsigned*>(ss + q * TS::PIECE + j * TS::LD + i) = cut[q];
+    });
+    const float* dec = a.dec + at * LC_DEC;
+    const int m = (warp & 3) * 16, n0 = (warp >> 2) * 16;
+    const float d0 = dec[m + g], d1 = dec[m + g + 8], G = dec[LC];
+    const bf16* ws = wbuf + (c & 1) * TW::ELEMS;
+    const float* us = ubuf + (c & 1) * LC * LU;
+    ts_wait<2>();                                     // behind W of this chunk came W of the next and K of this
+    __syncthreads();
+    {                                                 // X = U - W S0: 16 tokens by 16 columns a warp
+      float y[2][4], s[2][4], y1[2][4], s1[2][4];      // even and odd blocks of k in sums of their own: half as long a chain
+      lc_zero(y);
+      lc_zero(s);
+      lc_zero(y1);
+      lc_zero(s1);
+#pragma unroll
+      for (int kk = 0; kk < D / 16; kk++) {
+        unsigned fa[3][4], fb[3][4];
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          lc_a(fa[i], ws + i * TW::PIECE, TW::LD, m, kk * 16, lane);
+          lc_b(fb[i], ss + i * TS::PIECE, TS::LD, kk * 16, n0, lane);
+        }
+        if (kk & 1) lc_mma(y1, s1, fa, fb);
+        else lc_mma(y, s, fa, fb);
+      }
+#pragma unroll
+      for (int t = 0; t < 2; t++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) { y[t][e] += y1[t][e]; s[t][e] += s1[t][e]; }
+      float* xg = a.x + at * LC * DV + j0;
+#pragma unroll
+      for (int t = 0; t < 2; t++)
+#pragma unroll
+        for (int e = 0; e < 4; e += 2) {
+          const int p = m + g + 4 * e, j = n0 + t * 8 + t2;
+          const float2 u = *reinterpret_cast<const float2*>(us + p * LU + j);
+          const float x0 = u.x - (y[t][e] + s[t][e]), x1 = u.y - (y[t][e + 1] + s[t][e + 1]), d = e ? d1 : d0;
+          *reinterpret_cast<float2*>(xg + (size_t)p * DV + j) = make_float2(x0, x1);
+          unsigned cut[3];
+          lc_cut(d * x0, d * x1, cut);
+#pragma unroll
+          for (int q = 0; q < 3; q++) *reinterpret_cast<unsigned*>(xs + q * TX::PIECE + p * TX::LD + j) = cut[q];
+        }
+    }
+    __syncthreads();
+    if (c + 2 < chunks) ask_w(c + 2);
+    ts_commit();
+    ts_wait<1>();
+    __syncthreads();
+#pragma unroll
+    for (int np = 0; np < NP; np++) {
+      float y[2][2][4], s[2][2][4];
+#pragma unroll
+      for (int mt = 0; mt < 2; mt++) { lc_zero(y[mt]); lc_zero(s[mt]); }
+#pragma unroll
+      for (int kk = 0; kk < LC / 16; kk++) {
+        unsigned fa[2][3][4], fb[3][4];
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          lc_b_t(fb[i], ks + i * TW::PIECE, TW::LD, kk * 16, i0 + np * 16, lane);
+#pragma unroll
+          for (int mt = 0; mt < 2; mt++) lc_a_t(fa[mt][i], xs + i * TX::PIECE, TX::LD, mt * 16, kk * 16, lane);
+        }
+#pragma unroll
+        for (int mt = 0; mt < 2; mt++) lc_mma(y[mt], s[mt], fa[mt], fb);
+      }
+#pragma unroll
+      for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+        for (int t = 0; t < 2; t++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) S[mt][np][t][e] = fmaf(G, S[mt][np][t][e], y[mt][t][e] + s[mt][t][e]);
+    }
+    __syncthreads();
+    if (c + 1 < chunks) ask_k(c + 1);
+    ts_commit();
+  }
+  ts_wait<0>();
+  if (a.write_state)
+    each([&](float& x, float& y, int j, int i) { *reinterpret_cast<float2*>(state + (size_t)j * D + i) = make_float2(x, y); });
+}
+
+// ------------------------------------------------------------------------------------------------ the outputs
+// out[t, h] = o / sqrt(mean(o^2) + eps) (* norm) * gate * out_scale with o as above.  grid (chunks, H); a warp has 16 tokens by a
+// quarter of the columns, and of the products of q and k 16 tokens by 16.
+#define LC_OUT_THREADS 512
+template <int D, int DV, bool DELTA>
+__global__ void __launch_bounds__(LC_OUT_THREADS)
+linear_chunk_out_kernel(LinearChunk a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  extern __shared__ __align__(16) unsigned char lc_sm[];
+  using TK = LcTile<LC, D>;
+  using TS = LcTile<DV, D>;
+  using TX = LcTile<LC, DV>;
+  using TP = LcTile<LC, LC>;
+  constexpr int FIRST = TS::ELEMS > TK::ELEMS + TX::ELEMS ? TS::ELEMS : TK::ELEMS + TX::ELEMS;
+  static_assert(TP::ELEMS <= TK::ELEMS, "");
+  bf16* qs = reinterpret_cast<bf16*>(lc_sm);
+  bf16* ss = qs + TK::ELEMS;                          // the state; after it K and X
+  bf16* ks = ss;
+  bf16* xs = ks + TK::ELEMS;
+  bf16* ps = ks;                                      // d(s, p) (k_s . q_p), in the keys' place
+  float* dm = reinterpret_cast<float*>(ss + FIRST);   // [LC][LC_DM]
+  float* os = reinterpret_cast<float*>(qs);           // [LC][LO]: the outputs take the queries' place
+  constexpr int LO = DV + 4;
+  static_assert(LC * LO * 4 <= TK::ELEMS * 2, "the outputs fit where the queries were");
+  __shared__ float gs[LC];
+  int r, t0, n;
+  if (!lc_find(a, blockIdx.x, r, t0, n)) return;
+  const int h = blockIdx.y, gk = h / (a.H / a.G), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t2 = (lane & 3) * 2;
+  const size_t at = (size_t)blockIdx.x * a.H + h;
+  const float* xg = DELTA ? a.x + at * LC * DV : a.v + (size_t)t0 * a.ldv + (size_t)h * DV;
+  const long long ldx = DELTA ? DV : a.ldv;
+  lc_fill<LC, D, LC_OUT_THREADS>(qs, a.q + ((size_t)t0 * a.G + gk) * D, (long long)a.G * D, n);
+  lc_fill<DV, D, LC_OUT_THREADS>(ss, a.s0 + at * DV * D, D, DV);
+  lc_decays(a, t0, n, h, gs, dm);
+  // K and X are on their way while the state's product is made
+  float4 kx[LC * D / 4 / LC_OUT_THREADS], xx[LC * DV / 4 / LC_OUT_THREADS];
+  lc_ask<LC, D, LC_OUT_THREADS>(kx, a.k + ((size_t)t0 * a.G + gk) * D, (long long)a.G * D, n);
+  lc_ask<LC, DV, LC_OUT_THREADS>(xx, xg, ldx, n);
+  constexpr int NP = DV / 64;
+  // (a scheduler's four warps have all four rows of tiles: their triangular products are of different lengths)
+  const int part = warp >> 2, m = ((warp + part) & 3) * 16, c0 = part * (DV / 4);
+  float o[NP][2][4], s2[NP][2][4];
+  const float g0 = gs[0], G0 = dm[(m + g) * LC_DM] * g0, G1 = dm[(m + g + 8) * LC_DM] * g0;
+#pragma unroll
+  for (int np = 0; np < NP; np++) { lc_zero(o[np]); lc_zero(s2[np]); }
+#pragma unroll 2
+  for (int kk = 0; kk < D / 16; kk++) {               // G_p S0^T q_p
+    unsigned fa[3][4];
+#pragma unroll
+    for (int i = 0; i < 3; i++) lc_a(fa[i], qs + i * TK::PIECE, TK::LD, m, kk * 16, lane);
+#pragma unroll
+    for (int np = 0; np < NP; np++) {
+      unsigned fb[3][4];
+#pragma unroll
+      for (int i = 0; i < 3; i++) lc_b(fb[i], ss + i * TS::PIECE, TS::LD, kk * 16, c0 + np * 16, lane);
+      lc_mma(o[np], s2[np], fa, fb);
+    }
+  }
+#pragma unroll
+  for (int np = 0; np < NP; np++)
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        o[np][t][e] = (e < 2 ? G0 : G1) * (o[np][t][e] + s2[np][t][e]);
+        s2[np][t][e] = 0.f;
+      }
+  __syncthreads();
+  lc_put<LC, D, LC_OUT_THREADS>(ks, kx);
+  const bool odd = __syncthreads_or(lc_put<LC, DV, LC_OUT_THREADS>(xs, xx));
+  // the gate of what this thread stores in the end
+  constexpr int LANES = DV / 4, PER = LC_OUT_THREADS / LANES;
+  const int j = (tid % LANES) * 4;
+  float2 z[LC / PER][2];
+  float4 w = make_float4(1.f, 1.f, 1.f, 1.f);
+  if (a.norm) {
+    const float* norm = a.norm + (size_t)h * a.norm_ld + j;
+    w = make_float4(norm[0], norm[1], norm[2], norm[3]);
+  }
+#pragma unroll
+  for (int i = 0; i < LC / PER; i++) {
+    const int p = min(tid / LANES + i * PER, n - 1);
+    const float2* gate = reinterpret_cast<const float2*>(a.gate + (size_t)(t0 + p) * a.gate_ld + (size_t)h * DV + j);
+    z[i][0] = gate[0];
+    z[i][1] = gate[1];
+  }
+  float c[2][4], s[2][4];
+  lc_zero(c);
+  lc_zero(s);
+  if (part * 16 <= m) {                               // tokens s part * 16 .. + 15 for tokens p m .. m + 15
+#pragma unroll 2
+    for (int kk = 0; kk < D / 16; kk++) {
+      unsigned fa[3][4], fb[3][4];
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        lc_a(fa[i], qs + i * TK::PIECE, TK::LD, m, kk * 16, lane);
+        lc_b(fb[i], ks + i * TK::PIECE, TK::LD, kk * 16, part * 16, lane);
+      }
+      lc_mma(c, s, fa, fb);
+    }
+  }
+  __syncthreads();
+  if (part * 16 <= m) {
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+#pragma unroll
+      for (int e = 0; e < 4; e += 2) {
+        const int p = m + g + 4 * e, q = part * 16 + t * 8 + t2;
+        float2* d = reinterpret_cast<float2*>(dm + p * LC_DM + q);      // (this thread's alone)
+        const float x = q <= p ? d->x * (c[t][e] + s[t][e]) : 0.f, y = q + 1 <= p ? d->y * (c[t][e + 1] + s[t][e + 1]) : 0.f;
+        if (odd) *d = make_float2(x, y);
+        unsigned cut[3];
+        lc_cut(x, y, cut);
+#pragma unroll
+        for (int i = 0; i < 3; i++) *reinterpret_cast<unsigned*>(ps + i * TP::PIECE + p * TP::LD + q) = cut[i];
+      }
+  }
+  __syncthreads();
+  if (odd) {                                          // only what lies at or before a token joins its sum
+#pragma unroll
+    for (int np = 0; np < NP; np++)
+#pragma unroll
+      for (int t = 0; t < 2; t++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const int p = m + g + 8 * (e >> 1), j = c0 + np * 16 + t * 8 + t2 + (e & 1);
+          float y = 0.f;
+          for (int s = 0; s <= p && s < n; s++) y = fmaf(dm[p * LC_DM + s], xg[s * ldx + j], y);
+          s2[np][t][e] = y;
+        }
+  } else {
+#pragma unroll 1
+    for (int kb = 0; kb * 16 <= m; kb++) {
+      unsigned fa[3][4];
+#pragma unroll
+      for (int i = 0; i < 3; i++) lc_a(fa[i], ps + i * TP::PIECE, TP::LD, m, kb * 16, lane);
+#pragma unroll
+      for (int np = 0; np < NP; np++) {
+        unsigned fb[3][4];
+#pragma unroll
+        for (int i = 0; i < 3; i++) lc_b_t(fb[i], xs + i * TX::PIECE, TX::LD, kb * 16, c0 + np * 16, lane);
+        lc_mma(o[np], s2[np], fa, fb);
+      }
+    }
+  }
+#pragma unroll
+  for (int np = 0; np < NP; np++)
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+#pragma unroll
+      for (int e = 0; e < 4; e += 2)
+        *reinterpret_cast<float2*>(os + (m + g + 4 * e) * LO + c0 + np * 16 + t * 8 + t2) =
+            make_float2(o[np][t][e] + s2[np][t][e], o[np][t][e + 1] + s2[np][t][e + 1]);
+  __syncthreads();
+  // norm, gate, store: a group of DV / 4 lanes has a token
+#pragma unroll
+  for (int i = 0; i < LC / PER; i++) {
+    const int p = tid / LANES + i * PER;
+    const float4 y = *reinterpret_cast<const float4*>(os + p * LO + j);
+    float ss = y.x * y.x + y.y * y.y + y.z * y.z + y.w * y.w;
+#pragma unroll
+    for (int l = LANES / 2; l > 0; l >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, l);
+    const float f = a.out_scale / sqrtf(ss / (float)DV + a.eps);
+    auto gated = [&](float o, float w, float z) { return o * (f * w) * ((a.gate_kind ? 1.0f : z) / (1.0f + expf(-z))); };
+    const float r0 = gated(y.x, w.x, z[i][0].x), r1 = gated(y.y, w.y, z[i][0].y), r2 = gated(y.z, w.z, z[i][1].x), r3 = gated(y.w, w.w, z[i][1].y);
+    if (p < n) {
+      const size_t dst = (size_t)(t0 + p) * a.out_stride + (size_t)h * DV + j;
+      if (a.out_dtype == QD_F32) {
+        float2* to = reinterpret_cast<float2*>(reinterpret_cast<float*>(a.out) + dst);
+        to[0] = make_float2(r0, r1);
+        to[1] = make_float2(r2, r3);
+      } else {
+        unsigned* to = reinterpret_cast<unsigned*>(reinterpret_cast<bf16*>(a.out) + dst);
+        to[0] = lc_round2(r0, r1);
+        to[1] = lc_round2(r2, r3);
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------------ host
+// Whether the sizes are taken: whole heads of 64 x 64 (without the delta rule) or 128 x 128, and portions that are long enough on
+// the average.  Measured on a B200, us a call, chunks / token by token, 32 heads: plain, 64 x 64: 128 tokens 17.2 / 16.5, 256 18.7 / 29.2,
+// 1,500 66 / 155, three portions of 200 34 / 42, eight of 128 49 / 43; delta rule, 128 x 128: 400 tokens 85 / 87, 700 136 / 148,
+// 1,500 266 / 316, 2,048 344 / 429, three portions of 400 240 / 222.
+#define LC_MEAN_PLAIN 192
+#define LC_MEAN_DELTA 512
+static bool lc_takes(int T, int R, int d, int dv, int DP, bool delta, int nrm) {
+  return !nrm && d == DP && dv == d && (d == 128 || (d == 64 && !delta)) && (long long)T >= (long long)(delta ? LC_MEAN_DELTA : LC_MEAN_PLAIN) * R;
+}
+static long long lc_chunks(int T, int R) { return (long long)T / LC + R; }      // no fewer than there are
+
+// floats of scratch
+static long long lc_scratch(int T, int R, int H, int G, int d, bool delta) {
+  const long long c = lc_chunks(T, R);
+  long long n = c * H * LC_DEC + c * H * d * d;
+  if (delta) n += c * H * LC * d + (c * H * 3 * LC * d + c * G * 3 * LC * d) / 2;
+  return n;
+}
+
+template <int D>
+static int lc_launch(LinearChunk a, float* scratch, cudaStream_t stream) {
+  const long long c = lc_chunks(a.T, a.R);
+  if (c > 65535 || a.H > 65535 || a.R > 65535) return QD_ERR_UNSUPPORTED;
+  a.s0 = scratch;
+  a.dec = a.s0 + c * a.H * D * D;
+  a.x = a.dec + c * a.H * LC_DEC;
+  a.w = reinterpret_cast<bf16*>(a.x + c * a.H * LC * D);
+  a.kp = a.w + c * a.H * 3 * LC * D;
+  const dim3 grid((unsigned)c, a.H);
+  constexpr size_t tile = LcTile<LC, D>::ELEMS * sizeof(bf16), state = LcTile<D, D>::ELEMS * sizeof(bf16), dm = LC * LC_DM * sizeof(float);
+  constexpr size_t out = tile + (state > 2 * tile ? state : 2 * tile) + dm;
+  auto go = [&](auto kernel, dim3 g, size_t smem, int threads = LC_THREADS) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    qd_launch(kernel, g, dim3(threads), smem, stream, a);
+  };
+  if (a.beta) {
+    constexpr size_t delta = 3 * tile + (LcTile<LC_COLS, D>::ELEMS + LcTile<LC, LC_COLS>::ELEMS) * sizeof(bf16) + 2 * LC * (LC_COLS + 4) * sizeof(float);
+    if constexpr (D == 128) {
+      go(linear_chunk_solve_kernel<D, D>, grid, tile + 3 * dm);
+      go(linear_chunk_delta_kernel<D, D>, dim3(D / LC_COLS, a.H, a.R), delta);
+      go(linear_chunk_out_kernel<D, D, true>, grid, out, LC_OUT_THREADS);
+    } else {
+      return QD_ERR_UNSUPPORTED;
+    }
+  } else {
+    go(linear_chunk_add_kernel<D, D>, grid, 2 * tile);
+    go(linear_chunk_states_kernel<D, D>, dim3(D * D / 4 / LC_THREADS, a.H, a.R), 0);
+    go(linear_chunk_out_kernel<D, D, false>, grid, out, LC_OUT_THREADS);
+  }
+  return qd_last_error();
+}

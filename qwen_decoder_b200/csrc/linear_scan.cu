@@ -28,6 +28,7 @@
 // portion only: however a prompt is cut, the results agree up to the rounding of float32 sums.
 #include "common.cuh"
 #include "short_conv.cuh"
+#include "linear_chunk.cuh"
 #include <math.h>
 
 __device__ __forceinline__ void ls_st(void* p, int code, size_t i, float v) {
@@ -1000,6 +1001,8 @@ linear_step_kernel(LinearScan a, LinearFinish f, ExpGates eg) {
 // gate float32 rows ``gate_ld`` apart; norm float32 [dv] (norm_ld 0) or [H, dv] (norm_ld dv), or null; gate_kind 0 silu, 1 sigmoid.
 // ``nrm``: exponential gates.  S is [H, dv + 1, d] at ``s_off``, the maxima at ``m_off``; portions: nq scratch [T, H], g, low and k
 // as ``qd_linear_exp_gates`` and ``qd_linear_prep`` made them; single tokens: g unused, the logits are columns i_off, f_off of u.
+// ``chunk``: scratch of qd_linear_chunk_scratch floats, 16-byte aligned, for the form in chunks (linear_chunk.cuh; then o_buf and coef
+// are unused), or null.  It wants rows of v and state in 16-byte pieces, of gate in 8-byte ones, of out in pairs.
 // ``raw`` (single tokens): q and k are rows of G * d numbers ``q_ld`` apart that q_scale and k_scale still multiply.
 extern "C" int qd_linear_scan(const float* q, const float* k, const float* v, long long ldv, const float* g, int g_ld,
                               const float* beta, int T, int n_requests, int H, int G, int d, int dv, int DP,
@@ -1009,19 +1012,28 @@ extern "C" int qd_linear_scan(const float* q, const float* k, const float* v, lo
                               long long out_stride, const int* token_req, float* coef, int norm_ld, int gate_kind, int nrm,
                               float* nq, const float* low, const float* u, long long u_ld, int i_off, int f_off,
                               const float* ib, const float* fb, float cap, long long m_off, int raw, long long q_ld,
-                              float q_scale, float k_scale, cudaStream_t stream) {
+                              float q_scale, float k_scale, float* chunk, cudaStream_t stream) {
   if (T <= 0 || n_requests <= 0) return 0;
   if (H <= 0 || H > 65535 || n_requests > 65535 || G <= 0 || H % G || d <= 0 || dv <= 0 || dv > 8192 || d > DP ||
-      !state || !gate || (g_ld && g_ld != H) || (beta && T != n_requests && (!coef || ((uintptr_t)coef & 15))) || (out_dtype != QD_F32 && out_dtype != QD_BF16))
+      !state || !gate || (g_ld && g_ld != H) || (beta && T != n_requests && !chunk && (!coef || ((uintptr_t)coef & 15))) || (out_dtype != QD_F32 && out_dtype != QD_BF16))
     return QD_ERR_UNSUPPORTED;
   const bool single = T == n_requests;                // every request has at least one token
-  if (!single && !o_buf) return QD_ERR_UNSUPPORTED;
+  if (!single && !o_buf && !chunk) return QD_ERR_UNSUPPORTED;
   if (nrm && (beta || G != H || (single ? !u || !ib || !fb || !(cap > 0.f) : !nq || !low))) return QD_ERR_UNSUPPORTED;
   if (raw ? !single : (((uintptr_t)q | (uintptr_t)k) & 15) != 0) return QD_ERR_UNSUPPORTED;
   if (!g && !(nrm && single)) return QD_ERR_UNSUPPORTED;
   nrm = nrm ? 1 : 0;
   const int nc = dv + nrm;
   const int vec = d % 4 == 0 && state_stride % 4 == 0 && s_off % 4 == 0 && !((uintptr_t)state & 15);
+  if (chunk) {
+    if (single || !vec || !g || ldv % 4 || gate_ld % 2 || out_stride % 2 || (((uintptr_t)v | (uintptr_t)chunk) & 15) || ((uintptr_t)gate & 7) ||
+        ((uintptr_t)out & (out_dtype == QD_F32 ? 7 : 3)) || !lc_takes(T, n_requests, d, dv, DP, beta != nullptr, nrm))
+      return QD_ERR_UNSUPPORTED;
+    const LinearChunk c = {q, k, v, ldv, g, g_ld, beta, T, n_requests, H, G, state, state_stride, s_off, cu_tokens, slots, write_state,
+                           nullptr, nullptr, nullptr, nullptr, nullptr, gate, gate_ld, norm, norm_ld, eps, out_scale, gate_kind, out,
+                           out_dtype, out_stride};
+    return d == 64 ? lc_launch<64>(c, chunk, stream) : lc_launch<128>(c, chunk, stream);
+  }
   const LinearScan a = {q, k, v, ldv, g, g_ld, beta, coef, H, G, d, dv, state, state_stride, s_off, vec, cu_tokens, slots,
                         write_state, nrm, nq, raw, q_ld, q_scale, k_scale};
   const LinearFinish f = {gate, gate_ld, norm, norm_ld, eps, out_scale, gate_kind, nrm ? nq : nullptr, low, out, out_dtype,
@@ -1094,4 +1106,12 @@ extern "C" int qd_linear_scan(const float* q, const float* k, const float* v, lo
       qd_launch(linear_finish_kernel<32>, dim3((unsigned)((items + 7) / 8)), dim3(256), 0, stream, (const float*)o_buf, T, H, dv, f, fvec);
   }
   return qd_last_error();
+}
+
+// Floats of scratch with which qd_linear_scan takes these portions in chunks, 0: it does not.
+extern "C" long long qd_linear_chunk_scratch(int T, int n_requests, int H, int G, int d, int dv, int DP, int delta, int nrm) {
+  if (T <= 0 || n_requests <= 0 || T == n_requests || H <= 0 || G <= 0 || H > 65535 || n_requests > 65535 ||
+      lc_chunks(T, n_requests) > 65535 || !lc_takes(T, n_requests, d, dv, DP, delta != 0, nrm))
+    return 0;
+  return lc_scratch(T, n_requests, H, G, d, delta != 0);
 }

@@ -1671,6 +1671,13 @@ def linear_exp_gates(e: ExpGates, H: int, state: torch.Tensor, ctx, write_state:
     return g, inn, low
 
 
+def linear_chunk_scratch(T: int, R: int, H: int, G: int, d: int, dv: int, DP: int, delta: bool, nrm: int) -> int:
+    """Floats of scratch with which portions of T tokens of R requests go through the recurrence in chunks, 0: token by token."""
+    fn = library("linear_scan").qd_linear_chunk_scratch
+    fn.restype = ctypes.c_longlong
+    return int(fn(_I(T), _I(R), _I(H), _I(G), _I(d), _I(dv), _I(DP), _I(1 if delta else 0), _I(nrm)))
+
+
 def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: Optional[torch.Tensor], beta: Optional[torch.Tensor],
                 H: int, d: int, dv: int, state: torch.Tensor, s_off: int, ctx, write_state: bool, gate: torch.Tensor,
                 norm: Optional[torch.Tensor], eps: float, out_scale: float, out: torch.Tensor, gate_kind: int = 0,
@@ -1716,9 +1723,15 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: Optional[t
         assert beta is None and G == H and e.m_off + H <= state.shape[1]
         assert single or (low is not None and low.shape == (T, H) and low.dtype == torch.float32 and low.is_contiguous())
     new = lambda *shape: torch.empty(shape, dtype=torch.float32, device=q.device)
-    o = None if single else new(T, H * dv)
+    floats = 0
+    if not raw and v.data_ptr() % 16 == q.data_ptr() % 16 == k.data_ptr() % 16 == state.data_ptr() % 16 == 0 and v.stride(0) % 4 == 0 \
+            and state.stride(0) % 4 == s_off % 4 == 0 and gate.stride(0) % 2 == out.stride(0) % 2 == 0 and gate.data_ptr() % 8 == 0 \
+            and out.data_ptr() % (2 * out.element_size()) == 0:
+        floats = linear_chunk_scratch(T, ctx.num_requests, H, G, d, dv, DP, beta is not None, nrm)
+    chunk = new(floats) if floats else None           # long portions: in chunks
+    o = None if single or floats else new(T, H * dv)
     nq = new(T, H) if nrm and not single else None
-    coef = None if single or beta is None else new(T, H, 12)
+    coef = None if single or beta is None or floats else new(T, H, 12)
     _check(library("linear_scan").qd_linear_scan(
         _ptr(q), _ptr(k), _ptr(v), _LL(v.stride(0)), _ptr(g), _I(H if g is not None and g.dim() == 2 else 0), _ptr(beta), _I(T),
         _I(ctx.num_requests), _I(H), _I(G), _I(d), _I(dv), _I(DP), _ptr(state), _LL(state.stride(0)), _LL(s_off),
@@ -1727,9 +1740,9 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: Optional[t
         _ptr(coef), _I(dv if norm is not None and norm.numel() == H * dv else 0), _I(gate_kind), _I(nrm), _ptr(nq), _ptr(low),
         _ptr(e.u if nrm else None), _LL(e.u.stride(0) if nrm else 0), _I(e.i_off if nrm else 0), _I(e.f_off if nrm else 0),
         _ptr(e.i_bias if nrm else None), _ptr(e.f_bias if nrm else None), _F(e.cap if nrm else 1.0), _LL(e.m_off if nrm else 0),
-        _I(1 if raw else 0), _LL(q.stride(0) if raw else 0), _F(q_scale), _F(k_scale), _stream()), "linear_scan")
+        _I(1 if raw else 0), _LL(q.stride(0) if raw else 0), _F(q_scale), _F(k_scale), _ptr(chunk), _stream()), "linear_scan")
     if not single:
-        _launch_count[0] += 1 if coef is None else 2
+        _launch_count[0] += 2 if floats or coef is not None else 1
 
 
 # ------------------------------------------------------------------ norms in groups, before and after a branch

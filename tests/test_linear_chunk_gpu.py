@@ -1,0 +1,137 @@
+"""Linear attention of long portions in chunks (``csrc/linear_chunk.cuh``): against the recurrence in float64 and against the token by
+token kernels, for lengths that end anywhere in a chunk, several requests, both kinds of heads, strided rows and non-finite tokens."""
+import types
+
+import pytest
+import torch
+
+pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("guard_regions")]
+DEV = "cuda:0"
+
+
+def make(lengths, H, G, d, delta, per_token, seed=0, decay=(0.3, 1.0)):
+    T = sum(lengths)
+    g = torch.Generator(device=DEV).manual_seed(seed + T + d)
+    rnd = lambda *s: torch.empty(s, device=DEV).normal_(generator=g)
+    p = types.SimpleNamespace(H=H, G=G, d=d, lengths=lengths, T=T)
+    p.q, p.k = rnd(T, G, d), rnd(T, G, d)
+    if delta:
+        p.k /= p.k.norm(dim=-1, keepdim=True)
+    p.q *= d ** -0.5
+    p.wide = rnd(T, 2 * H * d + 8)                       # values and gate beside one another, rows with room between them
+    p.v, p.gate = p.wide[:, :H * d], p.wide[:, H * d:2 * H * d]
+    p.beta = torch.rand(T, H, device=DEV, generator=g) if delta else None
+    lo, hi = decay
+    p.g = lo + (hi - lo) * torch.rand((T, H) if per_token else (H,), device=DEV, generator=g)
+    p.norm = 1 + 0.1 * rnd(d)
+    p.state = rnd(len(lengths) + 2, H * d * d + 8)
+    cu = torch.tensor([0] + list(torch.tensor(lengths).cumsum(0)), dtype=torch.int32, device=DEV)
+    req = torch.repeat_interleave(torch.arange(len(lengths)), torch.tensor(lengths)).to(DEV, torch.int32)
+    slots = torch.arange(len(lengths), 0, -1, device=DEV).to(torch.int32)
+    p.ctx = types.SimpleNamespace(num_requests=len(lengths), cu_tokens=cu, state_slots=slots, token_request=req)
+    return p
+
+
+def run(p, monkeypatch, chunks, dtype=torch.float32, write=True, norm=True):
+    from qwen_decoder_b200 import kernels
+    state = p.state.clone()
+    room = torch.empty(p.T, p.H * p.d + 2, dtype=dtype, device=DEV)
+    out = room[:, :p.H * p.d]
+    asked, real = [], kernels.linear_chunk_scratch
+    def scratch(*a):
+        asked.append(real(*a))
+        return asked[-1] if chunks else 0
+    with monkeypatch.context() as m:
+        m.setattr(kernels, "linear_chunk_scratch", scratch)
+        kernels.linear_scan(p.q, p.k, p.v, p.g, p.beta, p.H, p.d, p.d, state, 4, p.ctx, write, p.gate, p.norm if norm else None, 1e-5, 0.7, out)
+    torch.cuda.synchronize()
+    return out, state, asked[0]
+
+
+def reference(p, norm=True):
+    H, G, d = p.H, p.G, p.d
+    out = torch.empty(p.T, H, d, dtype=torch.float64)
+    states = p.state.double().cpu().clone()
+    q, k = (x.double().cpu().repeat_interleave(H // G, dim=1) for x in (p.q, p.k))
+    v = p.v.double().cpu().view(p.T, H, d)
+    g = p.g.double().cpu().expand(p.T, H)
+    t = 0
+    for r, n in enumerate(p.lengths):
+        slot = int(p.ctx.state_slots[r])
+        S = states[slot, 4:4 + H * d * d].view(H, d, d).transpose(1, 2).clone()          # [H, keys, values]
+        for _ in range(n):
+            S = g[t][:, None, None] * S
+            x = v[t]
+            if p.beta is not None:
+                x = p.beta[t].double().cpu()[:, None] * (x - (S.transpose(1, 2) @ k[t][:, :, None])[..., 0])
+            S = S + k[t][:, :, None] * x[:, None, :]
+            out[t] = (S.transpose(1, 2) @ q[t][:, :, None])[..., 0]
+            t += 1
+        states[slot, 4:4 + H * d * d] = S.transpose(1, 2).reshape(-1)
+    out = out / torch.sqrt((out * out).mean(-1, keepdim=True) + 1e-5)
+    if norm:
+        out = out * p.norm.double().cpu()
+    z = p.gate.double().cpu().view(p.T, H, d)
+    return (out * z * torch.sigmoid(z) * 0.7).view(p.T, -1), states
+
+
+CASES = [([192], 2, 2, 64, False, False), ([300], 4, 2, 64, False, True), ([64, 1, 303, 400], 2, 1, 64, False, True), ([229, 160], 2, 2, 128, False, True),
+         ([513], 2, 1, 128, True, True), ([520], 4, 2, 128, True, False), ([127, 1, 1408], 2, 2, 128, True, True)]
+
+
+@pytest.mark.parametrize("lengths,H,G,d,delta,per_token", CASES)
+def test_against_float64(lengths, H, G, d, delta, per_token, monkeypatch):
+    p = make(lengths, H, G, d, delta, per_token)
+    want, states = reference(p)
+    got, state, floats = run(p, monkeypatch, True)
+    old, old_state, _ = run(p, monkeypatch, False)
+    assert floats > 0
+    err = lambda a, b: float((a.double().cpu() - b).norm() / b.norm())
+    # no further from float64 than the kernels that go token by token, but for a unit in the last place of float32
+    assert err(got, want) <= max(err(old, want), 2.0 ** -22), (err(got, want), err(old, want))
+    assert err(state, states) <= max(err(old_state, states), 2.0 ** -22), (err(state, states), err(old_state, states))
+    assert torch.equal(state[0], p.state[0]) and torch.equal(state[:, :4], p.state[:, :4])             # nobody else's
+
+
+@pytest.mark.parametrize("d,delta", [(64, False), (128, True)])
+def test_options(d, delta, monkeypatch):
+    p = make([980, 100], 2, 1, d, delta, True, seed=5)
+    want, _ = reference(p, norm=False)
+    got, state, _ = run(p, monkeypatch, True, dtype=torch.bfloat16, write=False, norm=False)
+    assert torch.equal(state, p.state)
+    assert float((got.double().cpu() - want).norm() / want.norm()) <= 2.0 ** -8
+    few = make([100, 100], 2, 1, d, delta, True)
+    assert run(few, monkeypatch, True)[2] == 0                                             # short portions go token by token
+
+
+@pytest.mark.parametrize("d,delta", [(64, False), (128, True)])
+@pytest.mark.parametrize("what", ["v", "k", "g"])
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.4e38])
+def test_tokens_before_a_bad_one(d, delta, what, value, monkeypatch):
+    p = make([960, 70], 2, 2, d, delta, True, seed=9, decay=(0.9, 1.0))
+    good, _, _ = run(p, monkeypatch, True)
+    at = 64 + 37
+    if what == "v":
+        p.v[at, 3] = value
+    elif what == "k":
+        p.k[at, 0, 5] = value
+    elif value == 3.4e38:
+        return
+    else:
+        p.g[at, 0] = value
+    got, state, _ = run(p, monkeypatch, True)
+    # tokens before it, and the other request: another order of sums at most
+    for a in (slice(0, at), slice(960, 1030)):
+        assert torch.isfinite(got[a]).all()
+        assert float((got[a] - good[a]).norm() / good[a].norm()) <= 1e-5
+
+
+def test_decays_of_all_sizes(monkeypatch):
+    """Decays whose products leave float32 within a chunk."""
+    for delta, d in ((False, 64), (True, 128)):
+        p = make([530], 2, 2, d, delta, True, seed=3, decay=(0.0, 0.3))
+        p.g[40:60] = 0.0
+        want, states = reference(p)
+        got, state, _ = run(p, monkeypatch, True)
+        assert float((got.double().cpu() - want).norm() / want.norm()) <= 1e-5
+        assert float((state.double().cpu() - states).norm() / states.norm()) <= 1e-6
