@@ -263,6 +263,50 @@ linear_prep_walk_kernel(LinearPrep a) {
   }
 }
 
+// Portions without a convolution (q and k alone; v and the gates stay where the product left them): DP / 4 neighbouring lanes a
+// (token, head), four neighbouring elements a lane, the partner of a half-split pair a shuffle away.  d = DP, 32, 64 or 128.
+// (1,500 tokens of 32 + 32 heads of 64: 12.5 us where the walk took 30.)
+template <int DP>
+__global__ void __launch_bounds__(256)
+linear_prep_heads_kernel(LinearPrep a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  constexpr int LANES = DP / 4;
+  const int lane = threadIdx.x & 31, l = lane % LANES, i = l * 4, half = a.rotary_dim / 2;
+  long long item = ((long long)blockIdx.x * 256 + threadIdx.x) / LANES;
+  const bool there = item < 2ll * a.T * a.G;
+  if (!there) item = 0;
+  const int t = (int)(item / (2 * a.G)), s = (int)(item - (long long)t * 2 * a.G), head = s < a.G ? s : s - a.G;
+  float4 x = *reinterpret_cast<const float4*>(a.u + (size_t)t * a.ld + (size_t)s * DP + i);
+  float f = s < a.G ? a.q_scale : a.k_scale;
+  if (a.unit) {
+    float ss = x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    f *= 1.0f / sqrtf(ss + a.unit_eps);
+  }
+  if (s >= a.G && a.k_mul) f *= a.k_mul[(size_t)t * a.G + head];
+  if (half) {
+    const size_t tab = (size_t)a.positions[t] * half;
+    if (a.pairing == 1) {
+      const bool low = i < half;
+      const int from = (lane - l + (low ? l + half / 4 : l - half / 4)) & 31;
+      const float4 y = make_float4(__shfl_sync(0xffffffffu, x.x, from), __shfl_sync(0xffffffffu, x.y, from),
+                                   __shfl_sync(0xffffffffu, x.z, from), __shfl_sync(0xffffffffu, x.w, from));
+      if (i < 2 * half) {
+        const float4 c = *reinterpret_cast<const float4*>(a.cos_t + tab + (low ? i : i - half));
+        const float4 n = *reinterpret_cast<const float4*>(a.sin_t + tab + (low ? i : i - half));
+        if (low) x = make_float4(x.x * c.x - y.x * n.x, x.y * c.y - y.y * n.y, x.z * c.z - y.z * n.z, x.w * c.w - y.w * n.w);
+        else x = make_float4(x.x * c.x + y.x * n.x, x.y * c.y + y.y * n.y, x.z * c.z + y.z * n.z, x.w * c.w + y.w * n.w);
+      }
+    } else if (i < 2 * half) {
+      const float2 c = *reinterpret_cast<const float2*>(a.cos_t + tab + i / 2), n = *reinterpret_cast<const float2*>(a.sin_t + tab + i / 2);
+      x = make_float4(x.x * c.x - x.y * n.x, x.y * c.x + x.x * n.x, x.z * c.y - x.w * n.y, x.w * c.y + x.z * n.y);
+    }
+  }
+  if (there) *reinterpret_cast<float4*>((s < a.G ? a.q : a.k) + ((size_t)t * a.G + head) * DP + i) = make_float4(x.x * f, x.y * f, x.z * f, x.w * f);
+}
+
 // grid (ceil(C / 256), requests): one thread per (request, channel) moves the channel's taps - 1 kept inputs on.
 __global__ void __launch_bounds__(256)
 linear_prep_state_kernel(const float* __restrict__ u, long long ld, int C, int taps, float* __restrict__ state,
@@ -313,7 +357,16 @@ extern "C" int qd_linear_prep(const float* u, long long ld, int T, int n_request
   // from 4 tokens of a CTA on, a thread that stays on its channel is the faster form; heads of 96 or 256 do not fill its rows
   const bool walks = !advance && tokens >= 4 && DP <= LP_THREADS && LP_THREADS % DP == 0;
   const size_t walk_smem = ((size_t)tokens * d + tokens) * sizeof(float);
-  if (walks && taps == 0) qd_launch(linear_prep_walk_kernel<0>, grid, dim3(LP_THREADS), walk_smem, stream, a);
+  const bool by_heads = taps == 0 && d == DP && (DP == 32 || DP == 64 || DP == 128) && b_off < 0 && a_off < 0 && ld % 4 == 0 &&
+                        !(((uintptr_t)u | (uintptr_t)q | (uintptr_t)k) & 15) && rotary_dim % (pairing == 1 ? 8 : 4) == 0 &&
+                        !(rotary_dim && (((uintptr_t)cos_t | (uintptr_t)sin_t) & 15));
+  if (by_heads) {
+    const dim3 heads((unsigned)((2ll * T * G * (DP / 4) + 255) / 256));
+    if (DP == 32) qd_launch(linear_prep_heads_kernel<32>, heads, dim3(256), 0, stream, a);
+    else if (DP == 64) qd_launch(linear_prep_heads_kernel<64>, heads, dim3(256), 0, stream, a);
+    else qd_launch(linear_prep_heads_kernel<128>, heads, dim3(256), 0, stream, a);
+  }
+  else if (walks && taps == 0) qd_launch(linear_prep_walk_kernel<0>, grid, dim3(LP_THREADS), walk_smem, stream, a);
   else if (walks && taps == 2) qd_launch(linear_prep_walk_kernel<2>, grid, dim3(LP_THREADS), walk_smem, stream, a);
   else if (walks && taps == 3) qd_launch(linear_prep_walk_kernel<3>, grid, dim3(LP_THREADS), walk_smem, stream, a);
   else if (walks && taps == 4) qd_launch(linear_prep_walk_kernel<4>, grid, dim3(LP_THREADS), walk_smem, stream, a);

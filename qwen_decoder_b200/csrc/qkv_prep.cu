@@ -146,6 +146,72 @@ qkv_prep_kernel(QkvPrep a) {
   }
 }
 
+// Without a convolution and without a norm over the whole projection: a warp per (token, head), a lane four neighbouring elements,
+// the partner of a half-split pair a shuffle away.  Heads and values of up to 128, sizes and halves multiples of 4, all rows in
+// 16-byte pieces.  (A CTA per token that first lays the row down in shared memory took 28 us for 1,500 tokens of 16 + 2 + 2 heads of 128,
+// whose bytes take 4; so 10.)
+__global__ void __launch_bounds__(256)
+qkv_prep_heads_kernel(QkvPrep a, int T) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int H = a.H, G = a.G, d = a.d, vd = a.vd, lane = threadIdx.x & 31, i = lane * 4, heads = H + (a.write_kv ? 2 * G : 0);
+  const long long item = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (item >= (long long)T * heads) return;
+  const int t = (int)(item / heads), s = (int)(item - (long long)t * heads);
+  const bool is_q = s < H, is_v = s >= H + G;
+  const int width = is_v ? vd : d, first = is_q ? s * d : is_v ? (H + G) * d + (s - H - G) * vd : s * d;
+  const bool there = i < width;
+  float4 x = there ? *reinterpret_cast<const float4*>(a.u + (size_t)t * a.ld + first + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  size_t dst = (size_t)t * H * d + (size_t)s * d + i;
+  if (!is_q) {
+    const size_t slot = (size_t)a.slot_map[t], page = slot / a.page_size, off = slot - page * a.page_size;
+    dst = page * G * a.page_size * (d + vd) + (is_v ? (size_t)G * a.page_size * d + ((size_t)(s - H - G) * a.page_size + off) * vd
+                                                    : ((size_t)(s - H) * a.page_size + off) * d) + i;
+  }
+  if (!is_v) {
+    const int half = a.rotary_dim / 2;
+    auto norm = [&]() {
+      const float f = 1.0f / sqrtf(warp_sum(x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w) / (float)d + a.eps);
+      x = make_float4(x.x * f, x.y * f, x.z * f, x.w * f);
+    };
+    if (a.norm_mode == 2 && !a.norm_after) norm();
+    if (half) {
+      const size_t tab = (size_t)a.positions[t] * half;
+      if (a.pairing == 1) {
+        // the first half of the rotated part turns to x cos - y sin, the second to y cos + x sin
+        const bool low = i < half, turned = i < 2 * half;
+        const int from = low ? lane + half / 4 : lane - half / 4;
+        const float4 y = make_float4(__shfl_sync(0xffffffffu, x.x, from & 31), __shfl_sync(0xffffffffu, x.y, from & 31),
+                                     __shfl_sync(0xffffffffu, x.z, from & 31), __shfl_sync(0xffffffffu, x.w, from & 31));
+        if (turned) {
+          const float4 c = *reinterpret_cast<const float4*>(a.cos_t + tab + (low ? i : i - half));
+          const float4 n = *reinterpret_cast<const float4*>(a.sin_t + tab + (low ? i : i - half));
+          if (low) x = make_float4(x.x * c.x - y.x * n.x, x.y * c.y - y.y * n.y, x.z * c.z - y.z * n.z, x.w * c.w - y.w * n.w);
+          else x = make_float4(x.x * c.x + y.x * n.x, x.y * c.y + y.y * n.y, x.z * c.z + y.z * n.z, x.w * c.w + y.w * n.w);
+        }
+      } else if (i < 2 * half) {
+        const float2 c = *reinterpret_cast<const float2*>(a.cos_t + tab + i / 2), n = *reinterpret_cast<const float2*>(a.sin_t + tab + i / 2);
+        x = make_float4(x.x * c.x - x.y * n.x, x.y * c.x + x.x * n.x, x.z * c.y - x.w * n.y, x.w * c.y + x.z * n.y);
+      }
+    }
+    if (a.norm_mode == 2 && a.norm_after) norm();
+  }
+  if (!there) return;
+  void* out = is_q ? a.q_out : a.kv;
+  if ((is_q ? a.q_dtype : a.kv_dtype) == QD_F32) {
+    *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + dst) = x;
+  } else {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(x.x, x.y), hi = __floats2bfloat162_rn(x.z, x.w);
+    *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(out) + dst) =
+        make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+  }
+}
+static bool qkv_heads_ok(const QkvPrep& a) {
+  const uintptr_t all = (uintptr_t)a.u | (uintptr_t)a.q_out | (a.write_kv ? (uintptr_t)a.kv : 0) | (a.rotary_dim ? (uintptr_t)a.cos_t | (uintptr_t)a.sin_t : 0);
+  return a.taps == 0 && a.norm_mode != 1 && a.d % 4 == 0 && a.d <= 128 && a.vd % 4 == 0 && a.vd <= 128 && a.ld % 4 == 0 && !(all & 15) &&
+         a.rotary_dim % (a.pairing == 1 ? 8 : 4) == 0;
+}
+
 // grid (ceil(C / 256), requests): one thread per (request, channel) moves the channel's taps - 1 kept inputs on.
 __global__ void __launch_bounds__(256)
 qkv_prep_state_kernel(const float* __restrict__ u, long long ld, int C, int taps, float* __restrict__ state,
@@ -189,6 +255,11 @@ extern "C" int qd_qkv_prep(const float* u, long long ld, int T, int n_requests, 
   QkvPrep a = {u, ld, H, G, d, vd, taps, conv_w, state, state_stride, state_off, token_req, cu_tokens, slots, advance,
                norm_mode, norm_after, wq, wk, eps, rotary_dim, pairing, cos_t, sin_t, positions, q_out, q_dtype, kv,
                kv_dtype, slot_map, page_size, write_kv};
+  if (qkv_heads_ok(a)) {
+    const long long items = (long long)T * (H + (write_kv ? 2 * G : 0));
+    qd_launch(qkv_prep_heads_kernel, dim3((unsigned)((items + 7) / 8)), dim3(256), 0, stream, a, T);
+    return qd_last_error();
+  }
   if (d <= 128) qd_launch(qkv_prep_kernel<2>, dim3(T), dim3(threads), smem, stream, a);
   else qd_launch(qkv_prep_kernel<QP_MAX_D / 64>, dim3(T), dim3(threads), smem, stream, a);
   if (update_state && taps > 1 && !advance)
