@@ -22,6 +22,9 @@
 //            are complete by then, so the softmax threads never wait for them.  With both A operands in tensor
 //            memory an MMA reads 4 KB of shared memory, not 8
 // Tensor memory: columns 0..255 the two S/P buffers, 256..383 O, 384..447 Q.  Shared memory: 3 stages of K and V.
+// EXT (an instance of its own) is the attention of attention_sink.cu with sinks, blocks, gates and two-piece weights: 1,500 tokens of
+// 16 + 2 heads of 128 in blocks of 1,024 take 36 us where its mma.sync form takes 87 (bound by its longest rows of tiles, as
+// above; the prompt of eight mixed layers 3.72 ms, with the preparation by heads and this 3.43).
 // Formulas: gpu_kernels.cu:223-311 of the reference (scores q.k / sqrt(d), causal, softmax, weighted sum).
 // Keys past a row's position are masked on the scores; their V rows are whatever finite values the
 // pages hold (the cache starts as zeros and is only ever written with finite numbers), times zero.
@@ -145,6 +148,11 @@ __device__ __forceinline__ void at_tmem_ld(unsigned taddr, float (&v)[N]) {
 }
 __device__ __forceinline__ void at_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void at_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ bool at_elect() {         // one lane of a whole warp
+  unsigned one;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+  return one;
+}
 __device__ __forceinline__ float at_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -172,6 +180,13 @@ struct AtParams {
   int R, H, G, page_size, window, tok_tile;
   float scale_log2e;
   int* status;
+  // EXT: more than the dense decoder's attention (attention_sink.cu states it): a query sees only the keys of its own block of
+  // ``chunk`` positions (0: all), exp(sink of the head) joins the denominator, the output row is multiplied by ``out_scale`` and
+  // the sigmoid of a logit per head or per element, rows of out ``out_stride`` apart; a weight enters the product as two bfloat16
+  // numbers (p = hi + lo), hi over the first half of its tile's scores and lo over the second
+  int chunk, gate_elem;
+  const float *sinks, *gate; long long gate_ld;
+  float out_scale; long long out_stride;
   // null, or nanosecond stamps for measurements: [0, 128) 16 x 8 of row 0's softmax thread and [128, 192) 16 x 4
   // of the MMA thread of the CTA of KV head 0 whose rows end at key 2047 (16 key tiles; slot 7 of the first seven
   // tiles holds the CTA's own phases: start, tensor memory allocated, request found, Q stored, last P stored, last
@@ -179,7 +194,15 @@ struct AtParams {
   long long* timeline;
 };
 
-template <int HD, int TPR>
+// The first key a query at ``pos`` sees.
+template <bool EXT>
+__device__ __forceinline__ int at_key_lo(const AtParams& p, int pos) {
+  int lo = p.window > 0 && pos - p.window + 1 > 0 ? pos - p.window + 1 : 0;
+  if (EXT && p.chunk > 0) lo = max(lo, pos - pos % p.chunk);
+  return lo;
+}
+
+template <int HD, int TPR, bool EXT>
 __global__ void __launch_bounds__(AT_THREADS_OF(TPR), 1)
 prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap kv_map, const AtParams p) {
   constexpr int AT_SOFTMAX_THREADS = AT_SOFTMAX_THREADS_OF(TPR);
@@ -266,7 +289,7 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap kv_map, const A
   }
   pdl_wait();
   const int key_hi = pos0 + n_tok;
-  const int key_lo_tile = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
+  const int key_lo_tile = at_key_lo<EXT>(p, pos0);
   const int kt_lo = key_lo_tile / AT_KEYS, kt_hi = idle ? kt_lo : (key_hi + AT_KEYS - 1) / AT_KEYS;
   const int n_kt = kt_hi - kt_lo;
 
@@ -310,7 +333,9 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap kv_map, const A
     }
   } else if (warp == W_MMA) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && !idle) {
+    // The whole warp goes through the tiles, one lane issues: with the loop in one lane alone an MMA cost 62 cycles of issue.
+    if (!idle) {
+      const bool one = at_elect();
       const unsigned idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(AT_KEYS >> 3) << 17) | ((unsigned)(AT_ROWS >> 4) << 24);
       const unsigned idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((unsigned)(HD >> 3) << 17) |
                                 ((unsigned)(AT_ROWS >> 4) << 24);
@@ -335,14 +360,16 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap kv_map, const A
           at_umma_ta(tmem + (unsigned)(j & 1) * AT_KEYS, tmem + T_Q + (unsigned)k * 8, k_lo + adv, desc_hi, idesc_qk, k ? 1u : 0u);
         }
       };
-      const bool mstamp = p.timeline && blockIdx.y == 0 && n_kt >= 16 && pos0 + n_tok == n_kt * AT_KEYS;
+      const bool mstamp = one && p.timeline && blockIdx.y == 0 && n_kt >= 16 && pos0 + n_tok == n_kt * AT_KEYS;
       if (!at_mbar_wait(&q_full, 0, &dead)) atomicCAS(p.status, 0, 3);
       for (int j = 0; j < 2; j++) {                     // slots -2 and -1: the first two tiles' scores
         slot_ready(j - 2);
         at_fence_after();
-        if (j < n_kt) scores(j);
-        at_commit(&kv_empty[j % NS]);
-        if (j < n_kt) at_commit(&s_full[j & 1]);
+        if (one) {
+          if (j < n_kt) scores(j);
+          at_commit(&kv_empty[j % NS]);
+          if (j < n_kt) at_commit(&s_full[j & 1]);
+        }
       }
       for (int j = 0; j < n_kt; j++) {
         const int s = (j + 2) % NS;
@@ -352,18 +379,23 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap kv_map, const A
         slot_ready(j);
         at_fence_after();
         const unsigned v_lo = v_lo0 + (unsigned)s * (TILE_BYTES >> 4);
+        if (one) {
 #pragma unroll
-        for (int k = 0; k < AT_KEYS / 16; k++) {
-          // 16 keys = two groups of 8 rows of V (2,048 bytes); P of this tile lies where its scores were: 16 keys
-          // = 8 columns of bfloat16 pairs per step
-          at_umma_ta(tmem + T_O, tmem + (unsigned)(j & 1) * AT_KEYS + (unsigned)k * 8, v_lo + (unsigned)k * (2048 >> 4), desc_hi,
-                      idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < AT_KEYS / 16; k++) {
+            // 16 keys = two groups of 8 rows of V (2,048 bytes); P of this tile lies where its scores were: 16 keys
+            // = 8 columns of bfloat16 pairs per step
+            at_umma_ta(tmem + T_O, tmem + (unsigned)(j & 1) * AT_KEYS + (unsigned)k * 8, v_lo + (unsigned)k * (2048 >> 4), desc_hi,
+                        idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
+            if (EXT)
+              at_umma_ta(tmem + T_O, tmem + (unsigned)(j & 1) * AT_KEYS + AT_KEYS / 2 + (unsigned)k * 8, v_lo + (unsigned)k * (2048 >> 4),
+                         desc_hi, idesc_pv, 1u);
+          }
+          if (mstamp) p.timeline[128 + j * 4 + 2] = at_now();
+          at_commit(j + 1 < n_kt ? &o_done : &o_last);
+          if (j + 2 < n_kt) scores(j + 2);
+          at_commit(&kv_empty[s]);
+          if (j + 2 < n_kt) at_commit(&s_full[j & 1]);
         }
-        if (mstamp) p.timeline[128 + j * 4 + 2] = at_now();
-        at_commit(j + 1 < n_kt ? &o_done : &o_last);
-        if (j + 2 < n_kt) scores(j + 2);
-        at_commit(&kv_empty[s]);
-        if (j + 2 < n_kt) at_commit(&s_full[j & 1]);
         if (mstamp) p.timeline[128 + j * 4 + 3] = at_now();
       }
     }
@@ -374,7 +406,7 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap kv_map, const A
     const int t = row / gs, hh = row - t * gs;
     const bool ok = !idle && t < n_tok;
     const int pos = pos0 + t;
-    const int lo = (p.window > 0 && pos - p.window + 1 > 0) ? pos - p.window + 1 : 0;
+    const int lo = at_key_lo<EXT>(p, pos);
     const unsigned t_lane = tmem + ((unsigned)((warp & 3) * 32) << 16);      // this warp's 32 lanes
     // this thread's share of the Q row into tensor memory: bfloat16 pairs as they lie in memory, a pair a column
     {
@@ -398,7 +430,7 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap kv_map, const A
     // keys every valid row of the tile sees need no test: all up to the first row's position and, with a
     // window, from the last row's first visible key on
     const int free_hi = pos0 + 1;
-    const int free_lo = (p.window > 0 && key_hi - p.window > 0) ? key_hi - p.window : 0;
+    const int free_lo = at_key_lo<EXT>(p, key_hi - 1);
     for (int j = 0; j < n_kt; j++) {
       const int tile_base = (kt_lo + j) * AT_KEYS;
       const int key_base = tile_base + h * KQ;
@@ -455,7 +487,7 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap kv_map, const A
       }
       const float ref = m == -INFINITY ? 0.f : m;
       // p = exp2(score - max) as bfloat16 pairs, kept in registers until the P tile is free
-      unsigned pk[KQ / 2];
+      unsigned pk[KQ / 2], pl[EXT ? KQ / 2 : 1];      // (EXT: and what the rounding left)
       float sum = 0.f;
       const float mul = interior ? p.scale_log2e : 1.0f;
 #pragma unroll
@@ -463,6 +495,7 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap kv_map, const A
         const float p0 = at_exp2(fmaf(sv[2 * i], mul, -ref)), p1 = at_exp2(fmaf(sv[2 * i + 1], mul, -ref));
         sum += p0 + p1;
         pk[i] = at_pack(p0, p1);
+        if (EXT) pl[EXT ? i : 0] = at_pack(p0 - __uint_as_float(pk[i] << 16), p1 - __uint_as_float(pk[i] & 0xFFFF0000u));
       }
       l += sum;
       if (stamp) p.timeline[j * 8 + 4] = at_now();
@@ -470,6 +503,19 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap kv_map, const A
       // its scores in registers since the barrier above): the product reads it from there as its A operand and
       // nothing passes through shared memory
       at_tmem_st<KQ / 2>(t_lane + (unsigned)(j & 1) * AT_KEYS + h * (KQ / 2), pk);
+      if constexpr (EXT) at_tmem_st<KQ / 2>(t_lane + (unsigned)(j & 1) * AT_KEYS + AT_KEYS / 2 + h * (KQ / 2), pl);
+      if (EXT && (tile_base < key_lo_tile || tile_base + AT_KEYS > key_hi)) {
+        // Values of keys that the tile's rows do not see are nobody's, or another request's, and may be no numbers: their weights
+        // are zero, and so are they.  (The stage is not taken back before the product that waits for P.)
+        const int i = j + 2;
+        if (!at_mbar_wait(&kv_full[i % NS], (i / NS) & 1, &dead) && lane == 0) atomicCAS(p.status, 0, 10);
+        unsigned char* v = v_s + (i % NS) * TILE_BYTES;
+        for (int e = threadIdx.x; e < AT_KEYS * NB * 8; e += AT_SOFTMAX_THREADS) {
+          const int key = tile_base + (e >> 3) % AT_KEYS;
+          if (key < key_lo_tile || key >= key_hi) *reinterpret_cast<uint4*>(v + e * 16) = make_uint4(0, 0, 0, 0);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      }
       at_fence_before();
       at_mbar_arrive(&p_full[j & 1]);
       if (stamp) p.timeline[j * 8 + 5] = at_now();
@@ -486,8 +532,18 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap kv_map, const A
       float l_all = l;
 #pragma unroll
       for (int o2 = 1; o2 < TPR; o2++) l_all += l_s[(h + o2) % TPR][row];
-      const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
-      bf16* d = p.out + (size_t)(tok0 + t) * p.H * HD + (size_t)(g * gs + hh) * HD + h * DH;
+      float inv = l_all > 0.f ? 1.f / l_all : 0.f;
+      bf16* d = p.out + (size_t)(tok0 + t) * (EXT ? p.out_stride : (long long)p.H * HD) + (size_t)(g * gs + hh) * HD + h * DH;
+      const float* gate = nullptr;
+      if (EXT && ok) {
+        if (p.sinks) {
+          const float sk = p.sinks[g * gs + hh] * 1.4426950408889634f, mn = fmaxf(m, sk), f = at_exp2(m - mn);
+          inv = f / (l_all * f + at_exp2(sk - mn));
+        }
+        inv *= p.out_scale;
+        if (p.gate && p.gate_elem) gate = p.gate + (size_t)(tok0 + t) * p.gate_ld + (size_t)(g * gs + hh) * HD + h * DH;
+        else if (p.gate) inv *= 1.0f / (1.0f + expf(-p.gate[(size_t)(tok0 + t) * p.gate_ld + g * gs + hh]));
+      }
 #pragma unroll
       for (int c = 0; c < DH; c += 32) {
         float ov[32];
@@ -495,6 +551,16 @@ prefill_attention_tc5_kernel(const __grid_constant__ CUtensorMap kv_map, const A
         if (ok) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {
+            if (EXT && gate) {
+#pragma unroll
+              for (int e = 0; e < 8; e += 4) {
+                const float4 z = *reinterpret_cast<const float4*>(gate + c + i + e);
+                ov[i + e] *= 1.0f / (1.0f + expf(-z.x));
+                ov[i + e + 1] *= 1.0f / (1.0f + expf(-z.y));
+                ov[i + e + 2] *= 1.0f / (1.0f + expf(-z.z));
+                ov[i + e + 3] *= 1.0f / (1.0f + expf(-z.w));
+              }
+            }
             uint4 v;
             v.x = at_pack(ov[i] * inv, ov[i + 1] * inv);
             v.y = at_pack(ov[i + 2] * inv, ov[i + 3] * inv);
@@ -553,10 +619,10 @@ static int* at_status_word() {
   return words[dev];
 }
 
-template <int HD, int TPR>
+template <int HD, int TPR, bool EXT>
 static int at_launch(const CUtensorMap& map, const AtParams& p, int tiles, cudaStream_t stream) {
   size_t smem = 1024 + (size_t)(2 * AT_STAGES) * AT_ROWS * HD * 2;
-  auto kernel = prefill_attention_tc5_kernel<HD, TPR>;
+  auto kernel = prefill_attention_tc5_kernel<HD, TPR, EXT>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     cudaGetLastError();
     return QD_ERR_UNSUPPORTED;
@@ -570,6 +636,8 @@ static int at_launch(const CUtensorMap& map, const AtParams& p, int tiles, cudaS
 // head (a tile's 128 rows hold floor(128 / group) tokens x the group's heads; with a group that does not
 // divide 128 the last rows of a tile stay empty: 2 of 128 at 7 heads, 3 at 5), page sizes that are multiples
 // of 16; refuses the rest (the caller has another kernel).
+static int at_go(const void* kv, long long n_pages, int d, AtParams& p, int T, float scale, bool ext, cudaStream_t stream);
+
 extern "C" int qd_prefill_attention_tc5(const void* q, long long q_stride, void* out, const void* kv, long long n_pages,
                                         const int* block_table, int max_blocks, const int* cu_tokens,
                                         const int* start_pos, int R, int T, int H, int G, int d, int page_size,
@@ -579,12 +647,21 @@ extern "C" int qd_prefill_attention_tc5(const void* q, long long q_stride, void*
   const int gs = H / G;
   if (gs > 16) return QD_ERR_UNSUPPORTED;
   if (((uintptr_t)q & 15) || ((uintptr_t)kv & 15) || ((uintptr_t)out & 15) || q_stride % 8 != 0) return QD_ERR_UNSUPPORTED;
+  AtParams p = {};
+  p.q = (const bf16*)q; p.q_stride = q_stride; p.out = (bf16*)out;
+  p.block_table = block_table; p.max_blocks = max_blocks; p.cu_tokens = cu_tokens; p.start_pos = start_pos;
+  p.R = R; p.H = H; p.G = G; p.page_size = page_size; p.window = window;
+  p.timeline = timeline;
+  return at_go(kv, n_pages, d, p, T, scale, false, stream);
+}
+
+static int at_go(const void* kv, long long n_pages, int d, AtParams& p, int T, float scale, bool ext, cudaStream_t stream) {
   AtEncodeFn fn = at_encode_fn();
   int* status = at_status_word();
   if (!fn || !status) return QD_ERR_UNSUPPORTED;
   // the cache as rows of d: [pages * 2 * G * page_size][d]; a box is 16 rows x 64 columns
   CUtensorMap map;
-  cuuint64_t dims[2] = {(cuuint64_t)d, (cuuint64_t)(n_pages * 2 * G * page_size)};
+  cuuint64_t dims[2] = {(cuuint64_t)d, (cuuint64_t)(n_pages * 2 * p.G * p.page_size)};
   cuuint64_t strides[1] = {(cuuint64_t)d * 2};
   cuuint32_t box[2] = {64, 16};
   cuuint32_t estr[2] = {1, 1};
@@ -592,15 +669,33 @@ extern "C" int qd_prefill_attention_tc5(const void* q, long long q_stride, void*
          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return QD_ERR_UNSUPPORTED;
-  AtParams p;
-  p.q = (const bf16*)q; p.q_stride = q_stride; p.out = (bf16*)out;
-  p.block_table = block_table; p.max_blocks = max_blocks; p.cu_tokens = cu_tokens; p.start_pos = start_pos;
-  p.R = R; p.H = H; p.G = G; p.page_size = page_size; p.window = window; p.tok_tile = AT_ROWS / gs;
+  p.tok_tile = AT_ROWS / (p.H / p.G);
   p.scale_log2e = scale * 1.4426950408889634f;
   p.status = status;
-  p.timeline = timeline;
-  const int tiles = (T + p.tok_tile - 1) / p.tok_tile + R;      // upper bound on the tiles of R requests
-  return d == 64 ? at_launch<64, 2>(map, p, tiles, stream) : at_launch<128, 2>(map, p, tiles, stream);
+  const int tiles = (T + p.tok_tile - 1) / p.tok_tile + p.R;      // upper bound on the tiles of R requests
+  if (ext) return d == 64 ? at_launch<64, 2, true>(map, p, tiles, stream) : at_launch<128, 2, true>(map, p, tiles, stream);
+  return d == 64 ? at_launch<64, 2, false>(map, p, tiles, stream) : at_launch<128, 2, false>(map, p, tiles, stream);
+}
+
+// The same for attention_sink.cu's attention where keys and values have one size, a multiple of 16 keys to a page, and scores no cap:
+// q [T, H * d] dense, out rows ``out_stride`` apart, pages of [G, page_size, d] keys and then [G, page_size, d] values; sinks float32
+// [H] or null; chunk, gate, gate_ld, gate_elem, out_scale as qd_sink_attention_mma.  gate rows in 16-byte pieces with ``gate_elem``.
+extern "C" int qd_sink_attention_tc5(const void* q, void* out, long long out_stride, const void* kv, long long n_pages, const int* block_table,
+                                     int max_blocks, const int* cu_tokens, const int* start_pos, int R, int T, int H, int G, int d,
+                                     int page_size, float scale, int window, const float* sinks, int chunk, const float* gate,
+                                     long long gate_ld, int gate_elem, float out_scale, cudaStream_t stream) {
+  if (T <= 0 || R <= 0) return 0;
+  if (G < 1 || H % G != 0 || H / G > 16 || page_size % 16 != 0 || (d != 64 && d != 128) || n_pages < 1 || chunk < 0 || window < 0)
+    return QD_ERR_UNSUPPORTED;
+  if ((((uintptr_t)q | (uintptr_t)kv | (uintptr_t)out) & 15) || out_stride % 8 != 0 ||
+      (gate && gate_elem && (((uintptr_t)gate & 15) || gate_ld % 4)))
+    return QD_ERR_UNSUPPORTED;
+  AtParams p = {};
+  p.q = (const bf16*)q; p.q_stride = (long long)H * d; p.out = (bf16*)out; p.out_stride = out_stride;
+  p.block_table = block_table; p.max_blocks = max_blocks; p.cu_tokens = cu_tokens; p.start_pos = start_pos;
+  p.R = R; p.H = H; p.G = G; p.page_size = page_size; p.window = window; p.chunk = chunk;
+  p.sinks = sinks; p.gate = gate; p.gate_ld = gate_ld; p.gate_elem = gate_elem; p.out_scale = out_scale;
+  return at_go(kv, n_pages, d, p, T, scale, true, stream);
 }
 
 // 0 if no kernel of this library has recorded a bounded-wait expiry on the current device.  Synchronises.

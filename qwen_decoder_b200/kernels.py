@@ -1444,6 +1444,17 @@ def sink_mma_supported(dtype: torch.dtype, H: int, G: int, d: int, vd: int) -> b
             and 0 < d <= 192 and 0 < vd <= 128)
 
 
+SINK_TC5 = _os.environ.get("QD_PREFILL_TC5", "1") != "0"
+
+
+def sink_tc5_supported(q: torch.Tensor, out: torch.Tensor, H: int, G: int, d: int, vd: int, page_size: int, gate: Optional[torch.Tensor],
+                       gate_elem: bool, cap: float) -> bool:
+    """What the tcgen05 form of the sink attention takes (``csrc/attention_tc5.cu``)."""
+    return (d == vd and d in (64, 128) and H // G <= 16 and page_size % 16 == 0 and not cap and out.stride(0) % 8 == 0
+            and q.data_ptr() % 16 == out.data_ptr() % 16 == 0
+            and not (gate is not None and gate_elem and (gate.data_ptr() % 16 or gate.stride(0) % 4)))
+
+
 def sink_attention_mma(q: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, block_table: torch.Tensor,
                        cu_tokens: torch.Tensor, start_pos: torch.Tensor, n_requests: int, n_tokens: int, H: int, G: int,
                        d: int, vd: int, page_size: int, scale: float, window: int, sinks: Optional[torch.Tensor],
@@ -1462,6 +1473,16 @@ def sink_attention_mma(q: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, blo
     assert cu_tokens.dtype == torch.int32 and start_pos.dtype == torch.int32
     assert sinks is None or (sinks.dtype == torch.float32 and sinks.numel() == H)
     _contig(q, "q"); _contig(kv, "kv"); _contig(block_table, "block_table")
+    # portions: the tcgen05 kernel was the faster one at every length (16 + 2 heads of 128, us: 2 tokens 17.5 and 12.6, 32 behind 900
+    # keys 68 and 24, 1,500 in blocks of 1,024 87 and 36)
+    if SINK_TC5 and splits == 1 and n_tokens > n_requests and kv.data_ptr() % 16 == 0 \
+            and sink_tc5_supported(q, out, H, G, d, vd, page_size, gate, gate_elem, cap):
+        _check(library("attention_tc5").qd_sink_attention_tc5(
+            _ptr(q), _ptr(out), _LL(out.stride(0)), _ptr(kv), _LL(kv.numel() // (2 * G * page_size * d)), _ptr(block_table),
+            _I(block_table.shape[1]), _ptr(cu_tokens), _ptr(start_pos), _I(n_requests), _I(n_tokens), _I(H), _I(G), _I(d), _I(page_size),
+            _F(scale), _I(window), _ptr(sinks), _I(chunk), _ptr(gate), _LL(gate.stride(0) if gate is not None else 0),
+            _I(1 if gate_elem else 0), _F(out_scale), _stream()), "sink_attention_tc5")
+        return
     ntok = SINK_MMA_ROWS // (H // G)
     tiles = n_tokens // ntok + n_requests            # at least sum over requests of ceil(tokens / ntok)
     part_o = part_ml = tickets = None
