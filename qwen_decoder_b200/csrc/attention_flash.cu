@@ -73,12 +73,14 @@ __device__ __forceinline__ float fast_exp2(float x) {
 // maxima m and denominators l of 16 rows each) are merged in shared memory; with one split the result is
 // written, otherwise it goes to scratch and the CTA that finishes last for its (token, kv head) adds up all
 // splits.  Every warp must be done with the stage buffers that start at smem_raw.
+// ``part0``: the place in scratch of the token's first partial result (they lie [head][split]).  ``same_lo`` .. ``same_hi`` - 1:
+// further rows that get the same result.
 template <int HD>
 __device__ __forceinline__ void dec_finish(float (&o)[HD / 8][4], float m0, float m1, float l0, float l1,
                                            unsigned char* smem_raw, int warp, int lane, int gs, int g, int t, int s,
                                            int H, int G, int splits, bf16* __restrict__ out,
                                            float* __restrict__ part_o, float* __restrict__ part_ml,
-                                           unsigned* __restrict__ tickets) {
+                                           unsigned* __restrict__ tickets, size_t part0, int same_lo, int same_hi) {
   l0 = quad_sum(l0);
   l1 = quad_sum(l1);
   __syncthreads();  // every warp is done with its stage buffers: reuse them for the merge
@@ -125,8 +127,9 @@ __device__ __forceinline__ void dec_finish(float (&o)[HD / 8][4], float m0, floa
       raw.x = pack_bf16(O.x * inv, O.y * inv);
       raw.y = pack_bf16(O.z * inv, O.w * inv);
       *reinterpret_cast<uint2*>(out + (size_t)t * H * HD + (size_t)h * HD + dim) = raw;
+      for (int r = same_lo; r < same_hi; r++) *reinterpret_cast<uint2*>(out + (size_t)r * H * HD + (size_t)h * HD + dim) = raw;
     } else {
-      const size_t pi = ((size_t)t * H + h) * splits + s;
+      const size_t pi = part0 + (size_t)h * splits + s;
       *reinterpret_cast<float4*>(part_o + pi * HD + dim) = O;
       if (dim == 0) { part_ml[pi * 2] = M; part_ml[pi * 2 + 1] = L; }
     }
@@ -152,7 +155,7 @@ __device__ __forceinline__ void dec_finish(float (&o)[HD / 8][4], float m0, floa
   constexpr int PB = 16;
   for (int idx = threadIdx.x; idx < gs * (HD / 4); idx += DEC_WARPS * 32) {
     const int row = idx / (HD / 4), d4 = idx - row * (HD / 4);
-    const size_t base = ((size_t)t * H + (size_t)g * gs + row) * splits;
+    const size_t base = part0 + ((size_t)g * gs + row) * splits;
     const float2* ml_g = reinterpret_cast<const float2*>(part_ml) + base;
     float2 mlv[PB];
     float4 pv[PB];
@@ -187,6 +190,8 @@ __device__ __forceinline__ void dec_finish(float (&o)[HD / 8][4], float m0, floa
     raw.x = pack_bf16(acc.x * invL, acc.y * invL);
     raw.y = pack_bf16(acc.z * invL, acc.w * invL);
     *reinterpret_cast<uint2*>(dst) = raw;
+    for (int r = same_lo; r < same_hi; r++)
+      *reinterpret_cast<uint2*>(out + (size_t)r * H * HD + ((size_t)g * gs + row) * HD + 4 * d4) = raw;
   }
   if (threadIdx.x == 0) tickets[(size_t)t * G + g] = 0;   // ready for the next launch
 }
@@ -343,7 +348,92 @@ decode_attention_kernel(const bf16* __restrict__ q, long long q_stride, bf16* __
   }
   cp_async_wait<0>();
   pdl_launch_dependents();
-  dec_finish<HD>(o, m0, m1, l0, l1, smem_raw, warp, lane, gs, g, t, s, H, G, splits, out, part_o, part_ml, tickets);
+  dec_finish<HD>(o, m0, m1, l0, l1, smem_raw, warp, lane, gs, g, t, s, H, G, splits, out, part_o, part_ml, tickets,
+                 (size_t)t * H * splits, 0, 0);
+}
+
+// ------------------------------------------------------------------ shares by length
+// A launch's CTAs all start together (two to a multiprocessor at head size 128, four at 64), and with the same number of shares for
+// every token the longest context's end last: 23 requests of 500 to 4,000 keys, padded to 32 (28 query and 4 kv heads of 128),
+// took 30.2 us where their bytes take 16.2.  So a list deals the CTAs out by length: shares of at most S chunks of 16 keys, S the
+// smallest for which there are no more shares than CTAs; 22.3 us.  It is made once a step, by a small launch before the first
+// attention that reads it.  Rows that pad a batch have no shares of their own (they repeat the first row, whose result is written to them
+// too): 40 requests padded to 64 19.9 -> 17.5 us.  Equal lengths take what they took: 64 of 2,048 keys 25.4 us.
+struct __align__(16) DecShare {
+  int ts, c, keys, n_same;      // token | share << 16; first chunk | end << 16; the token's keys; its shares | rows to copy to << 16
+  __device__ int t() const { return ts & 0xFFFF; }
+  __device__ int s() const { return ts >> 16; }
+  __device__ int c0() const { return c & 0xFFFF; }
+  __device__ int c1() const { return (int)((unsigned)c >> 16); }
+  __device__ int n() const { return n_same & 0xFFFF; }
+  __device__ int same() const { return n_same >> 16; }
+};
+#define DEC_SHARE_TOKENS 1024
+#define DEC_SHARE_MIN 10        // chunks: 2 and 8 tokens of 2,048 keys take 6.3 and 7.7 us in 12 shares, 10.8 and 10.9 in 4, 8.7 and 13.6 in 24
+#define DEC_SHARE_MOST 64       // of a token
+
+__global__ void __launch_bounds__(DEC_SHARE_TOKENS)
+decode_shares_kernel(const int* __restrict__ positions, const int* __restrict__ slot_map, int scratch_row, int T, int n_list,
+                     DecShare* __restrict__ list) {
+  __shared__ int chunks[DEC_SHARE_TOKENS], sums[32], pads[32];
+  const int i = threadIdx.x, warp = i >> 5, lane = i & 31;
+  int keys = 0, pad = 0;
+  if (i < T) {
+    keys = positions[i] + 1;
+    pad = i > 0 && slot_map[i] == scratch_row;
+  }
+  const int c = pad ? 0 : (keys + DEC_CHUNK - 1) / DEC_CHUNK;
+  chunks[i] = c;
+  const int most = __reduce_max_sync(0xffffffffu, c), n_pad = __reduce_add_sync(0xffffffffu, pad);
+  if (lane == 0) { sums[warp] = most; pads[warp] = n_pad; }
+  __syncthreads();
+  const int warps = blockDim.x >> 5;
+  const bool one = lane < warps;                    // a lane that looks at its warp's number
+  const int longest = __reduce_max_sync(0xffffffffu, one ? sums[lane] : 0), same = __reduce_add_sync(0xffffffffu, one ? pads[lane] : 0);
+  // the smallest S: as many candidates at a time as there are warps
+  int lo = max(DEC_SHARE_MIN, (longest + DEC_SHARE_MOST - 1) / DEC_SHARE_MOST), hi = max(lo, longest);
+  while (lo < hi) {
+    const int S = lo + (int)((long long)(hi - lo) * warp / warps);
+    int n = 0;
+    for (int j = lane; j < T; j += 32) n += (chunks[j] + S - 1) / S;
+    n = __reduce_add_sync(0xffffffffu, n);
+    __syncthreads();
+    if (lane == 0) sums[warp] = n;
+    __syncthreads();
+    const unsigned fits = __ballot_sync(0xffffffffu, one && sums[lane] <= n_list);
+    const int w = fits ? __ffs(fits) - 1 : warps, span = hi - lo, base = lo;
+    if (w < warps) hi = base + (int)((long long)span * w / warps);
+    if (w > 0) lo = base + (int)((long long)span * (w - 1) / warps) + 1;
+  }
+  const int n = (c + lo - 1) / lo;
+  // where a token's shares begin
+  int at = n;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, at, d);
+    if (lane >= d) at += v;
+  }
+  __syncthreads();
+  if (lane == 31) sums[warp] = at;
+  __syncthreads();
+  const int before = __reduce_add_sync(0xffffffffu, lane < warp ? sums[lane] : 0),
+            all = __reduce_add_sync(0xffffffffu, one ? sums[lane] : 0);
+  at += before - n;
+  pdl_wait();                   // all of the above runs beside the kernel before: positions and slots come with the step's copy
+  for (int s = 0; s < n && at + s < n_list; s++)
+    list[at + s] = DecShare{i | s << 16, (int)((long long)c * s / n) | (int)((long long)c * (s + 1) / n) << 16, keys, n | (i ? 0 : same) << 16};
+  for (int j = all + i; j < n_list; j += blockDim.x) list[j] = DecShare{0, 0, 0, 0};
+}
+
+// The list of shares of tokens 0 .. T-1 (up to 1,024) in ``n_list`` >= T entries of 16 bytes.  A row after the first whose slot
+// is ``scratch_row`` pads the batch.
+extern "C" int qd_decode_shares(const int* positions, const int* slot_map, int scratch_row, int T, int n_list, void* list,
+                                cudaStream_t stream) {
+  if (T <= 0) return 0;
+  if (T > DEC_SHARE_TOKENS || n_list < T || ((uintptr_t)list & 15)) return QD_ERR_UNSUPPORTED;
+  qd_launch(decode_shares_kernel, dim3(1), dim3(T <= 256 ? 256 : DEC_SHARE_TOKENS), 0, stream, positions, slot_map, scratch_row, T, n_list,
+            (DecShare*)list);
+  return qd_last_error();
 }
 
 // ------------------------------------------------------------------ the same with K/V through TMA
@@ -358,14 +448,17 @@ __device__ __forceinline__ bool fa_mbar_wait(unsigned long long* bar, unsigned p
   return qd_mbar_wait_bounded(fa_smem(bar), parity, dead, poll_limit, 1000000000ull);
 }
 
-template <int HD>
-__global__ void __launch_bounds__(DEC_WARPS * 32)
+// ``SHARES``: the CTA of kv head x and place y takes share y of the list ``shares`` (DecShare), whose rows have their tokens' block
+// tables; ``fresh``: the list is made by the launch before.
+template <int HD, bool SHARES>
+__global__ void __launch_bounds__(DEC_WARPS * 32, HD <= 64 ? 4 : 3)
 decode_attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const bf16* __restrict__ q, long long q_stride,
                             bf16* __restrict__ out, const int* __restrict__ block_table, int max_blocks,
                             const int* __restrict__ token_req, const int* __restrict__ positions, int H, int G,
                             int page_size, float scale_log2e, int window, int splits,
                             float* __restrict__ part_o, float* __restrict__ part_ml,
-                            unsigned* __restrict__ tickets, int* __restrict__ status) {
+                            unsigned* __restrict__ tickets, int* __restrict__ status,
+                            const DecShare* shares, int T, int fresh) {
   static_assert(HD % 64 == 0, "boxes of 64 columns");
   constexpr int NB = HD / 64;                      // boxes per K or V chunk
   constexpr int BOX = 16 * 64;                     // elements of a box (2 KB)
@@ -376,9 +469,17 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const bf
   __shared__ int page_ring[DEC_WARPS][64];
   // the swizzle pattern follows address bits 7-9: stages start on 1024-byte boundaries
   bf16* smem = reinterpret_cast<bf16*>(smem_raw + ((1024 - (fa_smem(smem_raw) & 1023)) & 1023));
-  const int s = blockIdx.x, g = blockIdx.y, t = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int gs = H / G;
+  const int gs = H / G, g = SHARES ? blockIdx.x : blockIdx.y;
+  int s = blockIdx.x, t = blockIdx.z;
+  DecShare mine = {0, 0, 0, 0};
+  if (SHARES) {
+    if (fresh) pdl_wait();
+    // on its way while the barriers are made; no plain load: a kernel that this one may overlap has written the list, and what is
+    // read through a const __restrict__ pointer may be read before the wait
+    asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(mine.ts), "=r"(mine.c), "=r"(mine.keys), "=r"(mine.n_same)
+                 : "l"(shares + blockIdx.y) : "memory");
+  }
   if (threadIdx.x == 0) {
     dead = 0;
     for (int w = 0; w < DEC_WARPS; w++)
@@ -387,14 +488,26 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const bf
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  const int pos = positions[t];
-  const int n_keys = pos + 1;
-  const int key_lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+  if (SHARES) {
+    splits = mine.n();
+    if (splits == 0) return;                         // fewer shares than CTAs
+    s = mine.s();
+    t = mine.t();
+    // a list of other tokens: nothing out of range is read for it
+    if (t >= T || (unsigned)s >= (unsigned)splits || splits > DEC_SHARE_MOST || s > (int)blockIdx.y ||
+        (int)blockIdx.y - s + splits > (int)gridDim.y || (unsigned)mine.same() >= (unsigned)T || mine.c0() > mine.c1() ||
+        mine.keys < 1 || mine.keys > max_blocks * page_size || mine.c1() > (mine.keys + DEC_CHUNK - 1) / DEC_CHUNK) {
+      if (threadIdx.x == 0) atomicExch(status, 2);
+      return;
+    }
+  }
+  const int n_keys = SHARES ? mine.keys : positions[t] + 1;
+  const int key_lo = !SHARES && window > 0 && n_keys > window ? n_keys - window : 0;
   const int chunk_lo = key_lo / DEC_CHUNK, chunk_hi = (n_keys + DEC_CHUNK - 1) / DEC_CHUNK;
   const int per = (chunk_hi - chunk_lo + splits - 1) / splits;
-  const int c0 = chunk_lo + s * per;
-  const int c1 = min(chunk_hi, c0 + per);
-  const int* bt = block_table + (size_t)token_req[t] * max_blocks;
+  const int c0 = SHARES ? mine.c0() : chunk_lo + s * per;
+  const int c1 = SHARES ? mine.c1() : min(chunk_hi, c0 + per);
+  const int* bt = block_table + (size_t)(SHARES ? t : token_req[t]) * max_blocks;
   bf16* wbuf = smem + (size_t)warp * DEC_STAGES * STAGE;
   const int first = c0 + warp;
   const int n_my = first < c1 ? (c1 - first + DEC_WARPS - 1) / DEC_WARPS : 0;
@@ -524,7 +637,8 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const bf
     __syncwarp();
   }
   pdl_launch_dependents();
-  dec_finish<HD>(o, m0, m1, l0, l1, smem_raw, warp, lane, gs, g, t, s, H, G, splits, out, part_o, part_ml, tickets);
+  dec_finish<HD>(o, m0, m1, l0, l1, smem_raw, warp, lane, gs, g, t, s, H, G, splits, out, part_o, part_ml, tickets,
+                 SHARES ? (size_t)(blockIdx.y - s) * H : (size_t)t * H * splits, SHARES ? T - mine.same() : 0, SHARES ? T : 0);
 }
 
 // out[t, h, :] = sum_s O_s * 2^(m_s - M) / sum_s l_s * 2^(m_s - M)
@@ -625,22 +739,35 @@ static int* fa_status_word() {
   return words[dev];
 }
 
-template <int HD>
+template <int HD, bool SHARES>
 static int launch_decode_tma(const CUtensorMap& map, const bf16* q, long long q_stride, bf16* out, const int* block_table,
                              int max_blocks, const int* token_req, const int* positions, int T, int H, int G,
                              int page_size, float scale, int window, int splits, float* part_o, float* part_ml,
-                             unsigned* tickets, int* status, cudaStream_t stream) {
+                             unsigned* tickets, int* status, const DecShare* shares, int fresh, cudaStream_t stream) {
   size_t smem = (size_t)DEC_WARPS * DEC_STAGES * 2 * DEC_CHUNK * HD * sizeof(bf16) + 1024;
-  if (cudaFuncSetAttribute(decode_attention_tma_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+  if (cudaFuncSetAttribute(decode_attention_tma_kernel<HD, SHARES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess) {
     cudaGetLastError();
     return QD_ERR_UNSUPPORTED;
   }
-  dim3 grid(splits, G, T);
-  qd_launch(decode_attention_tma_kernel<HD>, dim3(grid), dim3(DEC_WARPS * 32), smem, stream, map, q, q_stride, out,
+  const dim3 grid = SHARES ? dim3(G, splits) : dim3(splits, G, T);
+  qd_launch(decode_attention_tma_kernel<HD, SHARES>, dim3(grid), dim3(DEC_WARPS * 32), smem, stream, map, q, q_stride, out,
             block_table, max_blocks, token_req, positions, H, G, page_size, scale * 1.4426950408889634f, window, splits,
-            part_o, part_ml, tickets, status);
+            part_o, part_ml, tickets, status, shares, T, fresh);
   return qd_last_error();
+}
+
+// the cache as rows of d: [pages * 2 * G * page_size][d]; a box is 16 rows x 64 columns
+static bool decode_cache_map(CUtensorMap* map, const void* kv, long long n_pages, int G, int page_size, int d) {
+  FaEncodeFn fn = fa_encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[2] = {(cuuint64_t)d, (cuuint64_t)(n_pages * 2 * G * page_size)};
+  cuuint64_t strides[1] = {(cuuint64_t)d * 2};
+  cuuint32_t box[2] = {64, 16};
+  cuuint32_t estr[2] = {1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(kv), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // As qd_decode_attention with K/V fetched by TMA tensor copies: head size 64 or 128, tickets required when
@@ -656,27 +783,43 @@ extern "C" int qd_decode_attention_tma(const void* q, long long q_stride, void* 
     return QD_ERR_UNSUPPORTED;
   if (splits > 1 && (!part_o || !part_ml || !tickets)) return QD_ERR_UNSUPPORTED;
   if (((uintptr_t)kv & 15) || q_stride % 2 != 0) return QD_ERR_UNSUPPORTED;
-  FaEncodeFn fn = fa_encode_fn();
   int* status = fa_status_word();
-  if (!fn || !status) return QD_ERR_UNSUPPORTED;
-  // the cache as rows of d: [pages * 2 * G * page_size][d]; a box is 16 rows x 64 columns
   CUtensorMap map;
-  cuuint64_t dims[2] = {(cuuint64_t)d, (cuuint64_t)(n_pages * 2 * G * page_size)};
-  cuuint64_t strides[1] = {(cuuint64_t)d * 2};
-  cuuint32_t box[2] = {64, 16};
-  cuuint32_t estr[2] = {1, 1};
-  if (fn(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(kv), dims, strides, box, estr,
-         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return QD_ERR_UNSUPPORTED;
-  if (d == 64)
-    return launch_decode_tma<64>(map, (const bf16*)q, q_stride, (bf16*)out, block_table, max_blocks, token_req, positions,
-                                 T, H, G, page_size, scale, window, splits, part_o, part_ml, tickets, status, stream);
-  return launch_decode_tma<128>(map, (const bf16*)q, q_stride, (bf16*)out, block_table, max_blocks, token_req, positions,
-                                T, H, G, page_size, scale, window, splits, part_o, part_ml, tickets, status, stream);
+  if (!status || !decode_cache_map(&map, kv, n_pages, G, page_size, d)) return QD_ERR_UNSUPPORTED;
+#define GO(HD)                                                                                                                 \
+  return launch_decode_tma<HD, false>(map, (const bf16*)q, q_stride, (bf16*)out, block_table, max_blocks, token_req, positions, T, \
+                                      H, G, page_size, scale, window, splits, part_o, part_ml, tickets, status, nullptr, 0, stream)
+  if (d == 64) GO(64);
+  GO(128);
+#undef GO
 }
 
-// 0 if no bounded wait of the TMA decode kernel has run out on the current device (reported once).  Synchronises.
+// The same over all keys of each token with the list of shares that qd_decode_shares made for these T tokens: token t's keys lie in
+// the pages of row t of the block table.  Scratch: part_o n_list * H * d floats, part_ml n_list * H * 2, tickets T * G words (zero).
+// ``fresh``: the list is made by the launch before.
+extern "C" int qd_decode_attention_shares(const void* q, long long q_stride, void* out, const void* kv, long long n_pages,
+                                          const int* block_table, int max_blocks, int T, int H, int G, int d, int page_size,
+                                          float scale, const void* shares, int n_list, int fresh, float* part_o, float* part_ml,
+                                          unsigned* tickets, cudaStream_t stream) {
+  if (T <= 0) return 0;
+  if (G <= 0 || H % G != 0 || H / G > 16 || page_size % DEC_CHUNK != 0 || T > DEC_SHARE_TOKENS || n_list > 65535 ||
+      (d != 64 && d != 128) || n_pages < 1 || n_list < T || !shares || !part_o || !part_ml || !tickets)
+    return QD_ERR_UNSUPPORTED;
+  if (((uintptr_t)kv & 15) || q_stride % 2 != 0 || ((uintptr_t)shares & 15)) return QD_ERR_UNSUPPORTED;
+  int* status = fa_status_word();
+  CUtensorMap map;
+  if (!status || !decode_cache_map(&map, kv, n_pages, G, page_size, d)) return QD_ERR_UNSUPPORTED;
+#define GO(HD)                                                                                                               \
+  return launch_decode_tma<HD, true>(map, (const bf16*)q, q_stride, (bf16*)out, block_table, max_blocks, nullptr, nullptr, T, H, G, \
+                                     page_size, scale, 0, n_list, part_o, part_ml, tickets, status, (const DecShare*)shares, fresh, \
+                                     stream)
+  if (d == 64) GO(64);
+  GO(128);
+#undef GO
+}
+
+// 0 if no bounded wait of the TMA decode kernel has run out on the current device (reported once); 2: a list of shares was not its
+// tokens' own.  Synchronises.
 QD_DEFINE_WAIT_PROBE(qd_decode_attention_tma_wait_probe, fa_mbar_wait(bar, 0, dead, poll_limit), fa_status_word, 99)
 
 extern "C" int qd_decode_attention_tma_status() {

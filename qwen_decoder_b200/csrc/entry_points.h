@@ -24,6 +24,11 @@ int qd_decode_attention_tma(const void* q, long long q_stride, void* out, const 
                             const int* block_table, int max_blocks, const int* token_req, const int* positions, int T,
                             int H, int G, int d, int page_size, float scale, int window, int splits, float* part_o,
                             float* part_ml, unsigned* tickets, cudaStream_t stream);
+int qd_decode_shares(const int* positions, const int* slot_map, int scratch_row, int T, int n_list, void* list, cudaStream_t stream);
+int qd_decode_attention_shares(const void* q, long long q_stride, void* out, const void* kv, long long n_pages,
+                               const int* block_table, int max_blocks, int T, int H, int G, int d, int page_size, float scale,
+                               const void* shares, int n_list, int fresh, float* part_o, float* part_ml, unsigned* tickets,
+                               cudaStream_t stream);
 int qd_prefill_attention(const void* q, long long q_stride, void* out, const void* kv, const int* block_table,
                          int max_blocks, const int* cu_tokens, const int* start_pos, int R, int T, int H, int G,
                          int d, int page_size, float scale, int window, cudaStream_t stream);

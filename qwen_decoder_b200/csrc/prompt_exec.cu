@@ -53,6 +53,8 @@ struct PeFns {
   PeGemmBatched gemm_batched;
   decltype(&qd_elementwise_plain_next) plain_next;      // the elementwise library's next launch without the attribute
   decltype(&qd_gemm_pair) gemm_pair;                    // products on pairs of multiprocessors, where a plan below says so
+  decltype(&qd_decode_shares) decode_shares;            // the list of shares by length of a mixed step's single tokens
+  decltype(&qd_decode_attention_shares) attention_shares;       // the single tokens' attention with shares by length
 };
 
 // How a product is cut (``qd_gemm_pair_plan``); cg 0: the library's product
@@ -83,6 +85,9 @@ struct PeParams {
   PePlan wo_plan, wgu_plan, wd_plan;
   int sms;
   float* o_part;
+  // the single tokens' shares of decode attention (null: ``decode_splits`` for each); ``part_o`` and ``part_ml`` are theirs then
+  void* shares;
+  int n_shares, scratch_row;
 };
 
 extern "C" int qd_prompt_exec_struct_sizes(int* layer_bytes, int* params_bytes) {
@@ -132,6 +137,7 @@ extern "C" int qd_prompt_exec(const PeParams* pp, cudaStream_t stream) {
   if (shares < 0 || shares == 1 ||
       (shares > 1 && (!p.down_part || !p.fn.gemm_batched || !p.fn.plain_next || p.F % (8 * shares))))
     return QD_ERR_UNSUPPORTED;
+  if (p.shares && (!p.fn.attention_shares || !p.fn.decode_shares)) return QD_ERR_UNSUPPORTED;
   if ((p.wo_plan.cg || p.wgu_plan.cg || p.wd_plan.cg) && !p.fn.gemm_pair) return QD_ERR_UNSUPPORTED;
   if ((p.wo_plan.cg && p.wo_plan.splits > 1 && !p.o_part) || (p.wd_plan.cg && p.wd_plan.splits > 1 && !p.down_part)) return QD_ERR_UNSUPPORTED;
   const int T = p.T, D = p.D, H = p.H, G = p.G, d = p.d, F = p.F;
@@ -150,7 +156,11 @@ extern "C" int qd_prompt_exec(const PeParams* pp, cudaStream_t stream) {
     PE_TRY(p.fn.rope_kv_write(p.qkv, L.bqkv, T, H, G, d, p.rotary_dim, p.pairing, p.cos_t, p.sin_t, p.positions, L.kv,
                               p.slot_map, p.page_size, L.write_kv, stream));
     const int nd = p.n_decode;
-    if (nd > 0 && p.fn.attention_decode_tma && (p.decode_splits == 1 || p.tickets))
+    if (nd > 0 && p.shares && l == 0) PE_TRY(p.fn.decode_shares(p.positions, p.slot_map, p.scratch_row, nd, p.n_shares, p.shares, stream));
+    if (nd > 0 && p.shares)
+      PE_TRY(p.fn.attention_shares(p.qkv, n_qkv, p.attn, L.kv, p.n_pages, p.block_table, p.max_blocks, nd, H, G, d, p.page_size,
+                                   p.scale, p.shares, p.n_shares, l == 0, p.part_o, p.part_ml, p.tickets, stream));
+    else if (nd > 0 && p.fn.attention_decode_tma && (p.decode_splits == 1 || p.tickets))
       PE_TRY(p.fn.attention_decode_tma(p.qkv, n_qkv, p.attn, L.kv, p.n_pages, p.block_table, p.max_blocks, p.token_req,
                                        p.positions, nd, H, G, d, p.page_size, p.scale, p.window, p.decode_splits, p.part_o,
                                        p.part_ml, p.tickets, stream));

@@ -17,7 +17,7 @@ from ..cache import CacheManager, RequestCache
 from ..config import describe_model, load_config
 from ..parts.model import DecoderModel, build_model
 from ..weights import TensorSource, load_into, random_tensors
-from .batch import MetaLayout, StepEntry, StepError, build_context, fill, validate
+from .batch import MetaLayout, StepEntry, StepError, build_context, fill, uneven_contexts, validate
 
 DTYPES = {"bfloat16": torch.bfloat16, "bf16": torch.bfloat16, "float32": torch.float32, "f32": torch.float32,
           "fp32": torch.float32}
@@ -131,7 +131,7 @@ class ModelRunner:
         (``cache.log_tokens``).  Only for batches that run as a graph (``can_take_device_tokens``).
 
         A batch of single tokens that all want logits runs as a replayed CUDA graph (one per padded
-        batch size and block-table width) when ``use_graphs`` is set; the logits then live in a
+        batch size, block-table width and evenness of contexts) when ``use_graphs`` is set; the logits then live in a
         buffer that the next such step overwrites."""
         if ensure_pages:
             self._ensure(entries)
@@ -191,10 +191,11 @@ class ModelRunner:
             Bp *= 2
         mbs = tuple((max(len(e.cache.tables[g]) for e in entries) + 31) // 32 * 32
                     for g in range(len(self.cache.pools)))
-        key = (Bp, mbs, sampling is not None)
+        uneven = Bp > 16 and uneven_contexts(starts, Bp)      # up to 16 tokens attention has a kernel that does not ask
+        key = (Bp, mbs, sampling is not None, uneven)
         g = self._graphs.get(key)
         if g is None:
-            g = self._graphs[key] = _DecodeGraph(self, Bp, mbs, sampling is not None)
+            g = self._graphs[key] = _DecodeGraph(self, Bp, mbs, sampling is not None, uneven)
         host = g.next_host()
         h = host.numpy()
         fill(h, g.lay, entries, self.cache, lens, starts, slots, self.model.vocab_size)
@@ -230,7 +231,7 @@ class _NotOnHost:
 class _DecodeGraph:
     """One captured decode step for a padded batch size and block-table widths."""
 
-    def __init__(self, runner: "ModelRunner", Bp: int, mbs, with_sampling: bool):
+    def __init__(self, runner: "ModelRunner", Bp: int, mbs, with_sampling: bool, uneven: bool):
         # no reference back to the runner: a cycle would leave the captured graph to the garbage
         # collector, which might then destroy it in the middle of another capture
         self.model = runner.model
@@ -244,6 +245,7 @@ class _DecodeGraph:
         self.dev = torch.zeros(self.lay.total, dtype=torch.int32, device=runner.device)
         self.ctx = self.lay.context(self.dev, runner.cache, runner.device)
         self.ctx.all_decode = True
+        self.ctx.uneven = uneven
         self.ctx.max_portion = 1
         # nothing of a replayed step runs on the host: there are no host copies of its metadata
         self.ctx.host_cu_tokens = self.ctx.host_start_pos = self.ctx.host_state_slots = _NotOnHost()

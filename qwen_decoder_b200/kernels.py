@@ -714,6 +714,62 @@ def decode_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, kv: torc
         _I(window), _I(splits), _ptr(part_o), _ptr(part_ml), _ptr(tickets), _stream()), "decode_attention")
 
 
+DECODE_SHARE_TOKENS, DECODE_SHARE_KEYS = 1024, 65535 * 16
+
+
+def decode_ctas(d: int) -> int:
+    """CTAs of split-KV decode attention that run at a time: two to a multiprocessor, four at head sizes up to 64."""
+    return (4 if d <= 64 else 2) * sm_count()
+
+
+def decode_shares_supported(dtype, n_tokens: int, H: int, G: int, d: int, page_size: int, max_keys: int) -> bool:
+    """Whether decode attention over all keys may deal its CTAs out by the tokens' lengths.  Two tokens or more: one has all
+    CTAs anyway."""
+    return (flash_decode_supported(dtype, H, G, d, page_size) and decode_by_tma(d) and 2 <= n_tokens <= DECODE_SHARE_TOKENS
+            and n_tokens * G <= _TICKETS and max_keys <= DECODE_SHARE_KEYS)
+
+
+def decode_shares_list(n_tokens: int, G: int, d: int, device) -> torch.Tensor:
+    return torch.empty((max(n_tokens, decode_ctas(d) // G), 4), dtype=torch.int32, device=device)
+
+
+def decode_shares(positions: torch.Tensor, slot_map: torch.Tensor, scratch_row: int, n_tokens: int, G: int, d: int) -> torch.Tensor:
+    """The shares of decode attention, int32 [CTAs of a kv head, 4], for the first ``n_tokens`` tokens; a row after the first whose
+    slot is ``scratch_row`` pads the batch (it repeats the first)."""
+    assert positions.dtype == torch.int32 and slot_map.dtype == torch.int32
+    assert min(positions.numel(), slot_map.numel()) >= n_tokens
+    shares = decode_shares_list(n_tokens, G, d, positions.device)
+    _check(library("attention_flash").qd_decode_shares(
+        _ptr(positions), _ptr(slot_map), _I(scratch_row), _I(n_tokens), _I(shares.shape[0]), _ptr(shares), _stream()), "decode_shares")
+    return shares
+
+
+def decode_shares_scratch(n_list: int, H: int, d: int, device):
+    """(part_o, part_ml, tickets) for a launch over a list of ``n_list`` shares."""
+    tickets = _tickets.get(device)
+    if tickets is None:     # zero once; every launch leaves them zero again
+        tickets = _tickets[device] = torch.zeros(_TICKETS, dtype=torch.int32, device=device)
+    return (torch.empty((n_list * H, d), dtype=torch.float32, device=device),
+            torch.empty((n_list * H, 2), dtype=torch.float32, device=device), tickets)
+
+
+def decode_attention_shares(q: torch.Tensor, q_stride: int, out: torch.Tensor, kv: torch.Tensor, block_table: torch.Tensor,
+                            n_tokens: int, H: int, G: int, d: int, page_size: int, scale: float, shares: torch.Tensor,
+                            fresh: bool) -> None:
+    """As ``decode_attention`` over all keys, the CTAs dealt out by ``shares`` (``decode_shares`` of the same tokens; ``fresh``: they
+    are made by the launch before).  Token t's pages are row t of the block table."""
+    assert q.dtype == torch.bfloat16 and kv.dtype == torch.bfloat16 and out.dtype == torch.bfloat16
+    assert out.shape == (n_tokens, H * d) and tuple(kv.shape[1:]) == (2, G, page_size, d)
+    assert block_table.dtype == torch.int32 and block_table.dim() == 2 and block_table.shape[0] >= n_tokens
+    assert n_tokens * G <= _TICKETS
+    _contig(out, "out"); _contig(kv, "kv"); _contig(block_table, "block_table"); _contig(shares, "shares")
+    part_o, part_ml, tickets = decode_shares_scratch(shares.shape[0], H, d, q.device)
+    _check(library("attention_flash").qd_decode_attention_shares(
+        _ptr(q), _LL(q_stride), _ptr(out), _ptr(kv), _LL(kv.shape[0]), _ptr(block_table), _I(block_table.shape[1]), _I(n_tokens),
+        _I(H), _I(G), _I(d), _I(page_size), _F(scale), _ptr(shares), _I(shares.shape[0]), _I(int(fresh)), _ptr(part_o), _ptr(part_ml),
+        _ptr(tickets), _stream()), "decode_attention_shares")
+
+
 def decode_rope_supported(dtype: torch.dtype, H: int, G: int, d: int, page_size: int) -> bool:
     return (dtype == torch.bfloat16 and d in (16, 32, 48, 64, 96, 128) and H % G == 0 and H // G <= 16
             and page_size % 16 == 0)
@@ -1812,7 +1868,8 @@ class PromptFns(ctypes.Structure):
     """Addresses of the launchers and of the library product that the native prompt step calls."""
     _fields_ = [(n, ctypes.c_void_p) for n in ("add_rmsnorm", "rope_kv_write", "swiglu", "attention_regs",
                                                "attention_tc5", "attention_decode", "attention_decode_tma", "gemm_ex",
-                                               "blas", "gemm_batched", "plain_next", "gemm_pair")]
+                                               "blas", "gemm_batched", "plain_next", "gemm_pair",
+                                               "decode_shares", "attention_shares")]
 
 
 class PromptPlan(ctypes.Structure):
@@ -1832,7 +1889,8 @@ class PromptParams(ctypes.Structure):
         [("n_decode", ctypes.c_int), ("decode_splits", ctypes.c_int)] + \
         [(n, ctypes.c_void_p) for n in ("token_req", "part_o", "part_ml", "tickets", "down_part")] + \
         [("down_shares", ctypes.c_int), ("pad2", ctypes.c_int)] + \
-        [(n, PromptPlan) for n in ("wo_plan", "wgu_plan", "wd_plan")] + [("sms", ctypes.c_int), ("o_part", ctypes.c_void_p)]
+        [(n, PromptPlan) for n in ("wo_plan", "wgu_plan", "wd_plan")] + [("sms", ctypes.c_int), ("o_part", ctypes.c_void_p)] + \
+        [("shares", ctypes.c_void_p), ("n_shares", ctypes.c_int), ("scratch_row", ctypes.c_int)]
 
 
 def prompt_exec_struct_sizes_match() -> bool:
@@ -1875,6 +1933,8 @@ def prompt_fns(use_tc5: bool, with_decode: bool = False, decode_tma: bool = Fals
             fns.attention_decode = addr(library("attention_flash").qd_decode_attention)
             if decode_tma:
                 fns.attention_decode_tma = addr(library("attention_flash").qd_decode_attention_tma)
+                fns.decode_shares = addr(library("attention_flash").qd_decode_shares)
+                fns.attention_shares = addr(library("attention_flash").qd_decode_attention_shares)
         fns.gemm_ex = addr(_loaded_cublas().cublasGemmEx)
         fns.gemm_batched = addr(_loaded_cublas().cublasGemmStridedBatchedEx)
         fns.plain_next = addr(ew.qd_elementwise_plain_next)

@@ -93,13 +93,18 @@ class GQAttention(Mixer):
             qkv = self.qkv.forward(x)
             kernels.rope_kv_write(qkv, H, G, d, *rope, ctx.positions, cache.kv, cache.group.slot_map,
                                   cache.group.page_size, cache.write)
+        shares = step_decode_shares(ctx, cache, H, G, d, self.window, x.dtype)
         attn = torch.empty((x.shape[0], H * d), dtype=x.dtype, device=x.device)
         ps, window = cache.group.page_size, self.window or 0
         if ctx.all_decode and kernels.flash_decode_supported(x.dtype, H, G, d, ps):
-            kernels.decode_attention(
-                qkv, qkv.stride(0), attn, cache.kv, cache.group.block_table, ctx.token_request,
-                ctx.positions, ctx.num_tokens, H, G, d, ps, self.scale, window,
-                decode_splits(ctx.num_tokens * G, min(ctx.max_context, window or ctx.max_context)))
+            if shares is not None:
+                kernels.decode_attention_shares(qkv, qkv.stride(0), attn, cache.kv, cache.group.block_table, ctx.num_tokens, H, G, d,
+                                                ps, self.scale, *shares)
+            else:
+                kernels.decode_attention(
+                    qkv, qkv.stride(0), attn, cache.kv, cache.group.block_table, ctx.token_request,
+                    ctx.positions, ctx.num_tokens, H, G, d, ps, self.scale, window,
+                    decode_splits(ctx.num_tokens * G, min(ctx.max_context, window or ctx.max_context), kernels.decode_ctas(d)))
         elif kernels.flash_prefill_supported(x.dtype, H, G, d, ps) or \
                 (_PREFILL_TC5 and kernels.prefill_tc5_supported(x.dtype, H, G, d, ps)):
             # a mixed step: its single tokens (first in the batch) go to the decode kernel, which shares
@@ -107,11 +112,14 @@ class GQAttention(Mixer):
             nd = getattr(ctx, "num_decode", 0)
             if nd and not kernels.flash_decode_supported(x.dtype, H, G, d, ps):
                 nd = 0
-            if nd:
+            if nd and shares is not None:
+                kernels.decode_attention_shares(qkv, qkv.stride(0), attn[:nd], cache.kv, cache.group.block_table, nd, H, G, d, ps,
+                                                self.scale, *shares)
+            elif nd:
                 kernels.decode_attention(
                     qkv, qkv.stride(0), attn[:nd], cache.kv, cache.group.block_table, ctx.token_request[:nd],
                     ctx.positions[:nd], nd, H, G, d, ps, self.scale, window,
-                    decode_splits(nd * G, min(ctx.decode_max_context, window or ctx.decode_max_context)))
+                    decode_splits(nd * G, min(ctx.decode_max_context, window or ctx.decode_max_context), kernels.decode_ctas(d)))
             fn = kernels.prefill_attention_tc5 \
                 if _PREFILL_TC5 and kernels.prefill_tc5_supported(x.dtype, H, G, d, ps) else kernels.prefill_attention
             fn(qkv, qkv.stride(0), attn, cache.kv, cache.group.block_table[nd:], ctx.cu_tokens[nd:],
@@ -142,12 +150,28 @@ def decode_rope_splits(ctas_without_split: int, max_keys: int) -> int:
     return max(1, min(by_fill, by_work, 64))
 
 
+def step_decode_shares(ctx, cache: PagedCacheView, H: int, G: int, d: int, window: Optional[int], dtype: torch.dtype):
+    """(the list of shares of this step's single tokens, whether it was made just now) for decode attention over all keys, or None
+    where that does not apply.  The step's first layer that asks makes the list, in the launch before its attention; later layers of
+    the same kind read it."""
+    n, keys = (ctx.num_tokens, ctx.max_context) if ctx.all_decode else (ctx.num_decode, ctx.decode_max_context)
+    if not ctx.uneven or (window and window < keys) or not kernels.decode_shares_supported(dtype, n, H, G, d, cache.group.page_size, keys):
+        return None
+    key = ("decode_shares", G, d)
+    made = key not in ctx.shared
+    if made:
+        ctx.shared[key] = kernels.decode_shares(ctx.positions, cache.group.slot_map, ctx.cache.scratch_page * cache.group.page_size,
+                                                n, G, d)
+    return ctx.shared[key], made
+
+
 def decode_splits(ctas_without_split: int, max_keys: int, target_ctas: Optional[int] = None) -> int:
-    """How many CTAs share one (request, kv head) in decode attention: enough for one CTA on each of
-    the multiprocessors (more splits cost more in the combine than they gain: measured in whole decode steps at
-    batch 1, 8 and 64), but no CTA with fewer than four 16-key chunks."""
+    """How many CTAs share one (request, kv head) in decode attention: as many as run at a time (``target_ctas``: two to a
+    multiprocessor unless given), never a second wave of them, and no CTA with fewer than ten 16-key chunks.  Keys of 2,048 at 16
+    query and 2 kv heads of 128, us: 32 requests 14.3 in 4 shares, 14.9 in 3, 21.9 in 5; 17 requests 10.2 in 8, 11.3 in 5; 8 and 2
+    requests 7.7 and 6.3 in 12, 8.6 and 7.8 in 8, 9.3 and 8.1 in 18."""
     if target_ctas is None:
-        target_ctas = kernels.sm_count()
-    by_fill = max(1, -(-target_ctas // max(1, ctas_without_split)))
-    by_work = max(1, (max_keys + 63) // 64)
+        target_ctas = 2 * kernels.sm_count()
+    by_fill = target_ctas // max(1, ctas_without_split)
+    by_work = (max_keys + 159) // 160
     return max(1, min(by_fill, by_work, 64))

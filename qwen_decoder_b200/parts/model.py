@@ -165,6 +165,7 @@ class DecoderModel:
     # ---- forward -------------------------------------------------------------
     def forward(self, ctx) -> torch.Tensor:
         """Run the step's tokens through the model; float32 logits [n_wanted, vocab]."""
+        ctx.shared.clear()
         x = torch.empty((ctx.num_tokens, self.hidden_size), dtype=torch.float32, device=self.device)
         kernels.embedding(x, self.embedding, ctx.tokens, self.embedding_scale)
         if self.native_prompt is not None and self.native_prompt.takes(ctx):

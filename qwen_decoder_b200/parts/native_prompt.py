@@ -158,10 +158,16 @@ class NativePrompt:
             from .attention import decode_splits
             window = c["window"] or 0
             p.n_decode = nd
-            p.decode_splits = decode_splits(nd * G, min(ctx.decode_max_context, window or ctx.decode_max_context))
-            keep = kernels.decode_scratch(nd, H, d, G, p.decode_splits, dev)
+            p.decode_splits = decode_splits(nd * G, min(ctx.decode_max_context, window or ctx.decode_max_context), kernels.decode_ctas(d))
+            if ctx.uneven and not (window and window < ctx.decode_max_context) and \
+                    kernels.decode_shares_supported(bf, nd, H, G, d, group.page_size, ctx.decode_max_context):
+                shares = kernels.decode_shares_list(nd, G, d, dev)
+                p.shares, p.n_shares, p.scratch_row = shares.data_ptr(), shares.shape[0], ctx.cache.scratch_page * group.page_size
+                keep = kernels.decode_shares_scratch(p.n_shares, H, d, dev) + (shares,)
+            else:
+                keep = kernels.decode_scratch(nd, H, d, G, p.decode_splits, dev)
             p.token_req = ctx.token_request.data_ptr()
-            p.part_o, p.part_ml, p.tickets = (t.data_ptr() if t is not None else None for t in keep)
+            p.part_o, p.part_ml, p.tickets = (t.data_ptr() if t is not None else None for t in keep[:3])
         p.fn.blas = torch.cuda.current_blas_handle()
         p.layers = ctypes.cast(self._layer_array(ctx.cache), ctypes.c_void_p)
         p.n_layers = len(self.entries)
