@@ -1,19 +1,21 @@
 // Linear attention over portions in chunks of LC tokens, on the tensor cores (the general kernels of linear_scan.cu go token by
-// token, or four at a time: a serial chain of 0.1 to 0.2 us a token that leaves most of the GPU waiting).  For heads of 64 x 64 or
-// 128 x 128 (keys x values).  With S0 the state before a chunk, g_i the decays, G_p = g_0 .. g_p, d(s, p) = g_(s+1) .. g_p:
+// token: a serial chain of 0.1 us a token that leaves most of the GPU waiting).  For heads of 64 x 64 or 128 x 128 (keys x values)
+// without the delta rule.  With S0 the state before a chunk, g_i the decays, G_p = g_0 .. g_p, d(s, p) = g_(s+1) .. g_p:
 //
-//   plain       o_p = G_p S0^T q_p + sum_(s <= p) d(s, p) (k_s . q_p) x_s,   S <- G S0 + sum_s d(s, last) k_s x_s^T,   x = v
-//   delta rule  the same with x the solution of (1 + A) X = beta (V - G K S0), A[p, s] = beta_p d(s, p) (k_s . k_p) for s < p:
-//               with T = (1 + A)^-1,  X = U - W S0,  U = T (beta V),  W = T (beta G K)
+//   o_p = G_p S0^T q_p + sum_(s <= p) d(s, p) (k_s . q_p) v_s,   S <- G S0 + sum_s d(s, last) k_s v_s^T
 //
-// Three launches: what a chunk contributes by itself (plain: sum_s d(s, last) k_s v_s^T; delta rule: U and W), all chunks at once;
-// the states before the chunks, one after the other (plain: a sum; delta rule: X = U - W S0 and the state's product, with the state
-// in registers); the outputs with norm and gate, all chunks at once.
+// Three launches: what a chunk adds to the state, sum_s d(s, last) k_s v_s^T, all chunks at once; the states before the chunks, one
+// after the other; the outputs with norm and gate, all chunks at once.
+//
+// The delta rule has no such form here.  There the values' place is taken by the solution of a triangular system a chunk, and rounded
+// to float32 it was further from float64 than the kernels that go four tokens at a time: 512 tokens, keys and queries whose common part
+// is 0.9, decays from 0.9 on: outputs 2.8e-7 against 1.3e-7, states 2.2e-7 against 1.3e-7; decays from 0.99 on: outputs 4.6e-7 against
+// 1.6e-7 (266 us against 316 a call of 1,500 tokens, 32 heads of 128).  In a restatement with every sum rounded once the system's matrix,
+// its right sides, its solution and the products of keys and queries all had to carry more than float32 to come below.
 //
 // Numbers stay float32: every operand is cut into three bfloat16 pieces that sum to it exactly, and of the nine products of pieces
-// the six above 2^-24 are taken, the large one and the five small ones in sums of their own.  (T is made by float32 FMA.)  A chunk
-// that holds an infinity, NaN or a number beyond bfloat16's range takes its triangular products by FMA over s <= p only, so that
-// tokens before it stay as they are.
+// the six above 2^-24 are taken, the large one and the five small ones in sums of their own.  A chunk that holds an infinity, NaN or
+// a number beyond bfloat16's range takes its triangular products by FMA over s <= p only, so that tokens before it stay as they are.
 #pragma once
 #include "common.cuh"
 #include "mma_sync.cuh"
@@ -25,15 +27,12 @@
 struct LinearChunk {
   const float *q, *k;                     // [T, G, D]
   const float* v; long long ldv;
-  const float* g; int g_ld; const float* beta;
+  const float* g; int g_ld;
   int T, R, H, G;
   float* state; long long state_stride, s_off;
   const int *cu_tokens, *slots; int write_state;
   float* dec;                             // [chunk, H, LC_DEC]
-  float* x;                               // delta rule: [chunk, H, LC, DV]: U, then X
-  bf16* w;                                // delta rule: pieces of W [chunk, H, 3, LC, D]
-  bf16* kp;                               // delta rule: pieces of K [chunk, G, 3, LC, D]
-  float* s0;                              // [chunk, H, DV, D]: what the chunk adds to the state (plain), then the state before it
+  float* s0;                              // [chunk, H, DV, D]: what the chunk adds to the state, then the state before it
   // norm, gate and result, as LinearFinish in linear_scan.cu
   const float* gate; long long gate_ld; const float* norm; int norm_ld; float eps, out_scale; int gate_kind;
   void* out; int out_dtype; long long out_stride;
@@ -189,7 +188,7 @@ __device__ __forceinline__ void lc_decays(const LinearChunk& a, int t0, int n, i
 }
 
 // ------------------------------------------------------------------------------------- what a chunk contributes
-// Plain: s0[chunk, h, j, i] = sum_s d(s, last) v_s[j] k_s[i].  grid (chunks, H)
+// s0[chunk, h, j, i] = sum_s d(s, last) v_s[j] k_s[i].  grid (chunks, H)
 template <int D, int DV>
 __global__ void __launch_bounds__(LC_THREADS)
 linear_chunk_add_kernel(LinearChunk a) {
@@ -255,195 +254,8 @@ linear_chunk_add_kernel(LinearChunk a) {
   }
 }
 
-// Delta rule: U, the pieces of W, of K and the decays.  grid (chunks, H)
-template <int D, int DV>
-__global__ void __launch_bounds__(LC_THREADS, 2)
-linear_chunk_solve_kernel(LinearChunk a) {
-  pdl_launch_dependents();
-  pdl_wait();
-  static_assert(D == DV, "the values take the keys' place in shared memory");
-  extern __shared__ __align__(16) unsigned char lc_sm[];
-  using TK = LcTile<LC, D>;
-  bf16* ks = reinterpret_cast<bf16*>(lc_sm);
-  float* dm = reinterpret_cast<float*>(ks + TK::ELEMS);                 // [LC][LC_DM]: decays, then M of the inverse's steps
-  float* am = dm + LC * LC_DM;                                          // A, lower triangle
-  float* tm = am + LC * LC_DM;                                          // T
-  __shared__ float gs[LC], bs[LC], bg[LC];
-  int r, t0, n;
-  if (!lc_find(a, blockIdx.x, r, t0, n)) return;
-  const int h = blockIdx.y, per = a.H / a.G, gk = h / per, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const float* kg = a.k + ((size_t)t0 * a.G + gk) * D;
-  const float* vg = a.v + (size_t)t0 * a.ldv + (size_t)h * DV;
-  if (tid < LC) bs[tid] = tid < n ? a.beta[(size_t)(t0 + tid) * a.H + h] : 0.f;
-  bool odd = lc_fill<LC, D>(ks, kg, (long long)a.G * D, n);
-  lc_decays(a, t0, n, h, gs, dm);
-  if (tid < LC) {
-    bg[tid] = bs[tid] * (dm[tid * LC_DM] * gs[0]);
-    odd = odd || lc_odd(bs[tid]) || lc_odd(bg[tid]);
-    float* dec = a.dec + ((size_t)blockIdx.x * a.H + h) * LC_DEC;
-    dec[tid] = dm[(LC - 1) * LC_DM + tid];
-    if (tid == 0) dec[LC] = dm[(LC - 1) * LC_DM] * gs[0];
-  }
-  // (a scheduler's two warps have rows whose triangular products are five blocks together)
-  const int part = warp >> 2, m = (part ? 3 - (warp & 3) : warp & 3) * 16, g = lane >> 2, t2 = (lane & 3) * 2;
-  // A: a warp has 16 rows by every other pair of column tiles up to the diagonal
-  for (int np = part; np * 16 <= m; np += 2) {
-    float c[2][4], s[2][4];
-    lc_zero(c);
-    lc_zero(s);
-#pragma unroll 2
-    for (int kk = 0; kk < D / 16; kk++) {
-      unsigned fa[3][4], fb[3][4];
-#pragma unroll
-      for (int i = 0; i < 3; i++) {
-        lc_a(fa[i], ks + i * TK::PIECE, TK::LD, m, kk * 16, lane);
-        lc_b(fb[i], ks + i * TK::PIECE, TK::LD, kk * 16, np * 16, lane);
-      }
-      lc_mma(c, s, fa, fb);
-    }
-#pragma unroll
-    for (int t = 0; t < 2; t++)
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const int p = m + g + 8 * (e >> 1), q = np * 16 + t * 8 + t2 + (e & 1);
-        am[p * LC_DM + q] = q < p ? bs[p] * (dm[p * LC_DM + q] * (c[t][e] + s[t][e])) : 0.f;
-      }
-  }
-  for (int e = tid; e < LC * LC_DM; e += LC_THREADS) tm[e] = 0.f;
-  // the pieces of K, once for the value heads that share it
-  if (h == gk * per) {
-    bf16* to = a.kp + ((size_t)blockIdx.x * a.G + gk) * 3 * LC * D;
-    for (int e = tid; e < 3 * LC * (D / 8); e += LC_THREADS) {
-      const int row = e / (D / 8), c = (e - row * (D / 8)) * 8;
-      *reinterpret_cast<uint4*>(to + row * D + c) = *reinterpret_cast<const uint4*>(ks + row * TK::LD + c);
-    }
-  }
-  __syncthreads();
-  // T: blocks of 16 on the diagonal a column a thread, then blocks of 16 and of 32 below them: T21 = -T22 (A21 T11)
-  if (tid < LC) {
-    const int b = tid & ~15, col = tid & 15;
-    float t[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) t[i] = i == col ? 1.f : 0.f;
-#pragma unroll
-    for (int k = 0; k < 16; k++) {
-      if (k < col) t[k] = 0.f;                        // (above the diagonal, whatever A holds there)
-#pragma unroll
-      for (int i = k + 1; i < 16; i++) t[i] = fmaf(-am[(b + i) * LC_DM + b + k], t[k], t[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < 16; i++) tm[(b + i) * LC_DM + b + col] = t[i];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int half = 16; half < LC; half *= 2) {         // four neighbouring numbers a thread
-    const int blocks = LC / (2 * half), per_block = half * half / 4;
-    const int b = tid / per_block * 2 * half, i = tid % per_block / (half / 4), j = tid % (half / 4) * 4;
-    const bool mine = tid < blocks * per_block;
-    if (mine) {
-      float y[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-      for (int k = 0; k < half; k++) {
-        const float w = am[(b + half + i) * LC_DM + b + k];
-        const float2 lo = *reinterpret_cast<const float2*>(tm + (b + k) * LC_DM + b + j), hi = *reinterpret_cast<const float2*>(tm + (b + k) * LC_DM + b + j + 2);
-        y[0] = fmaf(w, lo.x, y[0]);
-        y[1] = fmaf(w, lo.y, y[1]);
-        y[2] = fmaf(w, hi.x, y[2]);
-        y[3] = fmaf(w, hi.y, y[3]);
-      }
-#pragma unroll
-      for (int c = 0; c < 4; c++) dm[(b + i) * LC_DM + j + c] = y[c];
-    }
-    __syncthreads();
-    if (mine) {
-      float y[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-      for (int k = 0; k < half; k++) {
-        if (k > i) break;                             // (rows behind this one may not be numbers)
-        const float w = -tm[(b + half + i) * LC_DM + b + half + k];
-        const float2 lo = *reinterpret_cast<const float2*>(dm + (b + k) * LC_DM + j), hi = *reinterpret_cast<const float2*>(dm + (b + k) * LC_DM + j + 2);
-        y[0] = fmaf(w, lo.x, y[0]);
-        y[1] = fmaf(w, lo.y, y[1]);
-        y[2] = fmaf(w, hi.x, y[2]);
-        y[3] = fmaf(w, hi.y, y[3]);
-      }
-#pragma unroll
-      for (int c = 0; c < 4; c++) tm[(b + half + i) * LC_DM + b + j + c] = y[c];
-    }
-    __syncthreads();
-  }
-  // T (f_s rows): 16 rows by half of the columns of a warp; ``put`` takes a pair of neighbouring results
-  odd = __syncthreads_or(odd);
-  constexpr int NP = D / 32;
-  auto scalar = [&](const float* f, const float* src, long long ld, auto&& put) {      // only what lies at or before a token joins its sum
-    for (int e = tid; e < LC * (D / 2); e += LC_THREADS) {
-      const int p = e / (D / 2), c = (e - p * (D / 2)) * 2;
-      float x = 0.f, y = 0.f;
-      for (int s = 0; s <= p && s < n; s++) {
-        const float w = tm[p * LC_DM + s] * f[s];
-        x = fmaf(w, src[s * ld + c], x);
-        y = fmaf(w, src[s * ld + c + 1], y);
-      }
-      put(p, c, x, y);
-    }
-  };
-  auto product = [&](const float* f, auto&& before, auto&& put) {
-    float c[NP][2][4], s[NP][2][4];
-#pragma unroll
-    for (int i = 0; i < NP; i++) { lc_zero(c[i]); lc_zero(s[i]); }
-#pragma unroll 1
-    for (int kk = 0; kk * 16 <= m; kk++) {
-      unsigned fa[3][4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const int p = m + g + 8 * (i & 1), q = kk * 16 + t2 + 8 * (i >> 1);
-        const float2 x = *reinterpret_cast<const float2*>(tm + p * LC_DM + q);
-        unsigned cut[3];
-        lc_cut(x.x * f[q], x.y * f[q + 1], cut);
-        fa[0][i] = cut[0]; fa[1][i] = cut[1]; fa[2][i] = cut[2];
-      }
-#pragma unroll
-      for (int np = 0; np < NP; np++) {
-        unsigned fb[3][4];
-#pragma unroll
-        for (int i = 0; i < 3; i++) lc_b_t(fb[i], ks + i * TK::PIECE, TK::LD, kk * 16, part * (D / 2) + np * 16, lane);
-        lc_mma(c[np], s[np], fa, fb);
-      }
-    }
-    before();
-#pragma unroll
-    for (int np = 0; np < NP; np++)
-#pragma unroll
-      for (int t = 0; t < 2; t++)
-#pragma unroll
-        for (int e = 0; e < 4; e += 2)
-          put(m + g + 4 * e, part * (D / 2) + np * 16 + t * 8 + t2, c[np][t][e] + s[np][t][e], c[np][t][e + 1] + s[np][t][e + 1]);
-  };
-  // W's pieces take K's place and go out in whole rows
-  auto w_put = [&](int p, int c, float x, float y) {
-    unsigned cut[3];
-    lc_cut(x, y, cut);
-#pragma unroll
-    for (int i = 0; i < 3; i++) *reinterpret_cast<unsigned*>(ks + (i * LC + p) * TK::LD + c) = cut[i];
-  };
-  if (odd) scalar(bg, kg, (long long)a.G * D, w_put);
-  else product(bg, [] { __syncthreads(); }, w_put);
-  __syncthreads();
-  bf16* wp = a.w + ((size_t)blockIdx.x * a.H + h) * 3 * LC * D;
-  for (int e = tid; e < 3 * LC * (D / 8); e += LC_THREADS) {
-    const int row = e / (D / 8), c = (e - row * (D / 8)) * 8;
-    *reinterpret_cast<uint4*>(wp + row * D + c) = *reinterpret_cast<const uint4*>(ks + row * TK::LD + c);
-  }
-  __syncthreads();
-  odd = __syncthreads_or(lc_fill<LC, DV>(ks, vg, a.ldv, n)) || odd;
-  float* u = a.x + ((size_t)blockIdx.x * a.H + h) * LC * DV;
-  auto u_put = [&](int p, int c, float x, float y) { *reinterpret_cast<float2*>(u + p * DV + c) = make_float2(x, y); };
-  if (odd) scalar(bs, vg, a.ldv, u_put);
-  else product(bs, [] {}, u_put);
-}
-
 // ----------------------------------------------------------------------------------- the states before the chunks
-// Plain.  grid (DV D / 4 / LC_THREADS, H, requests)
+// grid (DV D / 4 / LC_THREADS, H, requests)
 template <int D, int DV>
 __global__ void __launch_bounds__(LC_THREADS)
 linear_chunk_states_kernel(LinearChunk a) {
@@ -476,168 +288,11 @@ linear_chunk_states_kernel(LinearChunk a) {
   if (a.write_state) *S = s;
 }
 
-// Delta rule.  grid (DV / 32, H, requests): a CTA takes 32 value columns of a head through the request's chunks.  S [j][i] is 32 x D:
-// a warp has D / 8 of the i.
-#define LC_COLS 32
-template <int D, int DV>
-__global__ void __launch_bounds__(LC_THREADS)
-linear_chunk_delta_kernel(LinearChunk a) {
-  pdl_launch_dependents();
-  pdl_wait();
-  extern __shared__ __align__(16) unsigned char lc_sm[];
-  using TW = LcTile<LC, D>;
-  using TS = LcTile<LC_COLS, D>;
-  using TX = LcTile<LC, LC_COLS>;
-  bf16* wbuf = reinterpret_cast<bf16*>(lc_sm);                          // two chunks' pieces of W: the next one's are long on their way
-  bf16* ks = wbuf + 2 * TW::ELEMS;
-  bf16* ss = ks + TW::ELEMS;
-  bf16* xs = ss + TS::ELEMS;
-  float* ubuf = reinterpret_cast<float*>(xs + TX::ELEMS);               // two of [LC][LC_COLS + 4]
-  constexpr int LU = LC_COLS + 4, IW = D / 8, NP = IW / 16;             // a warp's columns of S; pairs of tiles among them
-  static_assert(IW % 16 == 0, "a warp has whole pairs of tiles");
-  const int h = blockIdx.y, req = blockIdx.z, j0 = blockIdx.x * LC_COLS, gk = h / (a.H / a.G);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t2 = (lane & 3) * 2;
-  int first = 0;
-  for (int r = 0; r < req; r++) first += (a.cu_tokens[r + 1] - a.cu_tokens[r] + LC - 1) / LC;
-  const int chunks = (a.cu_tokens[req + 1] - a.cu_tokens[req] + LC - 1) / LC;
-  if (!chunks) return;
-  auto pieces = [&](bf16* tile, const bf16* src) {
-    for (int e = tid; e < 3 * LC * (D / 8); e += LC_THREADS) {
-      const int row = e / (D / 8), c = (e - row * (D / 8)) * 8;
-      ts_cp_async16(tile + row * TW::LD + c, src + row * D + c, 16);
-    }
-  };
-  auto ask_w = [&](int c) {
-    const size_t at = (size_t)(first + c) * a.H + h;
-    float* us = ubuf + (c & 1) * LC * LU;
-    pieces(wbuf + (c & 1) * TW::ELEMS, a.w + at * 3 * LC * D);
-    for (int e = tid; e < LC * (LC_COLS / 4); e += LC_THREADS) {
-      const int row = e / (LC_COLS / 4), col = (e - row * (LC_COLS / 4)) * 4;
-      ts_cp_async16(us + row * LU + col, a.x + (at * LC + row) * DV + j0 + col, 16);
-    }
-  };
-  auto ask_k = [&](int c) { pieces(ks, a.kp + ((size_t)(first + c) * a.G + gk) * 3 * LC * D); };
-  ask_w(0);
-  ts_commit();
-  ask_k(0);
-  ts_commit();
-  if (chunks > 1) ask_w(1);
-  ts_commit();
-  // S: rows j of both tiles of 16, columns i of this warp
-  float* state = a.state + (size_t)a.slots[req] * a.state_stride + a.s_off + ((size_t)h * DV + j0) * D;
-  float S[2][NP][2][4];
-  const int i0 = warp * IW;
-  auto each = [&](auto&& f) {                         // f(pair of numbers, j, i)
-#pragma unroll
-    for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-      for (int np = 0; np < NP; np++)
-#pragma unroll
-        for (int t = 0; t < 2; t++)
-#pragma unroll
-          for (int e = 0; e < 4; e += 2) f(S[mt][np][t][e], S[mt][np][t][e + 1], mt * 16 + g + 4 * e, i0 + np * 16 + t * 8 + t2);
-  };
-  each([&](float& x, float& y, int j, int i) {
-    const float2 v = *reinterpret_cast<const float2*>(state + (size_t)j * D + i);
-    x = v.x;
-    y = v.y;
-  });
-  for (int c = 0; c < chunks; c++) {
-    const size_t at = (size_t)(first + c) * a.H + h;
-    float* s0 = a.s0 + (at * DV + j0) * D;
-    each([&](float& x, float& y, int j, int i) {      // the state before the chunk: for the outputs, and as pieces
-      *reinterpret_cast<float2*>(s0 + (size_t)j * D + i) = make_float2(x, y);
-      unsigned cut[3];
-      lc_cut(x, y, cut);
-#pragma unroll
-      for (int q = 0; q < 3; q++) *reinterpret_cast<unsigned*>(ss + q * TS::PIECE + j * TS::LD + i) = cut[q];
-    });
-    const float* dec = a.dec + at * LC_DEC;
-    const int m = (warp & 3) * 16, n0 = (warp >> 2) * 16;
-    const float d0 = dec[m + g], d1 = dec[m + g + 8], G = dec[LC];
-    const bf16* ws = wbuf + (c & 1) * TW::ELEMS;
-    const float* us = ubuf + (c & 1) * LC * LU;
-    ts_wait<2>();                                     // behind W of this chunk came W of the next and K of this
-    __syncthreads();
-    {                                                 // X = U - W S0: 16 tokens by 16 columns a warp
-      float y[2][4], s[2][4], y1[2][4], s1[2][4];      // even and odd blocks of k in sums of their own: half as long a chain
-      lc_zero(y);
-      lc_zero(s);
-      lc_zero(y1);
-      lc_zero(s1);
-#pragma unroll
-      for (int kk = 0; kk < D / 16; kk++) {
-        unsigned fa[3][4], fb[3][4];
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-          lc_a(fa[i], ws + i * TW::PIECE, TW::LD, m, kk * 16, lane);
-          lc_b(fb[i], ss + i * TS::PIECE, TS::LD, kk * 16, n0, lane);
-        }
-        if (kk & 1) lc_mma(y1, s1, fa, fb);
-        else lc_mma(y, s, fa, fb);
-      }
-#pragma unroll
-      for (int t = 0; t < 2; t++)
-#pragma unroll
-        for (int e = 0; e < 4; e++) { y[t][e] += y1[t][e]; s[t][e] += s1[t][e]; }
-      float* xg = a.x + at * LC * DV + j0;
-#pragma unroll
-      for (int t = 0; t < 2; t++)
-#pragma unroll
-        for (int e = 0; e < 4; e += 2) {
-          const int p = m + g + 4 * e, j = n0 + t * 8 + t2;
-          const float2 u = *reinterpret_cast<const float2*>(us + p * LU + j);
-          const float x0 = u.x - (y[t][e] + s[t][e]), x1 = u.y - (y[t][e + 1] + s[t][e + 1]), d = e ? d1 : d0;
-          *reinterpret_cast<float2*>(xg + (size_t)p * DV + j) = make_float2(x0, x1);
-          unsigned cut[3];
-          lc_cut(d * x0, d * x1, cut);
-#pragma unroll
-          for (int q = 0; q < 3; q++) *reinterpret_cast<unsigned*>(xs + q * TX::PIECE + p * TX::LD + j) = cut[q];
-        }
-    }
-    __syncthreads();
-    if (c + 2 < chunks) ask_w(c + 2);
-    ts_commit();
-    ts_wait<1>();
-    __syncthreads();
-#pragma unroll
-    for (int np = 0; np < NP; np++) {
-      float y[2][2][4], s[2][2][4];
-#pragma unroll
-      for (int mt = 0; mt < 2; mt++) { lc_zero(y[mt]); lc_zero(s[mt]); }
-#pragma unroll
-      for (int kk = 0; kk < LC / 16; kk++) {
-        unsigned fa[2][3][4], fb[3][4];
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-          lc_b_t(fb[i], ks + i * TW::PIECE, TW::LD, kk * 16, i0 + np * 16, lane);
-#pragma unroll
-          for (int mt = 0; mt < 2; mt++) lc_a_t(fa[mt][i], xs + i * TX::PIECE, TX::LD, mt * 16, kk * 16, lane);
-        }
-#pragma unroll
-        for (int mt = 0; mt < 2; mt++) lc_mma(y[mt], s[mt], fa[mt], fb);
-      }
-#pragma unroll
-      for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-        for (int t = 0; t < 2; t++)
-#pragma unroll
-          for (int e = 0; e < 4; e++) S[mt][np][t][e] = fmaf(G, S[mt][np][t][e], y[mt][t][e] + s[mt][t][e]);
-    }
-    __syncthreads();
-    if (c + 1 < chunks) ask_k(c + 1);
-    ts_commit();
-  }
-  ts_wait<0>();
-  if (a.write_state)
-    each([&](float& x, float& y, int j, int i) { *reinterpret_cast<float2*>(state + (size_t)j * D + i) = make_float2(x, y); });
-}
-
 // ------------------------------------------------------------------------------------------------ the outputs
 // out[t, h] = o / sqrt(mean(o^2) + eps) (* norm) * gate * out_scale with o as above.  grid (chunks, H); a warp has 16 tokens by a
 // quarter of the columns, and of the products of q and k 16 tokens by 16.
 #define LC_OUT_THREADS 512
-template <int D, int DV, bool DELTA>
+template <int D, int DV>
 __global__ void __launch_bounds__(LC_OUT_THREADS)
 linear_chunk_out_kernel(LinearChunk a) {
   pdl_launch_dependents();
@@ -650,7 +305,7 @@ linear_chunk_out_kernel(LinearChunk a) {
   constexpr int FIRST = TS::ELEMS > TK::ELEMS + TX::ELEMS ? TS::ELEMS : TK::ELEMS + TX::ELEMS;
   static_assert(TP::ELEMS <= TK::ELEMS, "");
   bf16* qs = reinterpret_cast<bf16*>(lc_sm);
-  bf16* ss = qs + TK::ELEMS;                          // the state; after it K and X
+  bf16* ss = qs + TK::ELEMS;                          // the state; after it K and V
   bf16* ks = ss;
   bf16* xs = ks + TK::ELEMS;
   bf16* ps = ks;                                      // d(s, p) (k_s . q_p), in the keys' place
@@ -663,15 +318,14 @@ linear_chunk_out_kernel(LinearChunk a) {
   if (!lc_find(a, blockIdx.x, r, t0, n)) return;
   const int h = blockIdx.y, gk = h / (a.H / a.G), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t2 = (lane & 3) * 2;
   const size_t at = (size_t)blockIdx.x * a.H + h;
-  const float* xg = DELTA ? a.x + at * LC * DV : a.v + (size_t)t0 * a.ldv + (size_t)h * DV;
-  const long long ldx = DELTA ? DV : a.ldv;
+  const float* xg = a.v + (size_t)t0 * a.ldv + (size_t)h * DV;
   lc_fill<LC, D, LC_OUT_THREADS>(qs, a.q + ((size_t)t0 * a.G + gk) * D, (long long)a.G * D, n);
   lc_fill<DV, D, LC_OUT_THREADS>(ss, a.s0 + at * DV * D, D, DV);
   lc_decays(a, t0, n, h, gs, dm);
-  // K and X are on their way while the state's product is made
+  // K and V are on their way while the state's product is made
   float4 kx[LC * D / 4 / LC_OUT_THREADS], xx[LC * DV / 4 / LC_OUT_THREADS];
   lc_ask<LC, D, LC_OUT_THREADS>(kx, a.k + ((size_t)t0 * a.G + gk) * D, (long long)a.G * D, n);
-  lc_ask<LC, DV, LC_OUT_THREADS>(xx, xg, ldx, n);
+  lc_ask<LC, DV, LC_OUT_THREADS>(xx, xg, a.ldv, n);
   constexpr int NP = DV / 64;
   // (a scheduler's four warps have all four rows of tiles: their triangular products are of different lengths)
   const int part = warp >> 2, m = ((warp + part) & 3) * 16, c0 = part * (DV / 4);
@@ -761,7 +415,7 @@ linear_chunk_out_kernel(LinearChunk a) {
         for (int e = 0; e < 4; e++) {
           const int p = m + g + 8 * (e >> 1), j = c0 + np * 16 + t * 8 + t2 + (e & 1);
           float y = 0.f;
-          for (int s = 0; s <= p && s < n; s++) y = fmaf(dm[p * LC_DM + s], xg[s * ldx + j], y);
+          for (int s = 0; s <= p && s < n; s++) y = fmaf(dm[p * LC_DM + s], xg[s * a.ldv + j], y);
           s2[np][t][e] = y;
         }
   } else {
@@ -815,24 +469,17 @@ linear_chunk_out_kernel(LinearChunk a) {
 }
 
 // ------------------------------------------------------------------------------------------------ host
-// Whether the sizes are taken: whole heads of 64 x 64 (without the delta rule) or 128 x 128, and portions that are long enough on
-// the average.  Measured on a B200, us a call, chunks / token by token, 32 heads: plain, 64 x 64: 128 tokens 17.2 / 16.5, 256 18.7 / 29.2,
-// 1,500 66 / 155, three portions of 200 34 / 42, eight of 128 49 / 43; delta rule, 128 x 128: 400 tokens 85 / 87, 700 136 / 148,
-// 1,500 266 / 316, 2,048 344 / 429, three portions of 400 240 / 222.
-#define LC_MEAN_PLAIN 192
-#define LC_MEAN_DELTA 512
+// Whether the sizes are taken: whole heads of 64 x 64 or 128 x 128 without the delta rule, and portions that are long enough on the
+// average.  Measured on a B200, us a call, chunks / token by token, 32 heads of 64 x 64: 128 tokens 17.2 / 16.5, 256 18.7 / 29.2,
+// 1,500 66 / 155, three portions of 200 34 / 42, eight of 128 49 / 43.
+#define LC_MEAN 192
 static bool lc_takes(int T, int R, int d, int dv, int DP, bool delta, int nrm) {
-  return !nrm && d == DP && dv == d && (d == 128 || (d == 64 && !delta)) && (long long)T >= (long long)(delta ? LC_MEAN_DELTA : LC_MEAN_PLAIN) * R;
+  return !nrm && !delta && d == DP && dv == d && (d == 128 || d == 64) && (long long)T >= (long long)LC_MEAN * R;
 }
 static long long lc_chunks(int T, int R) { return (long long)T / LC + R; }      // no fewer than there are
 
 // floats of scratch
-static long long lc_scratch(int T, int R, int H, int G, int d, bool delta) {
-  const long long c = lc_chunks(T, R);
-  long long n = c * H * LC_DEC + c * H * d * d;
-  if (delta) n += c * H * LC * d + (c * H * 3 * LC * d + c * G * 3 * LC * d) / 2;
-  return n;
-}
+static long long lc_scratch(int T, int R, int H, int d) { return lc_chunks(T, R) * H * (LC_DEC + d * d); }
 
 template <int D>
 static int lc_launch(LinearChunk a, float* scratch, cudaStream_t stream) {
@@ -840,9 +487,6 @@ static int lc_launch(LinearChunk a, float* scratch, cudaStream_t stream) {
   if (c > 65535 || a.H > 65535 || a.R > 65535) return QD_ERR_UNSUPPORTED;
   a.s0 = scratch;
   a.dec = a.s0 + c * a.H * D * D;
-  a.x = a.dec + c * a.H * LC_DEC;
-  a.w = reinterpret_cast<bf16*>(a.x + c * a.H * LC * D);
-  a.kp = a.w + c * a.H * 3 * LC * D;
   const dim3 grid((unsigned)c, a.H);
   constexpr size_t tile = LcTile<LC, D>::ELEMS * sizeof(bf16), state = LcTile<D, D>::ELEMS * sizeof(bf16), dm = LC * LC_DM * sizeof(float);
   constexpr size_t out = tile + (state > 2 * tile ? state : 2 * tile) + dm;
@@ -850,19 +494,8 @@ static int lc_launch(LinearChunk a, float* scratch, cudaStream_t stream) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     qd_launch(kernel, g, dim3(threads), smem, stream, a);
   };
-  if (a.beta) {
-    constexpr size_t delta = 3 * tile + (LcTile<LC_COLS, D>::ELEMS + LcTile<LC, LC_COLS>::ELEMS) * sizeof(bf16) + 2 * LC * (LC_COLS + 4) * sizeof(float);
-    if constexpr (D == 128) {
-      go(linear_chunk_solve_kernel<D, D>, grid, tile + 3 * dm);
-      go(linear_chunk_delta_kernel<D, D>, dim3(D / LC_COLS, a.H, a.R), delta);
-      go(linear_chunk_out_kernel<D, D, true>, grid, out, LC_OUT_THREADS);
-    } else {
-      return QD_ERR_UNSUPPORTED;
-    }
-  } else {
-    go(linear_chunk_add_kernel<D, D>, grid, 2 * tile);
-    go(linear_chunk_states_kernel<D, D>, dim3(D * D / 4 / LC_THREADS, a.H, a.R), 0);
-    go(linear_chunk_out_kernel<D, D, false>, grid, out, LC_OUT_THREADS);
-  }
+  go(linear_chunk_add_kernel<D, D>, grid, 2 * tile);
+  go(linear_chunk_states_kernel<D, D>, dim3(D * D / 4 / LC_THREADS, a.H, a.R), 0);
+  go(linear_chunk_out_kernel<D, D>, grid, out, LC_OUT_THREADS);
   return qd_last_error();
 }

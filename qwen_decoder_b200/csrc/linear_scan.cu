@@ -1068,7 +1068,7 @@ extern "C" int qd_linear_scan(const float* q, const float* k, const float* v, lo
                               float q_scale, float k_scale, float* chunk, cudaStream_t stream) {
   if (T <= 0 || n_requests <= 0) return 0;
   if (H <= 0 || H > 65535 || n_requests > 65535 || G <= 0 || H % G || d <= 0 || dv <= 0 || dv > 8192 || d > DP ||
-      !state || !gate || (g_ld && g_ld != H) || (beta && T != n_requests && !chunk && (!coef || ((uintptr_t)coef & 15))) || (out_dtype != QD_F32 && out_dtype != QD_BF16))
+      !state || !gate || (g_ld && g_ld != H) || (beta && T != n_requests && (!coef || ((uintptr_t)coef & 15))) || (out_dtype != QD_F32 && out_dtype != QD_BF16))
     return QD_ERR_UNSUPPORTED;
   const bool single = T == n_requests;                // every request has at least one token
   if (!single && !o_buf && !chunk) return QD_ERR_UNSUPPORTED;
@@ -1082,8 +1082,8 @@ extern "C" int qd_linear_scan(const float* q, const float* k, const float* v, lo
     if (single || !vec || !g || ldv % 4 || gate_ld % 2 || out_stride % 2 || (((uintptr_t)v | (uintptr_t)chunk) & 15) || ((uintptr_t)gate & 7) ||
         ((uintptr_t)out & (out_dtype == QD_F32 ? 7 : 3)) || !lc_takes(T, n_requests, d, dv, DP, beta != nullptr, nrm))
       return QD_ERR_UNSUPPORTED;
-    const LinearChunk c = {q, k, v, ldv, g, g_ld, beta, T, n_requests, H, G, state, state_stride, s_off, cu_tokens, slots, write_state,
-                           nullptr, nullptr, nullptr, nullptr, nullptr, gate, gate_ld, norm, norm_ld, eps, out_scale, gate_kind, out,
+    const LinearChunk c = {q, k, v, ldv, g, g_ld, T, n_requests, H, G, state, state_stride, s_off, cu_tokens, slots, write_state,
+                           nullptr, nullptr, gate, gate_ld, norm, norm_ld, eps, out_scale, gate_kind, out,
                            out_dtype, out_stride};
     return d == 64 ? lc_launch<64>(c, chunk, stream) : lc_launch<128>(c, chunk, stream);
   }
@@ -1166,5 +1166,5 @@ extern "C" long long qd_linear_chunk_scratch(int T, int n_requests, int H, int G
   if (T <= 0 || n_requests <= 0 || T == n_requests || H <= 0 || G <= 0 || H > 65535 || n_requests > 65535 ||
       lc_chunks(T, n_requests) > 65535 || !lc_takes(T, n_requests, d, dv, DP, delta != 0, nrm))
     return 0;
-  return lc_scratch(T, n_requests, H, G, d, delta != 0);
+  return lc_scratch(T, n_requests, H, d);
 }
