@@ -110,6 +110,22 @@ def test_delta_rule_with_keys_alike(common, monkeypatch):
         err(got, want), err(state.cpu()[slots], states[slots]))
 
 
+# outputs and states no further from float64 than token by token, but for two roundings to float32, 2^-24 each
+@pytest.mark.parametrize("decay", [(0.3, 1.0), (0.9, 1.0), (0.99, 1.0)])
+@pytest.mark.parametrize("common", [0.0, 0.9, 0.99])
+@pytest.mark.parametrize("d", [64, 128])
+def test_no_less_precise(d, common, decay, monkeypatch):
+    p = make([700], 4, 2, d, False, True, seed=2, decay=decay, common=common)
+    want, states = reference(p)
+    err = lambda a, b: float((a.double().cpu() - b).norm() / b.norm())
+    slots, errors = p.ctx.state_slots.long().cpu(), []
+    for chunks in (True, False):
+        out, state, floats = run(p, monkeypatch, chunks)
+        errors.append((err(out, want), err(state.cpu()[slots], states[slots])))
+        assert floats > 0
+    assert all(new <= max(before, 2.0 ** -23) for new, before in zip(*errors)), errors
+
+
 @pytest.mark.parametrize("d,delta", [(64, False), (128, False)])
 def test_options(d, delta, monkeypatch):
     p = make([980, 100], 2, 1, d, delta, True, seed=5)
