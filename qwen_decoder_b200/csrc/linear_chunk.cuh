@@ -4,7 +4,7 @@
 //
 //   o_p = G_p S0^T q_p + sum_(s <= p) d(s, p) (k_s . q_p) v_s,   S <- G S0 + sum_s d(s, last) k_s v_s^T
 //
-// Three launches: what a chunk adds to the state, sum_s d(s, last) k_s v_s^T, all chunks at once; the states before the chunks, one
+// Three launches a pass of as many chunks as the scratch holds: what a chunk adds to the state, sum_s d(s, last) k_s v_s^T, all chunks at once; the states before the chunks, one
 // after the other; the outputs with norm and gate, all chunks at once.
 //
 // The delta rule has no such form here.  There the values' place is taken by the solution of a triangular system a chunk, and rounded
@@ -40,14 +40,19 @@ struct LinearChunk {
   const int *cu_tokens, *slots; int write_state;
   float* dec;                             // [chunk, H, LC_DEC]
   float* s0;                              // [chunk, H, DV, D]: what the chunk adds to the state, then the state before it
+  // The pass: chunks c0 .. c0 + pass - 1 of all (the arrays above hold these), and the state of the request that is cut between two
+  // passes, [H, DV, D]: as the pass before left it, and for the next one (another place: two requests may meet in one pass).
+  int c0, pass;
+  const float* from; float* to;
   // norm, gate and result, as LinearFinish in linear_scan.cu
   const float* gate; long long gate_ld; const float* norm; int norm_ld; float eps, out_scale; int gate_kind;
   void* out; int out_dtype; long long out_stride;
 };
 
-// Chunk ``b`` of all: its request, its first token and how many it has; false past the last one.
+// The pass's chunk ``b``: its request, its first token and how many it has; false past the last one.
 __device__ __forceinline__ bool lc_find(const LinearChunk& a, int b, int& r, int& t0, int& n) {
   int at = 0;
+  b += a.c0;
   for (r = 0; r < a.R; r++) {
     const int begin = a.cu_tokens[r], end = a.cu_tokens[r + 1], chunks = (end - begin + LC - 1) / LC;
     if (b < at + chunks) {
@@ -286,11 +291,12 @@ linear_chunk_states_kernel(LinearChunk a) {
   pdl_launch_dependents();
   pdl_wait();
   const int h = blockIdx.y, req = blockIdx.z, e = blockIdx.x * LC_THREADS + threadIdx.x;
-  int first = 0;
-  for (int r = 0; r < req; r++) first += (a.cu_tokens[r + 1] - a.cu_tokens[r] + LC - 1) / LC;
-  const int chunks = (a.cu_tokens[req + 1] - a.cu_tokens[req] + LC - 1) / LC;
+  int at = -a.c0;                                     // where the request's first chunk is in the pass, or would be
+  for (int r = 0; r < req; r++) at += (a.cu_tokens[r + 1] - a.cu_tokens[r] + LC - 1) / LC;
+  const int end = at + (a.cu_tokens[req + 1] - a.cu_tokens[req] + LC - 1) / LC, first = max(at, 0), chunks = min(end, a.pass) - first;
+  if (chunks <= 0) return;
   float4* S = reinterpret_cast<float4*>(a.state + (size_t)a.slots[req] * a.state_stride + a.s_off + (size_t)h * DV * D) + e;
-  float4 s = *S;
+  float4 s = at < 0 ? reinterpret_cast<const float4*>(a.from + (size_t)h * DV * D)[e] : *S;
   constexpr int AHEAD = 8;
   for (int c0 = 0; c0 < chunks; c0 += AHEAD) {
     float4 add[AHEAD];
@@ -309,7 +315,8 @@ linear_chunk_states_kernel(LinearChunk a) {
         s = make_float4(fmaf(G[i], s.x, add[i].x), fmaf(G[i], s.y, add[i].y), fmaf(G[i], s.z, add[i].z), fmaf(G[i], s.w, add[i].w));
       }
   }
-  if (a.write_state) *S = s;
+  if (end > a.pass) reinterpret_cast<float4*>(a.to + (size_t)h * DV * D)[e] = s;      // goes on in the next pass
+  else if (a.write_state) *S = s;
 }
 
 // ------------------------------------------------------------------------------------------------ the outputs
@@ -502,24 +509,46 @@ static bool lc_takes(int T, int R, int d, int dv, int DP, bool delta, int nrm) {
 }
 static long long lc_chunks(int T, int R) { return (long long)T / LC + R; }      // no fewer than there are
 
-// floats of scratch
-static long long lc_scratch(int T, int R, int H, int d) { return lc_chunks(T, R) * H * (LC_DEC + d * d); }
+// Scratch.  A chunk of 32 heads of 128 takes 2.1 MB, 33 KB a token: a step of 32,768 tokens would take 1.1 GB beside a cache that was
+// given the rest of the memory.  So there are no more chunks at a time than LC_SCRATCH floats hold (64 MB: 1,800 of those tokens, 7,900
+// of 32 heads of 64), and where that is not one chunk, none.  A pass more costs 6 to 10 us where all fits into L2 and gives some back
+// where it does not: 1,500 tokens of 32 heads of 64 in one, two and four passes 69, 75 and 102 us, 6,000 of 128 734, 750 and 681.
+#define LC_SCRATCH (16ll << 20)
+static long long lc_floats(int H, int d) { return (long long)H * (LC_DEC + d * d); }       // of a chunk
+static long long lc_carry(int H, int d) { return 2ll * H * d * d; }                        // with more than one pass
+// chunks of a pass with ``floats`` of scratch, 0: too few
+static long long lc_pass(int T, int R, int H, int d, long long floats) {
+  const long long all = lc_chunks(T, R), one = lc_floats(H, d);
+  if (floats / one >= all) return all;
+  return floats < lc_carry(H, d) + one ? 0 : (floats - lc_carry(H, d)) / one;
+}
+static long long lc_scratch(int T, int R, int H, int d) {
+  const long long pass = lc_pass(T, R, H, d, LC_SCRATCH);
+  return pass * lc_floats(H, d) + (pass > 0 && pass < lc_chunks(T, R) ? lc_carry(H, d) : 0);
+}
 
 template <int D>
-static int lc_launch(LinearChunk a, float* scratch, cudaStream_t stream) {
-  const long long c = lc_chunks(a.T, a.R);
-  if (c > 65535 || a.H > 65535 || a.R > 65535) return QD_ERR_UNSUPPORTED;
+static int lc_launch(LinearChunk a, float* scratch, long long floats, cudaStream_t stream) {
+  const long long all = lc_chunks(a.T, a.R), c = lc_pass(a.T, a.R, a.H, D, floats);
+  if (c < 1 || all > 65535 || a.H > 65535 || a.R > 65535) return QD_ERR_UNSUPPORTED;
   a.s0 = scratch;
   a.dec = a.s0 + c * a.H * D * D;
-  const dim3 grid((unsigned)c, a.H);
+  float* carry = a.dec + c * a.H * LC_DEC;
   constexpr size_t tile = LcTile<LC, D>::ELEMS * sizeof(bf16), state = LcTile<D, D>::ELEMS * sizeof(bf16), dm = LC * LC_DM * sizeof(float);
   constexpr size_t out = tile + (state > 2 * tile ? state : 2 * tile) + dm;
   auto go = [&](auto kernel, dim3 g, size_t smem, int threads = LC_THREADS) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     qd_launch(kernel, g, dim3(threads), smem, stream, a);
   };
-  go(linear_chunk_add_kernel<D, D>, grid, 2 * tile);
-  go(linear_chunk_states_kernel<D, D>, dim3(D * D / 4 / LC_THREADS, a.H, a.R), 0);
-  go(linear_chunk_out_kernel<D, D>, grid, out, LC_OUT_THREADS);
+  for (long long c0 = 0, i = 0; c0 < all; c0 += c, i++) {
+    a.c0 = (int)c0;
+    a.pass = (int)(all - c0 < c ? all - c0 : c);
+    a.from = carry + (i & 1) * a.H * D * D;
+    a.to = carry + (~i & 1) * a.H * D * D;
+    const dim3 grid(a.pass, a.H);
+    go(linear_chunk_add_kernel<D, D>, grid, 2 * tile);
+    go(linear_chunk_states_kernel<D, D>, dim3(D * D / 4 / LC_THREADS, a.H, a.R), 0);
+    go(linear_chunk_out_kernel<D, D>, grid, out, LC_OUT_THREADS);
+  }
   return qd_last_error();
 }

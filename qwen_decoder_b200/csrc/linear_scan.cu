@@ -1054,8 +1054,8 @@ linear_step_kernel(LinearScan a, LinearFinish f, ExpGates eg) {
 // gate float32 rows ``gate_ld`` apart; norm float32 [dv] (norm_ld 0) or [H, dv] (norm_ld dv), or null; gate_kind 0 silu, 1 sigmoid.
 // ``nrm``: exponential gates.  S is [H, dv + 1, d] at ``s_off``, the maxima at ``m_off``; portions: nq scratch [T, H], g, low and k
 // as ``qd_linear_exp_gates`` and ``qd_linear_prep`` made them; single tokens: g unused, the logits are columns i_off, f_off of u.
-// ``chunk``: scratch of qd_linear_chunk_scratch floats, 16-byte aligned, for the form in chunks (linear_chunk.cuh; then o_buf and coef
-// are unused), or null.  It wants rows of v and state in 16-byte pieces, of gate in 8-byte ones, of out in pairs.
+// ``chunk``: scratch of ``chunk_floats`` floats (qd_linear_chunk_scratch says how many; fewer make more passes), 16-byte aligned, for
+// the form in chunks (linear_chunk.cuh; then o_buf and coef are unused), or null.  It wants rows of v and state in 16-byte pieces, of gate in 8-byte ones, of out in pairs.
 // ``raw`` (single tokens): q and k are rows of G * d numbers ``q_ld`` apart that q_scale and k_scale still multiply.
 extern "C" int qd_linear_scan(const float* q, const float* k, const float* v, long long ldv, const float* g, int g_ld,
                               const float* beta, int T, int n_requests, int H, int G, int d, int dv, int DP,
@@ -1065,7 +1065,7 @@ extern "C" int qd_linear_scan(const float* q, const float* k, const float* v, lo
                               long long out_stride, const int* token_req, float* coef, int norm_ld, int gate_kind, int nrm,
                               float* nq, const float* low, const float* u, long long u_ld, int i_off, int f_off,
                               const float* ib, const float* fb, float cap, long long m_off, int raw, long long q_ld,
-                              float q_scale, float k_scale, float* chunk, cudaStream_t stream) {
+                              float q_scale, float k_scale, float* chunk, long long chunk_floats, cudaStream_t stream) {
   if (T <= 0 || n_requests <= 0) return 0;
   if (H <= 0 || H > 65535 || n_requests > 65535 || G <= 0 || H % G || d <= 0 || dv <= 0 || dv > 8192 || d > DP ||
       !state || !gate || (g_ld && g_ld != H) || (beta && T != n_requests && (!coef || ((uintptr_t)coef & 15))) || (out_dtype != QD_F32 && out_dtype != QD_BF16))
@@ -1083,9 +1083,9 @@ extern "C" int qd_linear_scan(const float* q, const float* k, const float* v, lo
         ((uintptr_t)out & (out_dtype == QD_F32 ? 7 : 3)) || !lc_takes(T, n_requests, d, dv, DP, beta != nullptr, nrm))
       return QD_ERR_UNSUPPORTED;
     const LinearChunk c = {q, k, v, ldv, g, g_ld, T, n_requests, H, G, state, state_stride, s_off, cu_tokens, slots, write_state,
-                           nullptr, nullptr, gate, gate_ld, norm, norm_ld, eps, out_scale, gate_kind, out,
+                           nullptr, nullptr, 0, 0, nullptr, nullptr, gate, gate_ld, norm, norm_ld, eps, out_scale, gate_kind, out,
                            out_dtype, out_stride};
-    return d == 64 ? lc_launch<64>(c, chunk, stream) : lc_launch<128>(c, chunk, stream);
+    return d == 64 ? lc_launch<64>(c, chunk, chunk_floats, stream) : lc_launch<128>(c, chunk, chunk_floats, stream);
   }
   const LinearScan a = {q, k, v, ldv, g, g_ld, beta, coef, H, G, d, dv, state, state_stride, s_off, vec, cu_tokens, slots,
                         write_state, nrm, nq, raw, q_ld, q_scale, k_scale};
@@ -1161,10 +1161,16 @@ extern "C" int qd_linear_scan(const float* q, const float* k, const float* v, lo
   return qd_last_error();
 }
 
-// Floats of scratch with which qd_linear_scan takes these portions in chunks, 0: it does not.
+// Floats of scratch with which qd_linear_scan takes these portions in chunks, 0: it does not.  Never more than LC_SCRATCH.
 extern "C" long long qd_linear_chunk_scratch(int T, int n_requests, int H, int G, int d, int dv, int DP, int delta, int nrm) {
   if (T <= 0 || n_requests <= 0 || T == n_requests || H <= 0 || G <= 0 || H > 65535 || n_requests > 65535 ||
       lc_chunks(T, n_requests) > 65535 || !lc_takes(T, n_requests, d, dv, DP, delta != 0, nrm))
     return 0;
   return lc_scratch(T, n_requests, H, d);
+}
+
+// How many passes of three launches such portions take with ``floats`` of scratch.
+extern "C" int qd_linear_chunk_passes(int T, int n_requests, int H, int d, long long floats) {
+  const long long c = T > 0 && n_requests > 0 && H > 0 && d > 0 ? lc_pass(T, n_requests, H, d, floats) : 0;
+  return c ? (int)((lc_chunks(T, n_requests) + c - 1) / c) : 0;
 }

@@ -1749,7 +1749,8 @@ def linear_exp_gates(e: ExpGates, H: int, state: torch.Tensor, ctx, write_state:
 
 
 def linear_chunk_scratch(T: int, R: int, H: int, G: int, d: int, dv: int, DP: int, delta: bool, nrm: int) -> int:
-    """Floats of scratch with which portions of T tokens of R requests go through the recurrence in chunks, 0: token by token."""
+    """Floats of scratch with which portions of T tokens of R requests go through the recurrence in chunks, 0: token by token.  Never
+    more than 2^24: longer portions go in several passes."""
     fn = library("linear_scan").qd_linear_chunk_scratch
     fn.restype = ctypes.c_longlong
     return int(fn(_I(T), _I(R), _I(H), _I(G), _I(d), _I(dv), _I(DP), _I(1 if delta else 0), _I(nrm)))
@@ -1817,9 +1818,11 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: Optional[t
         _ptr(coef), _I(dv if norm is not None and norm.numel() == H * dv else 0), _I(gate_kind), _I(nrm), _ptr(nq), _ptr(low),
         _ptr(e.u if nrm else None), _LL(e.u.stride(0) if nrm else 0), _I(e.i_off if nrm else 0), _I(e.f_off if nrm else 0),
         _ptr(e.i_bias if nrm else None), _ptr(e.f_bias if nrm else None), _F(e.cap if nrm else 1.0), _LL(e.m_off if nrm else 0),
-        _I(1 if raw else 0), _LL(q.stride(0) if raw else 0), _F(q_scale), _F(k_scale), _ptr(chunk), _stream()), "linear_scan")
+        _I(1 if raw else 0), _LL(q.stride(0) if raw else 0), _F(q_scale), _F(k_scale), _ptr(chunk), _LL(floats), _stream()), "linear_scan")
     if not single:
-        _launch_count[0] += 2 if floats or coef is not None else 1
+        _launch_count[0] += 1 if coef is None else 2
+        if floats:
+            _launch_count[0] += 3 * library("linear_scan").qd_linear_chunk_passes(_I(T), _I(ctx.num_requests), _I(H), _I(d), _LL(floats)) - 2
 
 
 # ------------------------------------------------------------------ norms in groups, before and after a branch

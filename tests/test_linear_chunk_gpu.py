@@ -168,3 +168,29 @@ def test_decays_of_all_sizes(monkeypatch):
         got, state, _ = run(p, monkeypatch, True)
         assert float((got.double().cpu() - want).norm() / want.norm()) <= 1e-5
         assert float((state.double().cpu() - states).norm() / states.norm()) <= 1e-6
+
+
+@pytest.mark.parametrize("d,lengths", [(64, [700]), (128, [130, 64, 600, 3]), (64, [64, 1000])])
+@pytest.mark.parametrize("chunks", [1, 3, 7])
+@pytest.mark.parametrize("write", [True, False])
+def test_passes(d, lengths, chunks, write, monkeypatch):
+    """Less scratch than all chunks take: the same bits from several passes, wherever they cut the requests."""
+    from qwen_decoder_b200 import kernels
+    p = make(lengths, 4, 2, d, False, True, seed=1)
+    want, state, floats = run(p, monkeypatch, True, write=write)
+    less = chunks * 4 * (68 + d * d) + 2 * 4 * d * d
+    assert 0 < less < floats
+    monkeypatch.setattr(kernels, "linear_chunk_scratch", lambda *a: less)
+    before = kernels.launches()
+    got, state2, _ = run(p, monkeypatch, True, write=write)
+    assert kernels.launches() - before == 3 * -(-(p.T // 64 + len(lengths)) // chunks)
+    assert torch.equal(got, want) and torch.equal(state2, state)
+    assert write or torch.equal(state2, p.state)
+
+
+def test_scratch_has_a_limit():
+    from qwen_decoder_b200 import kernels
+    for T, R, H, d in ((1500, 1, 32, 64), (32768, 1, 32, 128), (1 << 20, 3, 64, 128), (4000000, 1, 8, 64)):
+        floats = kernels.linear_chunk_scratch(T, R, H, H, d, d, d, False, 0)
+        assert 0 < floats <= 1 << 24
+    assert kernels.linear_chunk_scratch(1 << 20, 1, 1024, 1024, 128, 128, 128, False, 0) == 0          # not two states and a chunk
