@@ -113,6 +113,12 @@ __device__ __forceinline__ void gp_bias16(float (&v)[16], const float* bias, int
   for (int i = 0; i < 16; i++)
     if (col + i < feats) v[i] += bias[col + i];
 }
+// As the activation's own kernel over bfloat16 sums gives it.  A gate of minus infinity is its own result there: the quotient, by an
+// infinite exponential, would be no number.
+__device__ __forceinline__ float gp_gated(float g, float u, int act) {
+  const float y = __fdividef(g, 1.0f + __expf(-qd_gate_arg(g, act)));
+  return (g == -INFINITY ? g : y) * u;
+}
 // 16 numbers as pieces of 16 bytes of a row of 64 in a warp's part of shared memory.  Rows lie side by side, the pieces of rows
 // 2 i and 2 i + 1 turned by i: eight lanes that write or read together meet no bank twice.
 template <typename TO>
@@ -299,7 +305,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
               if (EPI == GP_GATED) {
                 if (bias) gp_bias16(u[i], bias + p.feats, col, p.feats);
 #pragma unroll
-                for (int j = 0; j < 16; j++) v[i][j] = __fdividef(v[i][j], 1.0f + __expf(-qd_gate_arg(v[i][j], p.act))) * u[i][j];
+                for (int j = 0; j < 16; j++) v[i][j] = gp_gated(v[i][j], u[i][j], p.act);
               }
               gp_stage16<TO>(rows, lane, i * (int)sizeof(TO), v[i]);
             }

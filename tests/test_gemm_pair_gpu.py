@@ -71,6 +71,22 @@ def test_gate_far_from_zero():
     torch.testing.assert_close(out.double()[want.abs() < 3e38], want[want.abs() < 3e38], rtol=2.0 ** -8, atol=1e-35)
 
 
+@pytest.mark.parametrize("act", [0, 2])
+def test_infinite_gates(act):
+    """As the activation's own kernel: minus infinity stays, and takes the other factor's sign."""
+    from qwen_decoder_b200 import kernels
+    T, F, K = 20, 64, 64
+    x, w, b = operands(T, 2 * F, K)
+    b[:16], b[16:32], b[F + 8:F + 24] = float("-inf"), float("inf"), 0.0
+    w[F + 8:F + 24] = 0.0                                # factors of zero: no numbers
+    out, want = (torch.empty(T, F, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    kernels.gemm_pair(x, w, b, out, 1, 128, 1, kernels.EPI_SWIGLU + 256 * act)
+    kernels.swiglu((x.double() @ w.double().T + b.double()).bfloat16(), want, act)
+    at = slice(0, 32)
+    assert torch.equal(out[:, at].isnan(), want[:, at].isnan()) and bool(want[:, 8:24].isnan().all())
+    assert torch.equal(out[:, at].nan_to_num(0.0), want[:, at].nan_to_num(0.0)) and bool(want[:, :8].isinf().all())
+
+
 def test_refusals():
     from qwen_decoder_b200 import kernels
     x, w, _ = operands(20, 64, 64, pad=0)
