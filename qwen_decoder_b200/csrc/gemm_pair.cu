@@ -360,6 +360,40 @@ static int* status_word() {
 
 static int up(int a, int b) { return (a + b - 1) / b; }
 
+// The gated product of more than GP_PLAIN_TOKENS tokens: one multiprocessor to a tile of 128 tokens or two to one of 256, whichever leaves
+// fewer of the MMA's rows empty, or the library's product with the activation after it.  Clocks of 1.9 GHz, fitted to times of 257 to 2,048
+// tokens in captured graphs, cold weights, at the 3B, 7B and mixed sizes and two more (6 % rms): a worker's rounds of blocks of 64 k, or W's
+// bytes, the longer of both and some of the other; the library's: 1.62 times what the tensor cores need and 12 us, about its best, less 5 %
+// (a 3B prompt of 300 tokens took 1.4 % longer so where the estimates were 4 % apart the other way).  Measured on a B200, us, as chosen ("-": the library) / two multiprocessors to every tile / the library:
+//   tokens          3B                       7B                      mixed
+//     257     - / 34.6 / 31.9          - / 91.5 / 70.1         17.3 / 20.4 / 17.6
+//     300     - / 34.8 / 33.3          - / 96.2 / 77.7         17.4 / 20.3 / 18.5
+//     340  31.7 / 35.0 / 32.6          - / 92.7 / 82.3         17.5 / 20.4 / 20.3
+//     384  32.0 / 35.3 / 33.4       86.5 / 93.6 / 84.8         17.5 / 20.6 / 19.5
+//     400  35.9 / 35.9 / 37.7          - / 93.6 / 91.5         20.5 / 20.8 / 22.1
+//     450  35.6 / 35.6 / 42.1       93.9 / 93.9 / 101.1        20.9 / 20.9 / 22.9
+//     512  37.0 / 37.0 / 43.9       95.3 / 95.3 / 110.0        21.0 / 21.0 / 25.3
+//     513  45.5 / 50.5 / 49.3          - / 134.8 / 115.7       23.8 / 27.0 / 25.6
+//     600  45.9 / 50.1 / 53.1      128.3 / 137.3 / 127.5       24.3 / 27.0 / 28.3
+//     769     - / 63.9 / 62.6          - / 186.8 / 180.4       32.7 / 34.2 / 34.5
+//   1,025  75.3 / 76.4 / 78.6          - / 236.6 / 235.6       40.4 / 40.4 / 42.2
+static int gp_plan_many(int T, int N, int K, int sms, int* cg_out, int* bn_out) {
+  const double dram = 2.0 * N * K / 3300.0, lib = 23000.0 + fmax(1.62 * T * N * K / (4096.0 * sms), 1.03 * dram);
+  const int kb = up(K, GP_BK);
+  double best = 0;
+  for (int cg = 1; cg <= 2; cg++) {
+    const int n_tt = up(T, 128 * cg), mrows = up(up(T, cg * n_tt), 8) * 8, workers = sms / cg;
+    for (int bn = 96; bn <= 256; bn += 32) {
+      const long long rounds = ((long long)up(N / 2, bn / 2) * n_tt + workers - 1) / workers;
+      const double block = cg == 1 ? fmax((bn < 256 ? 3.0 : 2.85) * bn, 120 + 1.9 * bn + 0.8 * mrows)
+                                   : fmax((bn < 256 ? 2.65 : 2.6) * bn, 350.0 + bn);
+      const double work = rounds * (double)kb * block, cost = fmax(work, dram) + 0.18 * fmin(work, dram) + 20.0 * bn;
+      if (best == 0 || cost < best) { best = cost; *cg_out = cg; *bn_out = bn; }
+    }
+  }
+  return best <= 0.95 * lib;
+}
+
 // How a product is cut, and whether it belongs here: *cg, *bn, *splits; 0 if the library's product is the faster one.  ``epi`` as
 // below; GP_PARTIAL: the caller takes whole bfloat16 sums (splits 1) or float32 partial sums.
 //
@@ -381,6 +415,10 @@ extern "C" int qd_gemm_pair_plan(int T, int N, int K, int epi, int sms, int* cg_
   if ((long long)N * K < (1 << 20)) return 0;        // small models: a launch's own time
   if (epi != GP_GATED && T > GP_PLAIN_TOKENS && (T < GP_WIDE_TOKENS || N < 4 * K)) return 0;
   if (epi == GP_PARTIAL && T > 128 && K < 2 * N) return 0;
+  if (epi == GP_GATED && T > GP_PLAIN_TOKENS) {
+    *splits_out = 1;
+    return gp_plan_many(T, N, K, sms, cg_out, bn_out);
+  }
   const int cg = T <= 128 ? 1 : 2, workers = sms / cg, n_tt = up(T, 128 * cg), mrows = up(up(T, cg * n_tt), 8) * 8;
   const int feats = epi == GP_GATED ? N / 2 : N, kb = up(K, GP_BK);
   const double dram = 2.0 * N * K / 3300.0;          // clocks of 1.9 GHz
