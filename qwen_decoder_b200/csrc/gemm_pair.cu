@@ -32,8 +32,7 @@
 #define GP_STAGE_ROWS (32 * 64)       // of a warp's epilogue: 64 bytes of each of its rows
 #define GP_BK 64
 
-#define GP_PLAIN_TOKENS 256           // beyond these only the gated product is taken, and very wide ones of
-#define GP_WIDE_TOKENS 1024           // so many tokens
+#define GP_PLAIN_TOKENS 256           // beyond these only the gated product is taken
 
 #define GP_STORE 0
 #define GP_PARTIAL 1
@@ -400,20 +399,22 @@ static int gp_plan_many(int T, int N, int K, int sms, int* cg_out, int* bn_out) 
 // Up to 128 tokens one multiprocessor to a tile, beyond two.  The rest by what a worker's busiest share takes: rounds over its items
 // times blocks of k, a block being the longest of its MMAs (2 bn clocks), its bytes (60 a clock into shared memory) and the 350
 // clocks that one costs anyway; or W's bytes at 6.3 TB/s; the longer of both and some of the other; plus an item's epilogue and the partial sums' way through L2.
-// Measured on a B200, us, here / the library (the gated product with its activation, the others of 64 and 200 tokens with the norm
-// that follows), 3B and 7B sizes:
-//   tokens       gate and up        down              output proj.      q/k/v
-//     64      18.5 / 21.8 46.2/52.5  13.7 / 18.9 30.2/33.6   7.2 / 8.2 10.5/10.9   5.1 / 5.8  8.1/9.0
-//    200      22.4 / 29.6 55.3/62.2  16.4 / 20.0 38.7/46.0   8.9 / 8.8 14.9/13.8   6.5 / 7.2 10.6/12.7
-//    512      37.2 / 44.1 97.3/105.9 27.0 / 27.1 66.6/60.5  13.0 /10.8 20.4/17.4   9.6 / 7.5 16.9/15.1
-//   2048       123 /  147  359/385   75.5 / 72.7  213/207   23.6 /22.5 54.8/55.4  18.8 /17.2 45.8/44.8
-// A projection over the vocabulary of 17 to 100 tokens: 100 to 110 / 108 to 126 and 166 to 175 / 186 to 195; 2,048 to 12,352
-// features of 17, 48, 300 and 1,500 tokens 11 / 12, 11 / 12, 19 / 16, 57 / 59.
+// Measured on a B200, us, here / the library (the gated product with its activation, the others with the norm that follows), 3B and 7B:
+//   tokens       gate and up                down                 output projection
+//     64      18.1 / 21.7 45.0/51.8  14.0 / 19.0 29.0/33.9   7.3 / 8.2 11.3/11.2
+//    192      21.7 / 25.9 55.2/60.6  16.8 / 19.9 36.4/47.1     - / 8.7    - /12.4
+//    512      37.0 / 43.9 95.3/110     - / 27.1    - /60.5     - /10.8    - /17.4
+// Whole sums: a projection over the vocabulary alone.  float32 results, 151,936 x 2,048 and 152,064 x 3,584: 17 rows 99 / 107 and 166 / 185,
+// 128 rows 117 / 140 and 202 / 219, 256 rows 145 / 187 and 248 / 325; 32,000 x 2,048: 64 rows 26.5 / 27.8, 128 rows 28.3 / 30.9, but 160 rows
+// 31.9 / 31.2.  Fewer features are the library's at any number of tokens: 12,352 x 2,048, 64 rows 11.6 / 11.8, 129 rows 15.1 / 13.1, 1,025
+// rows 49.2 / 41.3, 1,500 rows 57.8 / 57.7; 8,192 x 2,048 in bfloat16, 64 rows 9.6 / 8.7, 1,281 rows 35.6 / 31.2; q/k/v of the 3B sizes, 64
+// rows 7.5 / 5.8.
 extern "C" int qd_gemm_pair_plan(int T, int N, int K, int epi, int sms, int* cg_out, int* bn_out, int* splits_out) {
   epi &= 255;
   if (T <= 0 || N <= 0 || K <= 0 || sms < 2) return 0;
   if ((long long)N * K < (1 << 20)) return 0;        // small models: a launch's own time
-  if (epi != GP_GATED && T > GP_PLAIN_TOKENS && (T < GP_WIDE_TOKENS || N < 4 * K)) return 0;
+  if (epi != GP_GATED && T > GP_PLAIN_TOKENS) return 0;
+  if (epi == GP_STORE && N < (T <= 128 ? 30000 : 100000)) return 0;
   if (epi == GP_PARTIAL && T > 128 && K < 2 * N) return 0;
   if (epi == GP_GATED && T > GP_PLAIN_TOKENS) {
     *splits_out = 1;
@@ -439,7 +440,7 @@ extern "C" int qd_gemm_pair_plan(int T, int N, int K, int epi, int sms, int* cg_
     }
   }
   // whole sums of a long k by few workers: the library shares k
-  return epi != GP_STORE || T > GP_PLAIN_TOKENS || best_work < 1.2 * dram;
+  return epi != GP_STORE || best_work < 1.2 * dram;
 }
 
 template <int EPI, typename TO, int CG>
