@@ -401,9 +401,12 @@ static int gp_plan_many(int T, int N, int K, int sms, int* cg_out, int* bn_out) 
 // clocks that one costs anyway; or W's bytes at 6.3 TB/s; the longer of both and some of the other; plus an item's epilogue and the partial sums' way through L2.
 // Measured on a B200, us, here / the library (the gated product with its activation, the others with the norm that follows), 3B and 7B:
 //   tokens       gate and up                down                 output projection
-//     64      18.1 / 21.7 45.0/51.8  14.0 / 19.0 29.0/33.9   7.3 / 8.2 11.3/11.2
+//     64      18.1 / 21.7 45.0/51.8  14.0 / 19.0 29.0/33.9   7.3 / 8.2    - /11.2
 //    192      21.7 / 25.9 55.2/60.6  16.8 / 19.9 36.4/47.1     - / 8.7    - /12.4
 //    512      37.0 / 43.9 95.3/110     - / 27.1    - /60.5     - /10.8    - /17.4
+// Sums for a norm, from where on the library shares K well enough by itself: 3,584 x 3,584, 17, 64, 112 and 128 tokens 10.6 / 10.9, 11.3 / 11.2,
+// 11.7 / 10.6 and 12.3 / 11.4; 5,120 x 5,120, 64 tokens 16.4 / 15.3; 2,048 x 4,096, 192 and 256 tokens 11.5 / 11.5 and 12.2 / 11.6; 2,048 x
+// 5,632, 256 tokens 13.6 / 13.7; 4,096 x 14,336, 144 and 256 tokens 31.7 / 29.2 and 36.9 / 33.8.
 // Whole sums: a projection over the vocabulary alone.  float32 results, 151,936 x 2,048 and 152,064 x 3,584: 17 rows 99 / 107 and 166 / 185,
 // 128 rows 117 / 140 and 202 / 219, 256 rows 145 / 187 and 248 / 325; 32,000 x 2,048: 64 rows 26.5 / 27.8, 128 rows 28.3 / 30.9, but 160 rows
 // 31.9 / 31.2.  Fewer features are the library's at any number of tokens: 12,352 x 2,048, 64 rows 11.6 / 11.8, 129 rows 15.1 / 13.1, 1,025
@@ -415,7 +418,7 @@ extern "C" int qd_gemm_pair_plan(int T, int N, int K, int epi, int sms, int* cg_
   if ((long long)N * K < (1 << 20)) return 0;        // small models: a launch's own time
   if (epi != GP_GATED && T > GP_PLAIN_TOKENS) return 0;
   if (epi == GP_STORE && N < (T <= 128 ? 30000 : 100000)) return 0;
-  if (epi == GP_PARTIAL && T > 128 && K < 2 * N) return 0;
+  if (epi == GP_PARTIAL && (T <= 128 ? K < 2 * N && N > 3072 : 2 * K < (T <= 192 ? 4 : 5) * N || N >= 4096)) return 0;
   if (epi == GP_GATED && T > GP_PLAIN_TOKENS) {
     *splits_out = 1;
     return gp_plan_many(T, N, K, sms, cg_out, bn_out);
