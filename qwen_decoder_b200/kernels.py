@@ -513,12 +513,15 @@ def gemm_pair_sizes_plan(T: int, N: int, K: int, epi: int, sms: int):
 def gemm_pair_plan(x: torch.Tensor, w: torch.Tensor, epi: int):
     """(cg, bn, splits) for ``gemm_pair`` of more tokens than the few-token kernels take, or None where it does not take the
     product or the library's is the faster one."""
-    T, K = x.shape
-    if not (x.is_cuda and x.dtype == w.dtype == torch.bfloat16 and not few_token_impl(T) and K % 8 == 0 and x.stride(1) == 1
-            and x.stride(0) % 8 == 0 and x.stride(0) >= K and w.is_contiguous() and x.data_ptr() % 16 == 0
-            and w.data_ptr() % 16 == 0):
+    if not x.is_cuda:
         return None
-    return gemm_pair_sizes_plan(T, w.shape[0], K, epi, sm_count())
+    T, K = x.shape
+    plan = gemm_pair_sizes_plan(T, w.shape[0], K, epi, sm_count())      # first: most products are not taken, and this is kept
+    if plan is None or not (x.dtype == w.dtype == torch.bfloat16 and not few_token_impl(T) and K % 8 == 0 and x.stride(1) == 1
+                            and x.stride(0) % 8 == 0 and x.stride(0) >= K and w.is_contiguous() and x.data_ptr() % 16 == 0
+                            and w.data_ptr() % 16 == 0):
+        return None
+    return plan
 
 
 def gemm_pair(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, cg: int, bn: int,
@@ -1748,12 +1751,19 @@ def linear_exp_gates(e: ExpGates, H: int, state: torch.Tensor, ctx, write_state:
     return g, inn, low
 
 
+@functools.lru_cache(maxsize=4096)
 def linear_chunk_scratch(T: int, R: int, H: int, G: int, d: int, dv: int, DP: int, delta: bool, nrm: int) -> int:
     """Floats of scratch with which portions of T tokens of R requests go through the recurrence in chunks, 0: token by token.  Never
     more than 2^24: longer portions go in several passes."""
     fn = library("linear_scan").qd_linear_chunk_scratch
     fn.restype = ctypes.c_longlong
     return int(fn(_I(T), _I(R), _I(H), _I(G), _I(d), _I(dv), _I(DP), _I(1 if delta else 0), _I(nrm)))
+
+
+@functools.lru_cache(maxsize=4096)
+def linear_chunk_passes(T: int, R: int, H: int, d: int, floats: int) -> int:
+    """Passes of three launches that those portions take with ``floats`` of scratch."""
+    return int(library("linear_scan").qd_linear_chunk_passes(_I(T), _I(R), _I(H), _I(d), _LL(floats)))
 
 
 def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: Optional[torch.Tensor], beta: Optional[torch.Tensor],
@@ -1822,7 +1832,7 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: Optional[t
     if not single:
         _launch_count[0] += 1 if coef is None else 2
         if floats:
-            _launch_count[0] += 3 * library("linear_scan").qd_linear_chunk_passes(_I(T), _I(ctx.num_requests), _I(H), _I(d), _LL(floats)) - 2
+            _launch_count[0] += 3 * linear_chunk_passes(T, ctx.num_requests, H, d, floats) - 2
 
 
 # ------------------------------------------------------------------ norms in groups, before and after a branch
