@@ -33,6 +33,7 @@
 #define GP_BK 64
 
 #define GP_PLAIN_TOKENS 256           // beyond these only the gated product is taken
+#define GP_STORE_FEATURES 10240       // of whole sums at least
 
 #define GP_STORE 0
 #define GP_PARTIAL 1
@@ -404,21 +405,24 @@ static int gp_plan_many(int T, int N, int K, int sms, int* cg_out, int* bn_out) 
 //     64      18.1 / 21.7 45.0/51.8  14.0 / 19.0 29.0/33.9   7.3 / 8.2    - /11.2
 //    192      21.7 / 25.9 55.2/60.6  16.8 / 19.9 36.4/47.1     - / 8.7    - /12.4
 //    512      37.0 / 43.9 95.3/110     - / 27.1    - /60.5     - /10.8    - /17.4
-// Sums for a norm, from where on the library shares K well enough by itself: 3,584 x 3,584, 17, 64, 112 and 128 tokens 10.6 / 10.9, 11.3 / 11.2,
-// 11.7 / 10.6 and 12.3 / 11.4; 5,120 x 5,120, 64 tokens 16.4 / 15.3; 2,048 x 4,096, 192 and 256 tokens 11.5 / 11.5 and 12.2 / 11.6; 2,048 x
-// 5,632, 256 tokens 13.6 / 13.7; 4,096 x 14,336, 144 and 256 tokens 31.7 / 29.2 and 36.9 / 33.8.
-// Whole sums: a projection over the vocabulary alone.  float32 results, 151,936 x 2,048 and 152,064 x 3,584: 17 rows 99 / 107 and 166 / 185,
-// 128 rows 117 / 140 and 202 / 219, 256 rows 145 / 187 and 248 / 325; 32,000 x 2,048: 64 rows 26.5 / 27.8, 128 rows 28.3 / 30.9, but 160 rows
-// 31.9 / 31.2.  Fewer features are the library's at any number of tokens: 12,352 x 2,048, 64 rows 11.6 / 11.8, 129 rows 15.1 / 13.1, 1,025
-// rows 49.2 / 41.3, 1,500 rows 57.8 / 57.7; 8,192 x 2,048 in bfloat16, 64 rows 9.6 / 8.7, 1,281 rows 35.6 / 31.2; q/k/v of the 3B sizes, 64
-// rows 7.5 / 5.8.
+// Sums for a norm, where the library shares K well enough by itself: 3,584 x 3,584, 17, 64, 112 and 128 tokens 10.6 / 10.9, 11.3 / 11.2,
+// 11.7 / 10.6 and 12.3 / 11.4; 5,120 x 5,120, 64 tokens 16.4 / 15.3; 4,096 x 14,336, 144 and 256 tokens 31.7 / 29.2 and 36.9 / 33.8.
+// Whole sums, float32: a projection over the vocabulary, 151,936 x 2,048 and 152,064 x 3,584: 17 rows 99 / 107 and 166 / 185, 128 rows 117 / 140
+// and 202 / 219, 256 rows 145 / 187 and 248 / 325; 32,000 x 2,048: 64 rows 26.5 / 27.8, 128 rows 28.3 / 30.9, 160 rows 31.9 / 31.2.
+// Layers' own: 12,352 x 2,048, 64 and 129 tokens 11.6 / 11.8 and 15.1 / 13.1.  These stay here up to 256 tokens all the same: steps of so
+// few tokens through such layers wait for the host, where a call of the library's costs 19 us more (a prompt of 130 tokens through eight
+// mixed layers 2,115 us, with the library's eight products 2,220; in 64 requests' replayed step, where the host does not count, 1,010 and
+// 968).  2,048 x 4,096 of 193 to 256 tokens for a norm for the same reason: 12.2 / 11.6, 200 tokens through eight layers 2,100 us and 2,270.
+// Beyond 256 tokens the library's are up to 16 % faster and never more than 5 % slower: 12,352 x 2,048, 1,025 and 1,500 tokens 49.2 / 41.3 and
+// 57.8 / 57.7.  So they are with fewer features: 8,192 x 2,048 in bfloat16, 32 and 129 tokens 10.3 / 8.5 and 11.6 / 9.9; q/k/v of the 3B
+// sizes, 64 tokens 7.5 / 5.8.
 extern "C" int qd_gemm_pair_plan(int T, int N, int K, int epi, int sms, int* cg_out, int* bn_out, int* splits_out) {
   epi &= 255;
   if (T <= 0 || N <= 0 || K <= 0 || sms < 2) return 0;
   if ((long long)N * K < (1 << 20)) return 0;        // small models: a launch's own time
   if (epi != GP_GATED && T > GP_PLAIN_TOKENS) return 0;
-  if (epi == GP_STORE && N < (T <= 128 ? 30000 : 100000)) return 0;
-  if (epi == GP_PARTIAL && (T <= 128 ? K < 2 * N && N > 3072 : 2 * K < (T <= 192 ? 4 : 5) * N || N >= 4096)) return 0;
+  if (epi == GP_STORE && N < GP_STORE_FEATURES) return 0;
+  if (epi == GP_PARTIAL && (T <= 128 ? K < 2 * N && N > 3072 : K < 2 * N || N >= 4096)) return 0;
   if (epi == GP_GATED && T > GP_PLAIN_TOKENS) {
     *splits_out = 1;
     return gp_plan_many(T, N, K, sms, cg_out, bn_out);
