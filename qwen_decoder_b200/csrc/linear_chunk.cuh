@@ -501,11 +501,21 @@ linear_chunk_out_kernel(LinearChunk a) {
 
 // ------------------------------------------------------------------------------------------------ host
 // Whether the sizes are taken: whole heads of 64 x 64 or 128 x 128 without the delta rule, and portions that are long enough on the
-// average.  Measured on a B200, us a call, chunks / token by token, 32 heads of 64 x 64: 128 tokens 17.2 / 16.5, 256 18.7 / 29.2,
-// 1,500 66 / 155, three portions of 200 34 / 42, eight of 128 49 / 43.
+// average.
 #define LC_MEAN 192
 static bool lc_takes(int T, int R, int d, int dv, int DP, bool delta, int nrm) {
   return !nrm && !delta && d == DP && dv == d && (d == 128 || d == 64) && (long long)T >= (long long)LC_MEAN * R;
+}
+// Whether they are the faster form, the longest portion having ``longest`` tokens: in chunks every (chunk, head) is work for itself, token
+// by token only every (request, head), which is enough where there are many of these.  us, fitted to captured calls with 4 to 128
+// heads.  Measured on a B200, chunks / token by token, 32 heads of 64: 256 tokens 19.5 / 29.3, 1,500 67.4 / 155, three portions of 200 36.8 /
+// 41.7, eight of 400 154 / 127; 64 heads, three of 200 67.9 / 53.4; 32 heads of 128: 256 tokens 35.6 / 49.9, 1,500 172 / 275, three of 200
+// 84.5 / 73.8, eight of 400 399 / 326; 128 heads of 128, 1,500 tokens 726 / 674.
+static bool lc_pays(int T, int R, int H, int d, int longest) {
+  const double work = (T / 64.0 + 0.5 * R) * H, side_by_side = (double)H * T / longest;
+  const double chunks = d == 64 ? 14 + 0.07 * work + 0.018 * fmax(0.0, work - 800) : 20 + 0.15 * work + 0.1 * fmax(0.0, work - 280);
+  const double tokens = 4 + longest * (d == 64 ? fmax(0.0965, 0.09 + 0.00095 * side_by_side) : fmax(0.155, 0.09 + 0.0029 * side_by_side));
+  return chunks <= tokens;
 }
 static long long lc_chunks(int T, int R) { return (long long)T / LC + R; }      // no fewer than there are
 

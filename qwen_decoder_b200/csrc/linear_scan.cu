@@ -1161,10 +1161,12 @@ extern "C" int qd_linear_scan(const float* q, const float* k, const float* v, lo
   return qd_last_error();
 }
 
-// Floats of scratch with which qd_linear_scan takes these portions in chunks, 0: it does not.  Never more than LC_SCRATCH.
-extern "C" long long qd_linear_chunk_scratch(int T, int n_requests, int H, int G, int d, int dv, int DP, int delta, int nrm) {
+// Floats of scratch with which qd_linear_scan takes these portions, the longest of ``longest`` tokens, in chunks, 0: it does not, or
+// goes token by token in less time.  Never more than LC_SCRATCH.
+extern "C" long long qd_linear_chunk_scratch(int T, int n_requests, int H, int G, int d, int dv, int DP, int delta, int nrm, int longest) {
   if (T <= 0 || n_requests <= 0 || T == n_requests || H <= 0 || G <= 0 || H > 65535 || n_requests > 65535 ||
-      lc_chunks(T, n_requests) > 65535 || !lc_takes(T, n_requests, d, dv, DP, delta != 0, nrm))
+      lc_chunks(T, n_requests) > 65535 || longest <= 0 || !lc_takes(T, n_requests, d, dv, DP, delta != 0, nrm) ||
+      !lc_pays(T, n_requests, H, d, longest))
     return 0;
   return lc_scratch(T, n_requests, H, d);
 }

@@ -1752,12 +1752,13 @@ def linear_exp_gates(e: ExpGates, H: int, state: torch.Tensor, ctx, write_state:
 
 
 @functools.lru_cache(maxsize=4096)
-def linear_chunk_scratch(T: int, R: int, H: int, G: int, d: int, dv: int, DP: int, delta: bool, nrm: int) -> int:
-    """Floats of scratch with which portions of T tokens of R requests go through the recurrence in chunks, 0: token by token.  Never
-    more than 2^24: longer portions go in several passes."""
+def linear_chunk_scratch(T: int, R: int, H: int, G: int, d: int, dv: int, DP: int, delta: bool, nrm: int, longest: int = 0) -> int:
+    """Floats of scratch with which portions of T tokens of R requests, the longest of ``longest`` (0: all alike), go through the
+    recurrence in chunks, 0: token by token.  Never more than 2^24: longer portions go in several passes."""
     fn = library("linear_scan").qd_linear_chunk_scratch
     fn.restype = ctypes.c_longlong
-    return int(fn(_I(T), _I(R), _I(H), _I(G), _I(d), _I(dv), _I(DP), _I(1 if delta else 0), _I(nrm)))
+    return int(fn(_I(T), _I(R), _I(H), _I(G), _I(d), _I(dv), _I(DP), _I(1 if delta else 0), _I(nrm),
+                  _I(longest or -(-T // R))))
 
 
 @functools.lru_cache(maxsize=4096)
@@ -1815,7 +1816,8 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: Optional[t
     if not raw and v.data_ptr() % 16 == q.data_ptr() % 16 == k.data_ptr() % 16 == state.data_ptr() % 16 == 0 and v.stride(0) % 4 == 0 \
             and state.stride(0) % 4 == s_off % 4 == 0 and gate.stride(0) % 2 == out.stride(0) % 2 == 0 and gate.data_ptr() % 8 == 0 \
             and out.data_ptr() % (2 * out.element_size()) == 0:
-        floats = linear_chunk_scratch(T, ctx.num_requests, H, G, d, dv, DP, beta is not None, nrm)
+        floats = linear_chunk_scratch(T, ctx.num_requests, H, G, d, dv, DP, beta is not None, nrm,
+                                      getattr(ctx, "max_portion", 0))
     chunk = new(floats) if floats else None           # long portions: in chunks
     o = None if single or floats else new(T, H * dv)
     nq = new(T, H) if nrm and not single else None

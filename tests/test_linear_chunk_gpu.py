@@ -190,7 +190,20 @@ def test_passes(d, lengths, chunks, write, monkeypatch):
 
 def test_scratch_has_a_limit():
     from qwen_decoder_b200 import kernels
-    for T, R, H, d in ((1500, 1, 32, 64), (32768, 1, 32, 128), (1 << 20, 3, 64, 128), (4000000, 1, 8, 64)):
+    for T, R, H, d in ((1500, 1, 32, 64), (32768, 1, 32, 128), (1 << 20, 3, 4, 128), (4000000, 1, 8, 64)):
         floats = kernels.linear_chunk_scratch(T, R, H, H, d, d, d, False, 0)
         assert 0 < floats <= 1 << 24
     assert kernels.linear_chunk_scratch(1 << 20, 1, 1024, 1024, 128, 128, 128, False, 0) == 0          # not two states and a chunk
+
+
+# heads, size of one, portions, us in chunks, us token by token (a B200, captured calls): the faster form, or one 5 % from it
+@pytest.mark.parametrize("H,d,lengths,chunks,tokens", [
+    (32, 64, [192], 19.1, 23.0), (32, 64, [1500], 67.4, 154.9), (32, 64, [200] * 3, 36.8, 41.7), (32, 64, [192] * 8, 74.5, 62.1),
+    (32, 64, [400] * 8, 153.6, 127.1), (16, 64, [400] * 8, 79.6, 81.6), (16, 64, [600] * 16, 233.3, 190.0), (64, 64, [200] * 3, 67.9, 53.4),
+    (128, 64, [1500], 255.7, 301.6), (32, 64, [3, 5, 600], 38.4, 109.6), (4, 64, [600] * 16, 62.0, 91.7),
+    (32, 128, [200] * 3, 84.5, 73.8), (32, 128, [600], 78.1, 111.8), (64, 128, [192] * 8, 417.8, 310.1), (16, 128, [600] * 16, 632.6, 487.2),
+    (128, 128, [400], 196.8, 182.1), (128, 128, [1500], 726.1, 673.9), (64, 128, [1500], 340.1, 405.0), (8, 128, [400] * 8, 103.2, 109.1)])
+def test_the_faster_form(H, d, lengths, chunks, tokens):
+    from qwen_decoder_b200 import kernels
+    taken = kernels.linear_chunk_scratch(sum(lengths), len(lengths), H, H, d, d, d, False, 0, max(lengths)) > 0
+    assert (chunks if taken else tokens) <= 1.05 * min(chunks, tokens)
