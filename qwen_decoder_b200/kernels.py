@@ -1514,15 +1514,26 @@ def sink_tc5_supported(q: torch.Tensor, out: torch.Tensor, H: int, G: int, d: in
             and not (gate is not None and gate_elem and (gate.data_ptr() % 16 or gate.stride(0) % 4)))
 
 
+def sink_tc5_faster(n_tokens: int, n_requests: int, H: int, G: int, d: int, keys: int, sms: int) -> bool:
+    """Whether the tcgen05 form takes no longer for portions that see up to ``keys`` keys: rounds of its CTAs (128 rows, one to a
+    multiprocessor) against rounds of the mma.sync form's (64 rows, two or four), us a round by the keys.  Measured on a B200, us, mma.sync /
+    tcgen05: 16 + 2 heads of 128: 2 tokens 6.6 / 6.9, 17 7.9 / 8.1, 32 behind 900 57 / 17, 1,500 108 / 24; 16 + 16 heads of 128: 16 portions
+    of 3 behind 50 9.4 / 16.8, behind 1,000 74 / 36; 8 + 8 heads of 64: 60 portions of 2 behind 200 30 / 39."""
+    gs = H // G
+    rounds = lambda rows, at_a_time: -(-(n_tokens // (rows // gs) + n_requests) * G // (sms * at_a_time))
+    return rounds(128, 1) * (5.2 + 0.0105 * keys) <= rounds(64, 2 if d > 64 else 4) * ((4.6 + 0.053 * keys) if d > 64 else (4.3 + 0.039 * keys))
+
+
 def sink_attention_mma(q: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, block_table: torch.Tensor,
                        cu_tokens: torch.Tensor, start_pos: torch.Tensor, n_requests: int, n_tokens: int, H: int, G: int,
                        d: int, vd: int, page_size: int, scale: float, window: int, sinks: Optional[torch.Tensor],
                        splits: int = 1, chunk: int = 0, gate: Optional[torch.Tensor] = None,
-                       out_scale: float = 1.0, gate_elem: bool = False, cap: float = 0.0) -> None:
+                       out_scale: float = 1.0, gate_elem: bool = False, cap: float = 0.0, max_keys: int = 0) -> None:
     """``sink_attention_generic`` on tensor cores for portions of ``n_requests`` requests (rows cu_tokens[r] ..
     cu_tokens[r+1]-1 of q and out, at positions start_pos[r]..): a decoded token is a portion of one.  ``splits`` > 1
     shares every tile's keys among that many CTAs (for steps of few tokens over long contexts).  ``chunk``, ``gate``,
-    ``gate_elem``, ``out_scale``, ``cap`` and strided rows of ``out`` as for the generic kernel."""
+    ``gate_elem``, ``out_scale``, ``cap`` and strided rows of ``out`` as for the generic kernel.  ``max_keys``: the most keys of a
+    request (0: what its block table holds)."""
     assert q.dtype == out.dtype == kv.dtype == torch.bfloat16 and q.shape[1] == H * d and out.shape[1] == H * vd
     assert out.stride(1) == 1 and out.stride(0) % 2 == 0
     assert gate is None or (gate.dtype == torch.float32 and gate.stride(1) == 1)
@@ -1532,10 +1543,10 @@ def sink_attention_mma(q: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, blo
     assert cu_tokens.dtype == torch.int32 and start_pos.dtype == torch.int32
     assert sinks is None or (sinks.dtype == torch.float32 and sinks.numel() == H)
     _contig(q, "q"); _contig(kv, "kv"); _contig(block_table, "block_table")
-    # portions: the tcgen05 kernel was the faster one at every length (16 + 2 heads of 128, us: 2 tokens 17.5 and 12.6, 32 behind 900
-    # keys 68 and 24, 1,500 in blocks of 1,024 87 and 36)
+    keys = max_keys or block_table.shape[1] * page_size
     if SINK_TC5 and splits == 1 and n_tokens > n_requests and kv.data_ptr() % 16 == 0 \
-            and sink_tc5_supported(q, out, H, G, d, vd, page_size, gate, gate_elem, cap):
+            and sink_tc5_supported(q, out, H, G, d, vd, page_size, gate, gate_elem, cap) \
+            and sink_tc5_faster(n_tokens, n_requests, H, G, d, min(keys, window or keys, chunk or keys), sm_count()):
         _check(library("attention_tc5").qd_sink_attention_tc5(
             _ptr(q), _ptr(out), _LL(out.stride(0)), _ptr(kv), _LL(kv.numel() // (2 * G * page_size * d)), _ptr(block_table),
             _I(block_table.shape[1]), _ptr(cu_tokens), _ptr(start_pos), _I(n_requests), _I(n_tokens), _I(H), _I(G), _I(d), _I(page_size),

@@ -198,7 +198,8 @@ class MaskedAttention(Mixer):
                                            *args, splits=splits, **extra)
             if nd < T:
                 kernels.sink_attention_mma(q, out, paged.kv, grp.block_table[nd:], ctx.cu_tokens[nd:],
-                                           ctx.start_pos[nd:], ctx.num_requests - nd, T - nd, *args, **extra)
+                                           ctx.start_pos[nd:], ctx.num_requests - nd, T - nd, *args, **extra,
+                                           max_keys=ctx.max_context)
             return
         kernels.sink_attention_generic(q, out, paged.kv, grp.block_table, ctx.token_request, ctx.positions, H, G, d, vd,
                                        ps, self.scale, window, self.sinks, **extra)

@@ -122,7 +122,7 @@ class SinkAttention(Mixer):
                                            nd, nd, *args, splits=splits)
             if nd < T:
                 kernels.sink_attention_mma(q, attn, cache.kv, cache.group.block_table[nd:], ctx.cu_tokens[nd:],
-                                           ctx.start_pos[nd:], ctx.num_requests - nd, T - nd, *args)
+                                           ctx.start_pos[nd:], ctx.num_requests - nd, T - nd, *args, max_keys=ctx.max_context)
             return self.out.forward_partial(attn)
         kernels.sink_attention_generic(q, attn, cache.kv, cache.group.block_table, ctx.token_request, ctx.positions,
                                        H, G, d, vd, ps, self.scale, window, self.sinks)

@@ -100,3 +100,16 @@ def test_sinks_far_from_the_scores(monkeypatch):
         want = reference(q, kv, table, [140], [0], 4, 1, 64, 16, 0.125, 0, 0, sinks, None, False, 1.0)
         assert torch.isfinite(out).all()
         assert float((out.double() - want).abs().max()) <= 2.0 ** -7 * max(1e-30, float(want.abs().max()))
+
+
+# query and kv heads, size, tokens a portion, portions, keys, us on mma.sync, us on tcgen05 (a B200, captured calls)
+@pytest.mark.parametrize("H,G,d,n,R,keys,mma,tc5", [
+    (16, 2, 128, 2, 1, 2, 6.6, 6.9), (16, 2, 128, 2, 1, 902, 53.8, 15.5), (16, 2, 128, 17, 1, 17, 7.9, 8.1), (16, 2, 128, 1500, 1, 1500, 107.7, 24.3),
+    (16, 2, 128, 3, 16, 53, 9.3, 7.3), (8, 8, 64, 2, 1, 2, 5.2, 5.9), (8, 8, 64, 17, 1, 17, 5.8, 5.9), (8, 8, 64, 2, 60, 202, 30.5, 39.2),
+    (8, 8, 64, 20, 8, 320, 17.6, 8.6), (16, 16, 128, 3, 16, 53, 9.4, 16.8), (16, 16, 128, 3, 16, 1003, 74.0, 36.4), (16, 16, 128, 2, 60, 202, 82.2, 84.0),
+    (32, 4, 64, 2, 60, 202, 21.0, 23.3), (32, 4, 64, 32, 1, 932, 41.7, 14.3), (32, 8, 128, 2, 1, 2, 6.3, 7.1), (32, 8, 128, 17, 1, 17, 8.2, 6.9),
+    (32, 8, 128, 2, 60, 202, 45.1, 44.1)])
+def test_the_faster_form(H, G, d, n, R, keys, mma, tc5):
+    from qwen_decoder_b200 import kernels
+    taken = kernels.sink_tc5_faster(n * R, R, H, G, d, keys, 148)
+    assert (tc5 if taken else mma) <= 1.06 * min(mma, tc5)
