@@ -18,6 +18,7 @@ from typing import List, Optional, Sequence
 import numpy as np
 import torch
 
+from .. import kernels
 from ..cache import CacheManager, RequestCache
 
 
@@ -81,8 +82,10 @@ _SPLIT_MIXED = True
 def uneven_contexts(starts: Sequence[int], rows: int) -> bool:
     """Whether single tokens after ``starts`` tokens each, padded to ``rows`` rows, differ so much that shares by length pay: the same
     shares for every row would read more than 1.15 times the keys there are.  (64 of equal length: 2,805 us a step with the same
-    shares, 2,816 with shares by length; 23 of 500 to 4,000, padded to 32: 3,732 and 3,492.)"""
-    return len(starts) > 1 and (max(starts) + 1) * rows > 1.15 * (sum(starts) + len(starts))
+    shares, 2,816 with shares by length; 23 of 500 to 4,000, padded to 32: 3,732 and 3,492.)  Below two shares of keys there is
+    nothing to deal out (24 requests of up to 300 keys, 40 + 8 heads of 128: attention 6.3 us, with shares by length 7.5)."""
+    return (len(starts) > 1 and max(starts) + 1 >= kernels.SHARED_KEYS
+            and (max(starts) + 1) * rows > 1.15 * (sum(starts) + len(starts)))
 
 
 def _pad4(n: int) -> int:

@@ -718,6 +718,7 @@ def decode_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, kv: torc
 
 
 DECODE_SHARE_TOKENS, DECODE_SHARE_KEYS = 1024, 65535 * 16
+SHARED_KEYS = 320     # a token's keys from where on several CTAs of decode attention share them: twenty 16-key chunks
 
 
 def decode_ctas(d: int) -> int:

@@ -167,11 +167,11 @@ def step_decode_shares(ctx, cache: PagedCacheView, H: int, G: int, d: int, windo
 
 def decode_splits(ctas_without_split: int, max_keys: int, target_ctas: Optional[int] = None) -> int:
     """How many CTAs share one (request, kv head) in decode attention: as many as run at a time (``target_ctas``: two to a
-    multiprocessor unless given), never a second wave of them, and no CTA with fewer than ten 16-key chunks.  Keys of 2,048 at 16
-    query and 2 kv heads of 128, us: 32 requests 14.3 in 4 shares, 14.9 in 3, 21.9 in 5; 17 requests 10.2 in 8, 11.3 in 5; 8 and 2
+    multiprocessor unless given), never a second wave of them, one for every ten 16-key chunks (the last of them for what is left), and
+    one alone below 20 chunks (24 requests of 300 keys, 8 heads of 64: 5.0 us, two shares 6.3).  Keys of 2,048 at 16 query and 2 kv heads of 128, us: 32 requests 14.3 in 4 shares, 14.9 in 3, 21.9 in 5; 17 requests 10.2 in 8, 11.3 in 5; 8 and 2
     requests 7.7 and 6.3 in 12, 8.6 and 7.8 in 8, 9.3 and 8.1 in 18."""
     if target_ctas is None:
         target_ctas = 2 * kernels.sm_count()
     by_fill = target_ctas // max(1, ctas_without_split)
-    by_work = (max_keys + 159) // 160
+    by_work = (max_keys + 159) // 160 if max_keys >= kernels.SHARED_KEYS else 1
     return max(1, min(by_fill, by_work, 64))

@@ -74,3 +74,10 @@ def test_when_shares_by_length_pay():
     from qwen_decoder_b200.engine.batch import uneven_contexts
     assert not uneven_contexts([2048] * 64, 64) and uneven_contexts([2048] * 40, 64) and uneven_contexts([500, 4000, 900], 3)
     assert not uneven_contexts([], 0) and not uneven_contexts([4000], 1) and not uneven_contexts([0, 0], 2)
+    assert not uneven_contexts([299, 20, 30], 3) and uneven_contexts([319, 20, 30], 3)
+
+
+def test_shares_of_equal_contexts():
+    from qwen_decoder_b200.parts.attention import decode_splits
+    assert [decode_splits(48, k, 592) for k in (1, 160, 300, 319, 320, 330, 2048)] == [1, 1, 1, 1, 2, 3, 12]
+    assert decode_splits(700, 4000, 592) == 1 and decode_splits(2, 1 << 20, 592) == 64
