@@ -474,9 +474,11 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const bf
   int s = blockIdx.x, t = blockIdx.z;
   DecShare mine = {0, 0, 0, 0};
   if (SHARES) {
+    // The list's first reader comes right behind the launch that makes it and waits for it.  Later ones read it before their wait: no
+    // launch behind that first reader begins before all of its CTAs have passed this wait, since they let others begin
+    // (pdl_launch_dependents, below) or return only after it.  So the first reader must be told ``fresh``, and the trigger must not move up.
     if (fresh) pdl_wait();
-    // on its way while the barriers are made; no plain load: a kernel that this one may overlap has written the list, and what is
-    // read through a const __restrict__ pointer may be read before the wait
+    // on its way while the barriers are made; no plain load: what is read through a const __restrict__ pointer may be read before the wait
     asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(mine.ts), "=r"(mine.c), "=r"(mine.keys), "=r"(mine.n_same)
                  : "l"(shares + blockIdx.y) : "memory");
   }
@@ -636,7 +638,7 @@ decode_attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const bf
     }
     __syncwarp();
   }
-  pdl_launch_dependents();
+  pdl_launch_dependents();      // not before the wait for a fresh list: see there
   dec_finish<HD>(o, m0, m1, l0, l1, smem_raw, warp, lane, gs, g, t, s, H, G, splits, out, part_o, part_ml, tickets,
                  SHARES ? (size_t)(blockIdx.y - s) * H : (size_t)t * H * splits, SHARES ? T - mine.same() : 0, SHARES ? T : 0);
 }

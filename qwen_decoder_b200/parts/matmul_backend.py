@@ -87,11 +87,10 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: 
 # faster: decode steps at the 3B sizes 3.11 -> 2.92 ms at batch 64 and 2.60 -> 2.44 at batch 32 (2 and 8 shares:
 # 2.95), at the 7B sizes 3.81 -> 3.69 at batch 32, nothing with 5,120 output features; the product alone on cold
 # weights 17.5 -> 12.0 us at 128 tokens and 18.8 -> 13.5 at 256.
-# It is OFF (``library_split_k = 0``; 4 turns it on).  With it on, tests at the 3B and 7B sizes saw, in about one
-# run of ten, one row tile of a LATER prompt step's logits wrong (a 268- or 291-token portion, always the rows from
-# 128 on), also when that step's own products were plain ones and with the batched product's reader and writer
-# ordered by plain launches; five runs with it off showed none, as did all runs before it existed.  The cause was
-# not found (what the library's kernels keep between calls cannot be seen from here), so the plain product stands.
+# It is OFF (``library_split_k = 0``; 4 turns it on): the partial sums of ``csrc/gemm_pair.cu`` serve these products now, 14.0 and
+# 18.1 us with the norm at 64 and 256 tokens of the 3B sizes where the plain library product takes 19.0 and 20.3.  (While it was on, rows
+# from 128 on of a later prompt step came out wrong in about one run of ten.  That was the prompt attention's wait for its last product,
+# mended since; this product had no part in it.)
 library_split_k = 0
 LIBRARY_SPLIT_MAX_FEATURES = 4096
 LIBRARY_SPLIT_MAX_TOKENS = 256

@@ -138,8 +138,7 @@ def test_options(d, delta, monkeypatch):
 
 
 @pytest.mark.parametrize("d,delta", [(64, False), (128, False)])
-@pytest.mark.parametrize("what", ["v", "k", "g"])
-@pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.4e38])
+@pytest.mark.parametrize("what,value", [(w, x) for w in "vkg" for x in (float("inf"), float("nan"), 3.4e38) if (w, x) != ("g", 3.4e38)])
 def test_tokens_before_a_bad_one(d, delta, what, value, monkeypatch):
     p = make([960, 70], 2, 2, d, delta, True, seed=9, decay=(0.9, 1.0))
     good, _, _ = run(p, monkeypatch, True)
@@ -148,8 +147,6 @@ def test_tokens_before_a_bad_one(d, delta, what, value, monkeypatch):
         p.v[at, 3] = value
     elif what == "k":
         p.k[at, 0, 5] = value
-    elif value == 3.4e38:
-        return
     else:
         p.g[at, 0] = value
     got, state, _ = run(p, monkeypatch, True)
