@@ -131,8 +131,8 @@ class ModelRunner:
         (``cache.log_tokens``).  Only for batches that run as a graph (``can_take_device_tokens``).
 
         A batch of single tokens that all want logits runs as a replayed CUDA graph (one per padded
-        batch size, block-table width and evenness of contexts) when ``use_graphs`` is set; the logits then live in a
-        buffer that the next such step overwrites."""
+        batch size, block-table width and evenness of contexts; the first step of each is captured, tens of
+        milliseconds) when ``use_graphs`` is set; the logits then live in a buffer that the next such step overwrites."""
         if ensure_pages:
             self._ensure(entries)
         if self.can_take_device_tokens(entries):

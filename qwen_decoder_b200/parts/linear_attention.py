@@ -29,7 +29,7 @@ exponential gates [H, vd + 1, d], n as one more column, and then the H maxima), 
 rows [q | k | v] before the convolution; a fresh row is zero.  All projections of h are one stacked product with float32
 sums; everything between them and the rounded input of the output matrix is float32 in both engine dtypes
 (``csrc/linear_scan.cu``).  The recurrence runs in the tokens' order, the delta rule of longer portions in runs of four
-tokens (the same rule written out).  Single tokens whose q and k need nothing but their constants are read where the
+tokens (the same rule written out), long portions without it in chunks of 64 where that is faster (``csrc/linear_chunk.cuh``).  Single tokens whose q and k need nothing but their constants are read where the
 product left them: the step is one launch.
 
 ``inner`` computes everything up to the output projection into a tensor the caller gives, times ``out_scale``.
